@@ -7,16 +7,20 @@
 // One thread per particle keeps its state in registers for all steps; the
 // only memory traffic is the 64-byte particle record read once and one
 // atomic increment per recorded frame into the histogram (L2-resident for
-// the reference's 64^3 grid). The work is FP64 arithmetic, term by term in
-// the reference's order (built with -fmad=false): r^2.5 correctly rounded,
-// the sub-cycle rule, the Boris rotation and the periodic wrap are those of
-// the reference, so trajectories and counts match its host build.
+// the reference's 64^3 grid). The arithmetic is FP64, term by term in the
+// reference's order (built with -fmad=false): r^2.5 correctly rounded, the
+// sub-cycle rule, the Boris rotation and the periodic wrap are those of the
+// reference, so trajectories and counts match its host build. What bounds it
+// is the FP64 pipe (37 instructions per particle step at 64 to 76 cycles per
+// warp, 83 % busy), which is why most of the step's roundings are made on
+// the integer pipe (dipole64.cuh) and the rare comparisons sit behind calls:
+// 16M particles x 151 steps 641 -> 163 ms, 20k x 41 steps 432 -> 162 us.
 #include <cmath>
-#include <cstring>
 #include <mutex>
 
 #include "../../include/ipic3d_gpu.h"
 #include "launch.h"
+#include "dipole64.cuh"
 #include "particle_kernels.cuh"
 
 namespace ipg {
@@ -29,9 +33,10 @@ struct TraceArgs {
     double extent[3];        // width * size (the wrap distance)
     double w[3];             // cell width (getCellCoordinates)
     double center[3];        // objectCenter
-    int center_zero;         // objectCenter == 0: the planet test's r^2 is the next step's field r^2
-    int int_cmp;             // box and planet radius finite: comparisons on bit patterns
-    long long key_low[3], key_high[3];  // order_key of low, high
+    int quick_planet;        // objectCenter == 0 and R^2 finite: the planet test's r^2 is the next step's field r^2
+    int quick_box;           // the box is finite: order_key_hi - key_in < key_span lies strictly inside it
+    int32_t key_in[3];
+    uint32_t key_span[3];
     double r2max;            // planetRadius^2
     double mft;              // -Bext.z * pow(planetRadius, 3), host libm
     double dt, c;
@@ -44,16 +49,11 @@ struct TraceArgs {
     uint32_t* counts;
 };
 
-// An integer that orders finite and infinite doubles as their values do
-// (+0 and -0 both map to 0); NaN is tested apart. The comparisons of the
-// step loop run on these keys, in the integer pipe, which the FP64-bound
-// loop leaves idle.
-__device__ __forceinline__ long long order_key(double x) {
-    const long long b = __double_as_longlong(x);
-    return b >= 0 ? b : -(b & 0x7fffffffffffffffLL);
-}
-__device__ __forceinline__ bool is_nan_bits(double x) {
-    return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+// An integer that orders doubles by their high words as their values do
+// (negative ones below positive ones, NaN outside every finite value).
+__host__ __device__ __forceinline__ int32_t order_key_hi(double x) {
+    const int32_t h = (int32_t)(soft::bits_of(x) >> 32);
+    return h ^ ((h >> 31) & 0x7fffffff);
 }
 
 __device__ __forceinline__ double sum_sq(double a, double b, double c) {
@@ -61,6 +61,16 @@ __device__ __forceinline__ double sum_sq(double a, double b, double c) {
     r += b * b;
     r += c * c;
     return r;
+}
+
+// The rare steps' comparisons, in FP64.
+__device__ __noinline__ double wrapped(double p, double low, double high, double extent) {
+    if (p > high) p = p - extent;
+    if (p < low) p = p + extent;
+    return p;
+}
+__device__ __noinline__ bool inside_planet(double x, double y, double z, double r2max) {
+    return sum_sq(x, y, z) <= r2max;
 }
 
 __global__ void __launch_bounds__(kTraceThreads) k_trace(const TraceArgs A) {
@@ -79,7 +89,12 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const TraceArgs A) {
         if (P[a] > A.high[a] || P[a] < A.low[a]) return;
 
     int64_t next_record = 0, frame = 0;
-    double rf2 = sum_sq(P[0], P[1], P[2]);  // |position|^2 of the field
+    const DipoleSpecies K = dipole_species(A.mft, qom, A.dt, A.inv_pic);
+    // the squares of the position: the field's, and the planet test's with
+    // the object at the origin
+    bool fast = K.usable && coordinates_regular(P[0], P[1], P[2]);
+    SquaredPosition S = {};
+    if (fast) S = squared_position(P[0], P[1], P[2]);
     for (int t = 0; t < A.steps; ++t) {
         const bool record = t == next_record;  // t % frame_interval == 0
         int64_t cx = 0, cy = 0, cz = 0;
@@ -88,52 +103,48 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const TraceArgs A) {
             cy = (int64_t)((P[1] - A.low[1]) / A.w[1]);
             cz = (int64_t)((P[2] - A.low[2]) / A.w[2]);
         }
-        // dipole B at the absolute position, E = 0 (pic_tracer.cxx:104-111)
-        const double x = P[0], y = P[1], z = P[2];
-        const double fac1 = A.mft / pow25_rn(rf2);
-        const double bx = 3.0 * x * z * fac1;
-        const double by = 3.0 * y * z * fac1;
-        const double bz = (2.0 * (z * z) - (x * x) - (y * y)) * fac1;
-        // adaptive sub-cycling (pic_tracer.cxx:113-118)
-        double dts;
-        const int ns = sub_cycles_dt(A.dt, A.c, A.inv_pic, qom, sum_sq(bx, by, bz), dts);
-        for (int s = 0; s < ns; ++s) {
-            boris_e0(u, v, w, bx, by, bz, qom, dts);  // updateVelocity (particle.h:31-49)
-            P[0] = P[0] + u * dts;                    // updatePosition (particle.h:24-26)
-            P[1] = P[1] + v * dts;
-            P[2] = P[2] + w * dts;
-        }
-        // periodic wrap (pic_tracer.cxx:129-133)
-        if (A.int_cmp) {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const bool nan = is_nan_bits(P[a]);  // NaN compares false both ways
-                long long k = order_key(P[a]);
-                if (!nan && k > A.key_high[a]) {
-                    P[a] = P[a] - A.extent[a];
-                    k = order_key(P[a]);
-                }
-                if (!nan && k < A.key_low[a]) P[a] = P[a] + A.extent[a];
-            }
+        // dipole B at the absolute position, E = 0 (pic_tracer.cxx:104-111),
+        // Boris rotation and position (particle.h:24-49)
+        if (fast && dipole_rotate(K, P[0], P[1], P[2], S, u, v, w)) {
+            advance_position(P[0], P[1], P[2], u, v, w, A.dt);
         } else {
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if (P[a] > A.high[a]) P[a] = P[a] - A.extent[a];
-                if (P[a] < A.low[a]) P[a] = P[a] + A.extent[a];
+            const double x = P[0], y = P[1], z = P[2];
+            const double fac1 = A.mft / pow25_rn(sum_sq(x, y, z));
+            const double bx = 3.0 * x * z * fac1;
+            const double by = 3.0 * y * z * fac1;
+            const double bz = (2.0 * (z * z) - (x * x) - (y * y)) * fac1;
+            // adaptive sub-cycling (pic_tracer.cxx:113-118)
+            double dts;
+            const int ns = sub_cycles_dt(A.dt, A.c, A.inv_pic, qom, sum_sq(bx, by, bz), dts);
+            for (int s = 0; s < ns; ++s) {
+                boris_e0(u, v, w, bx, by, bz, qom, dts);  // updateVelocity (particle.h:31-49)
+                P[0] = P[0] + u * dts;                    // updatePosition (particle.h:24-26)
+                P[1] = P[1] + v * dts;
+                P[2] = P[2] + w * dts;
             }
+        }
+        // periodic wrap (pic_tracer.cxx:129-133). The high words settle that
+        // a position lies strictly inside the box; only the others compare
+        // and add in FP64 (a call, so that no FP64 instruction is issued,
+        // predicated off, for every particle: 11 of 56 a step were)
+        const bool inside = A.quick_box && (uint32_t)(order_key_hi(P[0]) - A.key_in[0]) < A.key_span[0] &&
+                            (uint32_t)(order_key_hi(P[1]) - A.key_in[1]) < A.key_span[1] &&
+                            (uint32_t)(order_key_hi(P[2]) - A.key_in[2]) < A.key_span[2];
+        if (!inside) {
+            P[0] = wrapped(P[0], A.low[0], A.high[0], A.extent[0]);
+            P[1] = wrapped(P[1], A.low[1], A.high[1], A.extent[1]);
+            P[2] = wrapped(P[2], A.low[2], A.high[2], A.extent[2]);
         }
         // tracing stops inside the planet (pic_tracer.cxx:135-141); with the
         // object at the origin, p - center is p itself, so the test's r^2 is
         // the one the next step's field needs
-        rf2 = sum_sq(P[0], P[1], P[2]);
-        const double rp2 =
-            A.center_zero ? rf2 : sum_sq(P[0] - A.center[0], P[1] - A.center[1], P[2] - A.center[2]);
-        // rp2 is >= 0 or NaN and r2max finite >= 0: their bit patterns
-        // without the sign order as the values (a NaN of either sign lies
-        // above everything, so "<=" fails as in FP64)
-        if (A.int_cmp ? (__double_as_longlong(rp2) & 0x7fffffffffffffffLL) <= __double_as_longlong(A.r2max)
-                      : rp2 <= A.r2max)
+        fast = K.usable && coordinates_regular(P[0], P[1], P[2]);
+        if (fast) S = squared_position(P[0], P[1], P[2]);
+        if (fast && A.quick_planet) {  // both positive: their bit patterns order as the values
+            if (soft::bits_of(soft::pack(S.r2)) <= soft::bits_of(A.r2max)) break;
+        } else if (inside_planet(P[0] - A.center[0], P[1] - A.center[1], P[2] - A.center[2], A.r2max)) {
             break;
+        }
         if (record) {
             // ParticleCount::increment(t / frame_interval, pos): the flat
             // index of its row-major vector, coordinates cast to int
@@ -171,17 +182,15 @@ int trace_args(const ipic3d_props* props, uint64_t n, int32_t steps, int32_t fra
         A.center[a] = props->object_center[a];
         A.size[a] = props->size[a];
     }
-    A.center_zero = props->object_center[0] == 0.0 && props->object_center[1] == 0.0 && props->object_center[2] == 0.0;
     A.r2max = props->planet_radius * props->planet_radius;
-    A.int_cmp = std::isfinite(A.r2max) && A.r2max >= 0.0;
+    A.quick_planet = props->object_center[0] == 0.0 && props->object_center[1] == 0.0 &&
+                     props->object_center[2] == 0.0 && std::isfinite(A.r2max);
+    A.quick_box = 1;
     for (int a = 0; a < 3; ++a) {
-        A.int_cmp = A.int_cmp && std::isfinite(A.low[a]) && std::isfinite(A.high[a]);
-        // order_key on the host: the same mapping
-        long long bl, bh;
-        std::memcpy(&bl, &A.low[a], 8);
-        std::memcpy(&bh, &A.high[a], 8);
-        A.key_low[a] = bl >= 0 ? bl : -(bl & 0x7fffffffffffffffLL);
-        A.key_high[a] = bh >= 0 ? bh : -(bh & 0x7fffffffffffffffLL);
+        if (!std::isfinite(A.low[a]) || !std::isfinite(A.high[a])) A.quick_box = 0;
+        A.key_in[a] = order_key_hi(A.low[a]) + 1;
+        const int64_t span = (int64_t)order_key_hi(A.high[a]) - A.key_in[a];
+        A.key_span[a] = span > 0 ? (uint32_t)span : 0u;
     }
     A.mft = -props->external_b[2] * std::pow(props->planet_radius, 3);
     A.dt = props->dt;
