@@ -17,6 +17,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "fp64_int.cuh"
+
 namespace ipg {
 
 constexpr int kVec = 4;                 // particles per thread (one float4 / 2x double2)
@@ -143,6 +145,35 @@ struct Push32Set {
     Push32Const c[kSetPops];
 };
 
+// Constants of a species' steps in the dipole field (dipole64.cuh).
+struct DipoleSpecies {
+    soft::Num mft;  // -Bext.z R^3
+    soft::Num k;    // q/m dt / 2
+    int e_max;      // largest biased exponent of a B component that surely needs one sub-cycle
+    int usable;     // the constants are in the range that dipole_rotate takes
+};
+
+// Host-computed constants of an FP64 population's push (push64.cuh).
+struct Push64Const {
+    DipoleSpecies d;
+    double k1;           // q/m dt / 2
+    double field_scale;  // 1 / vol with the gather normalisation, else 1
+};
+struct Push64Set {
+    Push64Const c[kSetPops];
+};
+
+template <typename T>
+struct PushConst;
+template <>
+struct PushConst<float> {
+    using type = Push32Const;
+};
+template <>
+struct PushConst<double> {
+    using type = Push64Const;
+};
+
 // ---- batched ensemble ------------------------------------------------------
 // One population of one universe of a batch: everything a batched particle
 // kernel needs, read from a device table indexed by job.
@@ -150,7 +181,7 @@ template <typename T>
 struct alignas(16) PopJob {  // 16-byte multiple: the FP32 push bulk-copies records
     Geom g;
     Pop<T> P;
-    Push32Const pc;         // FP32 populations: the push constants
+    typename PushConst<T>::type pc;
     int32_t* sort_tmp;      // placement scratch [capacity]
     uint32_t* pend_count;   // P.pending_in_count (written by the rotation)
 };

@@ -17,23 +17,15 @@
 
 namespace ipg {
 
-// Constants of a species' steps.
-struct DipoleSpecies {
-    soft::Num mft;  // -Bext.z R^3
-    soft::Num k;    // q/m dt / 2
-    int e_max;      // largest biased exponent of a B component that surely needs one sub-cycle
-    bool usable;    // the constants are in the range that dipole_step takes
-};
-
 // |B|^2 <= 3 2^(2 (e - 1023) + 2) for components of biased exponent <= e; one
 // sub-cycle is sure while the estimate of sub_cycles_dt is below 1/2.
-__device__ __forceinline__ DipoleSpecies dipole_species(double mft, double qom, double dt, double inv_pic) {
+__host__ __device__ __forceinline__ DipoleSpecies dipole_species(double mft, double qom, double dt, double inv_pic) {
     DipoleSpecies s;
     const double k = qom * 0.5 * dt;
     const double lim = (0.49 / 3.0) / ((dt * (4.0 * fabs(qom))) * inv_pic);
     s.mft = soft::unpack(mft);
     s.k = soft::unpack(k);
-    s.e_max = 1023 + ((soft::exponent_of(lim) - 1023 - 2) >> 1);
+    s.e_max = soft::regular(lim, 1000) ? 1023 + ((soft::exponent_of(lim) - 1023 - 2) >> 1) : -1;
     s.usable = soft::regular(dt, 100) && soft::regular(mft, 200) && soft::regular(k, 100) && soft::regular(lim, 1000);
     return s;
 }

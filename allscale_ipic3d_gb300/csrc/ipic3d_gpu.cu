@@ -2090,7 +2090,7 @@ void fill_consts(PopJob<T>& J);
 template <>
 void fill_consts<float>(PopJob<float>& J) { J.pc = push32_const(J.g, J.P); }
 template <>
-void fill_consts<double>(PopJob<double>&) {}
+void fill_consts<double>(PopJob<double>& J) { J.pc = push64_const(J.g, J.P); }
 
 // Builds the job records; uploads them (and the block maps) when they differ
 // from the ones on the device.

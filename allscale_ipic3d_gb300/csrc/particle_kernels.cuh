@@ -155,228 +155,6 @@ struct PState {
     T x, y, z, u, v, w;
 };
 
-// Trilinear field gather at fractional position r inside cell (cx,cy,cz):
-// trilinearInterpolationF2P (cell.h:867-885) applied to the node E and B of
-// the cell's 8 corners as in the commented mover (cell.h:905-937).
-__device__ __forceinline__ void gather64(const Geom& g, int cx, int cy, int cz, double rx, double ry, double rz,
-                                         double& ex, double& ey, double& ez, double& bx, double& by, double& bz) {
-    ex = ey = ez = bx = by = bz = 0.0;
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                double fac = (i == 0 ? (1 - rx) : rx) * (j == 0 ? (1 - ry) : ry) * (k == 0 ? (1 - rz) : rz);
-                const double* n = g.field + 9 * field_index(g, cx + i + 1, cy + j + 1, cz + k + 1);
-                ex = ex + __ldg(n + 0) * fac;
-                ey = ey + __ldg(n + 1) * fac;
-                ez = ez + __ldg(n + 2) * fac;
-                bx = bx + __ldg(n + 3) * fac;
-                by = by + __ldg(n + 4) * fac;
-                bz = bz + __ldg(n + 5) * fac;
-            }
-    if (g.flags & 2u /*IPIC3D_F_GATHER_DIV_VOL*/) {
-        ex = ex / g.vol; ey = ey / g.vol; ez = ez / g.vol;
-        bx = bx / g.vol; by = by / g.vol; bz = bz / g.vol;
-    }
-}
-
-__device__ __forceinline__ void gather32(const Geom& g, int cx, int cy, int cz, float rx, float ry, float rz, float& ex,
-                                         float& ey, float& ez, float& bx, float& by, float& bz) {
-    ex = ey = ez = bx = by = bz = 0.f;
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                float fac = (i == 0 ? (1.f - rx) : rx) * (j == 0 ? (1.f - ry) : ry) * (k == 0 ? (1.f - rz) : rz);
-                int64_t n = field_index(g, cx + i + 1, cy + j + 1, cz + k + 1);
-                float4 e = __ldg(g.node32 + 2 * n), b = __ldg(g.node32 + 2 * n + 1);
-                ex += e.x * fac; ey += e.y * fac; ez += e.z * fac;
-                bx += b.x * fac; by += b.y * fac; bz += b.z * fac;
-            }
-    if (g.flags & 2u) {
-        float iv = (float)(1.0 / g.vol);
-        ex *= iv; ey *= iv; ez *= iv; bx *= iv; by *= iv; bz *= iv;
-    }
-}
-
-// ---- mover + export for one particle ---------------------------------------
-// FP64: absolute position; the expressions follow cell.h term by term.
-__device__ __forceinline__ int step_particle(const Geom& g, int cx, int cy, int cz, double qom, PState<double>& p,
-                                             int& dest) {
-    // -- moveParticles (cell.h:896-964) --
-    double ex = 0.0, ey = 0.0, ez = 0.0, bx = 0.0, by = 0.0, bz = 0.0;
-    const bool field_mover = g.mover == 1;
-    if (field_mover) {
-        double ox = g.origin[0] + (double)cx * g.w[0], oy = g.origin[1] + (double)cy * g.w[1],
-               oz = g.origin[2] + (double)cz * g.w[2];
-        gather64(g, cx, cy, cz, (p.x - ox) / g.w[0], (p.y - oy) / g.w[1], (p.z - oz) / g.w[2], ex, ey, ez, bx, by, bz);
-    }
-    if (!field_mover || (g.flags & 4u /*IPIC3D_F_DIPOLE_IN_GATHER*/)) {
-        double r2 = p.x * p.x;
-        r2 += p.y * p.y;
-        r2 += p.z * p.z;
-        double fac1 = g.mft / pow25_rn(r2);
-        double dbx = 3.0 * p.x * p.z * fac1;
-        double dby = 3.0 * p.y * p.z * fac1;
-        double dbz = (2.0 * (p.z * p.z) - (p.x * p.x) - (p.y * p.y)) * fac1;
-        if (field_mover) {
-            bx = bx + dbx; by = by + dby; bz = bz + dbz;
-        } else {
-            bx = dbx; by = dby; bz = dbz;
-        }
-    }
-    double bmag = bx * bx;
-    bmag += by * by;
-    bmag += bz * bz;
-    double dts;
-    const int ns = sub_cycles_dt(g.dt, g.c, g.inv_pic, qom, bmag, dts);
-    for (int s = 0; s < ns; ++s) {
-        if (field_mover)
-            boris<double>(p.u, p.v, p.w, ex, ey, ez, bx, by, bz, qom, dts);
-        else
-            boris_e0(p.u, p.v, p.w, bx, by, bz, qom, dts);
-        p.x = p.x + p.u * dts;  // updatePosition (particle.h:24-26)
-        p.y = p.y + p.v * dts;
-        p.z = p.z + p.w * dts;
-    }
-    // -- exportParticles (cell.h:1093-1146) --
-    const int pos[3] = {cx, cy, cz};
-    const int size[3] = {g.sx, g.sy, g.sz};
-    double P[3] = {p.x, p.y, p.z};
-    double center[3], rel[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        center[a] = (g.origin[a] + (double)pos[a] * g.w[a]) + g.w[a] / 2.0;
-        rel[a] = P[a] - center[a];
-    }
-    bool invert = false, drop = false;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (pos[a] == 0 && rel[a] < -g.half_w[a]) {
-            if (g.bc_lo[a] == 0) { invert = true; P[a] = P[a] + g.half_w[a]; }
-            else if (g.bc_lo[a] == 2) drop = true;
-        } else if (pos[a] == size[a] - 1 && rel[a] > g.half_w[a]) {
-            if (g.bc_hi[a] == 0) { invert = true; P[a] = P[a] - g.half_w[a]; }
-            else if (g.bc_hi[a] == 2) drop = true;
-        }
-    }
-    if (invert) { p.u = p.u * -1.0; p.v = p.v * -1.0; p.w = p.w * -1.0; }
-    if (drop) return kDrop;
-    double dx = P[0] - g.object_center[0], dy = P[1] - g.object_center[1], dz = P[2] - g.object_center[2];
-    double r2 = dx * dx;
-    r2 += dy * dy;
-    r2 += dz * dz;
-    if (r2 <= g.planet_r2) return kDrop;
-    int d[3];
-    bool out = false;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        rel[a] = P[a] - center[a];
-        out |= fabs(rel[a]) > g.half_w[a];
-        d[a] = rel[a] < -g.half_w[a] ? -1 : (rel[a] > g.half_w[a] ? 1 : 0);
-    }
-    p.x = P[0]; p.y = P[1]; p.z = P[2];
-    if (!out) return kStay;
-    int n[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        int t = pos[a] + d[a];
-        if (t < 0) {
-            t += size[a];
-            if (g.bc_lo[a] == 1) P[a] += (double)size[a] * g.w[a];
-        } else if (t >= size[a]) {
-            t -= size[a];
-            if (g.bc_hi[a] == 1) P[a] -= (double)size[a] * g.w[a];
-        }
-        n[a] = t;
-    }
-    p.x = P[0]; p.y = P[1]; p.z = P[2];
-    dest = cell_id(g, n[0], n[1], n[2]);
-    return kMove;
-}
-
-// FP32: position relative to the cell origin in cell widths; inside <=> [0,1]
-// on every axis, which is the reference's |relPos| <= halfWidth test.
-__device__ __forceinline__ int step_particle(const Geom& g, int cx, int cy, int cz, float qom, PState<float>& p,
-                                             int& dest) {
-    const float w0 = (float)g.w[0], w1 = (float)g.w[1], w2 = (float)g.w[2];
-    const float iw0 = (float)g.inv_w[0], iw1 = (float)g.inv_w[1], iw2 = (float)g.inv_w[2];
-    float ex = 0.f, ey = 0.f, ez = 0.f, bx0 = 0.f, by0 = 0.f, bz0 = 0.f;
-    const bool field_mover = g.mover == 1;
-    const bool with_dipole = !field_mover || (g.flags & 4u);
-    if (field_mover) gather32(g, cx, cy, cz, p.x, p.y, p.z, ex, ey, ez, bx0, by0, bz0);
-    // cell origin relative to the dipole centre (the origin of coordinates)
-    const float ox = (float)(g.origin[0] + (double)cx * g.w[0]);
-    const float oy = (float)(g.origin[1] + (double)cy * g.w[1]);
-    const float oz = (float)(g.origin[2] + (double)cz * g.w[2]);
-    const float mft = (float)g.mft;
-    const float dt = (float)g.dt, c = (float)g.c;
-    // the dipole B of the reference mover is evaluated at the particle before
-    // the sub-cycles (cell.h:940-945)
-    float bx = bx0, by = by0, bz = bz0;
-    if (with_dipole) {
-        float X = ox + p.x * w0, Y = oy + p.y * w1, Z = oz + p.z * w2;
-        float r2 = X * X + Y * Y + Z * Z;
-        float fac1 = mft / (r2 * r2 * sqrtf(r2));
-        bx += 3.f * X * Z * fac1;
-        by += 3.f * Y * Z * fac1;
-        bz += (2.f * Z * Z - X * X - Y * Y) * fac1;
-    }
-    int ns = sub_cycles<float>(dt, c, qom, bx * bx + by * by + bz * bz);
-    float dts = dt / (float)ns;
-    float sx = dts * iw0, sy = dts * iw1, sz = dts * iw2;
-    for (int s = 0; s < ns; ++s) {
-        boris<float>(p.u, p.v, p.w, ex, ey, ez, bx, by, bz, qom, dts);
-        p.x += p.u * sx;
-        p.y += p.v * sy;
-        p.z += p.w * sz;
-    }
-    const int pos[3] = {cx, cy, cz};
-    const int size[3] = {g.sx, g.sy, g.sz};
-    float R[3] = {p.x, p.y, p.z};
-    bool invert = false, drop = false;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (pos[a] == 0 && R[a] < 0.f) {
-            if (g.bc_lo[a] == 0) { invert = true; R[a] += 0.5f; }
-            else if (g.bc_lo[a] == 2) drop = true;
-        } else if (pos[a] == size[a] - 1 && R[a] > 1.f) {
-            if (g.bc_hi[a] == 0) { invert = true; R[a] -= 0.5f; }
-            else if (g.bc_hi[a] == 2) drop = true;
-        }
-    }
-    if (invert) { p.u = -p.u; p.v = -p.v; p.w = -p.w; }
-    if (drop) return kDrop;
-    {
-        float dx = (float)(g.origin[0] + (double)cx * g.w[0] - g.object_center[0]) + R[0] * w0;
-        float dy = (float)(g.origin[1] + (double)cy * g.w[1] - g.object_center[1]) + R[1] * w1;
-        float dz = (float)(g.origin[2] + (double)cz * g.w[2] - g.object_center[2]) + R[2] * w2;
-        if (dx * dx + dy * dy + dz * dz <= (float)g.planet_r2) return kDrop;  // cell.h:1123-1128
-    }
-    int d[3];
-    bool out = false;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        d[a] = R[a] < 0.f ? -1 : (R[a] > 1.f ? 1 : 0);
-        out |= d[a] != 0;
-        R[a] -= (float)d[a];
-    }
-    p.x = R[0]; p.y = R[1]; p.z = R[2];
-    if (!out) return kStay;
-    int n[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        int t = pos[a] + d[a];
-        n[a] = t < 0 ? t + size[a] : (t >= size[a] ? t - size[a] : t);
-    }
-    dest = cell_id(g, n[0], n[1], n[2]);
-    return kMove;
-}
-
 // ---- deposit -----------------------------------------------------------------
 // Cloud-in-cell weights of projectToDensityField (cell.h:810-816): a particle
 // at fractional position r in cell c adds q v fac and q fac to node c+(i,j,k)
@@ -504,233 +282,6 @@ __device__ __forceinline__ void register_arrival(const Pop<T>& P, uint32_t o, co
         if (pi < P.pending_cap) P.pending_out[pi] = m;
         else atomicAdd(&P.ctr->lost, 1u);
     }
-}
-
-// ---- the fused push kernel ----------------------------------------------------
-// CTA b covers slots [b*kSlotsPerCta, (b+1)*kSlotsPerCta) of one population;
-// thread t the 4 slots from 4t (one cell, start[] is 4-aligned). mode 0 =
-// step (mover + export + deposit), mode 1 = deposit only (the projector over
-// the stored particles, cell.h:787-824).
-// push_body is the work of CTA `blk`; the single-universe kernel passes its
-// block index, the batched kernel the block index within its job.
-template <typename T>
-__device__ __forceinline__ void push_body(const Geom& g, const Pop<T>& P, int64_t blk, int mode) {
-    __shared__ int64_t s_start[kMaxCellsPerCta + 1];
-    __shared__ int s_count[kMaxCellsPerCta];
-    const int64_t base = blk * kSlotsPerCta;
-    // the cells this CTA's slots belong to (fixed between re-layouts)
-    const int2 cc = __ldg(P.cta_cells + blk);
-    const int c0 = cc.x, nc = cc.y;
-    for (int i = threadIdx.x; i <= nc; i += blockDim.x) s_start[i] = P.start[c0 + i];
-    for (int i = threadIdx.x; i < nc; i += blockDim.x) s_count[i] = P.count[c0 + i];
-    __syncthreads();
-
-    const int lane = threadIdx.x & 31;
-    const int64_t s0 = base + (int64_t)threadIdx.x * kVec;
-    int lc = 0;
-    {
-        int lo = 0, hi = nc - 1;
-        while (lo < hi) {
-            int mid = (lo + hi + 1) >> 1;
-            if (s_start[mid] <= s0) lo = mid; else hi = mid - 1;
-        }
-        lc = lo;
-    }
-    const int cell = c0 + lc;
-    int nv = 0;
-    if (s0 < P.capacity) {
-        int64_t e = s_start[lc] + s_count[lc] - s0;
-        nv = e <= 0 ? 0 : (e >= kVec ? kVec : (int)e);
-    }
-    int cx, cy, cz;
-    cell_coords(g, cell, cx, cy, cz);
-    const T qom = (T)P.qom;
-    const double q = P.q;
-
-    PState<T> ps[kVec];
-    if (nv > 0) {
-        if constexpr (std::is_same<T, float>::value) {
-            float4 X = *reinterpret_cast<const float4*>(P.x + s0), Y = *reinterpret_cast<const float4*>(P.y + s0),
-                   Z = *reinterpret_cast<const float4*>(P.z + s0), U = *reinterpret_cast<const float4*>(P.u + s0),
-                   V = *reinterpret_cast<const float4*>(P.v + s0), W = *reinterpret_cast<const float4*>(P.w + s0);
-            ps[0] = {X.x, Y.x, Z.x, U.x, V.x, W.x};
-            ps[1] = {X.y, Y.y, Z.y, U.y, V.y, W.y};
-            ps[2] = {X.z, Y.z, Z.z, U.z, V.z, W.z};
-            ps[3] = {X.w, Y.w, Z.w, U.w, V.w, W.w};
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                double2 X = *reinterpret_cast<const double2*>(P.x + s0 + 2 * h);
-                double2 Y = *reinterpret_cast<const double2*>(P.y + s0 + 2 * h);
-                double2 Z = *reinterpret_cast<const double2*>(P.z + s0 + 2 * h);
-                double2 U = *reinterpret_cast<const double2*>(P.u + s0 + 2 * h);
-                double2 V = *reinterpret_cast<const double2*>(P.v + s0 + 2 * h);
-                double2 W = *reinterpret_cast<const double2*>(P.w + s0 + 2 * h);
-                ps[2 * h] = {X.x, Y.x, Z.x, U.x, V.x, W.x};
-                ps[2 * h + 1] = {X.y, Y.y, Z.y, U.y, V.y, W.y};
-            }
-        }
-    }
-
-    const bool deposit = g.deposit != 0;
-    // per-thread node sums of its (up to 4) staying particles: FP32 for the
-    // FP32 path, FP64 otherwise; the node accumulation itself is FP64
-    T acc[32];
-#pragma unroll
-    for (int l = 0; l < 32; ++l) acc[l] = T(0);
-    bool has_acc = false;
-    int outc[kVec], dst[kVec];
-
-#pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-        outc[j] = -1;
-        dst[j] = cell;
-        if (j >= nv) continue;
-        int outcome = kStay, dest = cell;
-        if (mode == 0) outcome = step_particle(g, cx, cy, cz, qom, ps[j], dest);
-        outc[j] = outcome;
-        dst[j] = dest;
-        if (outcome == kStay && deposit) {
-            T rx, ry, rz;
-            frac_in_cell(g, cx, cy, cz, ps[j], rx, ry, rz);
-#pragma unroll
-            for (int corner = 0; corner < 8; ++corner) {
-                T fac = cic_weight<T>(corner, rx, ry, rz);
-                if constexpr (std::is_same<T, double>::value) {
-                    acc[corner * 4 + 0] += (q * ps[j].u) * fac;
-                    acc[corner * 4 + 1] += (q * ps[j].v) * fac;
-                    acc[corner * 4 + 2] += (q * ps[j].w) * fac;
-                    acc[corner * 4 + 3] += q * fac;
-                } else {
-                    const float qf = (float)q;
-                    acc[corner * 4 + 0] += qf * ps[j].u * fac;
-                    acc[corner * 4 + 1] += qf * ps[j].v * fac;
-                    acc[corner * 4 + 2] += qf * ps[j].w * fac;
-                    acc[corner * 4 + 3] += qf * fac;
-                }
-            }
-            has_acc = true;
-        }
-    }
-
-    // leavers -> outbox (one warp-aggregated append per vector lane), arrival
-    // lists of the destination cells, deposit relative to the destination
-    uint32_t nmig = 0, nrem = 0;
-#pragma unroll
-    for (int j = 0; j < kVec; ++j) {
-        const bool leave = outc[j] == kMove;
-        const uint32_t o = warp_append(&P.ctr->outbox, leave);
-        if (leave) {
-            Mover<T> m;
-            m.cell = dst[j];
-            m.id = P.id ? P.id[s0 + j] : 0u;
-            m.x = ps[j].x; m.y = ps[j].y; m.z = ps[j].z;
-            m.u = ps[j].u; m.v = ps[j].v; m.w = ps[j].w;
-            if (o < P.outbox_cap) {  // sized for one entry per slot: never full
-                P.outbox[o] = m;
-                register_arrival(P, o, m);
-            } else {
-                atomicAdd(&P.ctr->lost, 1u);
-            }
-            ++nmig;
-        }
-        if (outc[j] == kMove || outc[j] == kDrop) {
-            file_hole(P, cell, s_start[lc], s0 + j);
-            if (outc[j] == kDrop) ++nrem;
-        }
-    }
-    if (deposit) {
-#pragma unroll
-        for (int j = 0; j < kVec; ++j) warp_deposit_leavers<T>(g, outc[j] == kMove, dst[j], ps[j], q);
-    }
-    nmig = __reduce_add_sync(0xffffffffu, nmig);
-    nrem = __reduce_add_sync(0xffffffffu, nrem);
-    if (lane == 0) {
-        if (nmig) atomicAdd(&P.ctr->migrated, nmig);
-        if (nrem) atomicAdd(&P.ctr->removed, nrem);
-    }
-
-    // stayers: write the updated state back in place (vector stores)
-    if (mode == 0 && nv > 0) {
-        if constexpr (std::is_same<T, float>::value) {
-            *reinterpret_cast<float4*>(P.x + s0) = make_float4(ps[0].x, ps[1].x, ps[2].x, ps[3].x);
-            *reinterpret_cast<float4*>(P.y + s0) = make_float4(ps[0].y, ps[1].y, ps[2].y, ps[3].y);
-            *reinterpret_cast<float4*>(P.z + s0) = make_float4(ps[0].z, ps[1].z, ps[2].z, ps[3].z);
-            *reinterpret_cast<float4*>(P.u + s0) = make_float4(ps[0].u, ps[1].u, ps[2].u, ps[3].u);
-            *reinterpret_cast<float4*>(P.v + s0) = make_float4(ps[0].v, ps[1].v, ps[2].v, ps[3].v);
-            *reinterpret_cast<float4*>(P.w + s0) = make_float4(ps[0].w, ps[1].w, ps[2].w, ps[3].w);
-        } else {
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                *reinterpret_cast<double2*>(P.x + s0 + 2 * h) = make_double2(ps[2 * h].x, ps[2 * h + 1].x);
-                *reinterpret_cast<double2*>(P.y + s0 + 2 * h) = make_double2(ps[2 * h].y, ps[2 * h + 1].y);
-                *reinterpret_cast<double2*>(P.z + s0 + 2 * h) = make_double2(ps[2 * h].z, ps[2 * h + 1].z);
-                *reinterpret_cast<double2*>(P.u + s0 + 2 * h) = make_double2(ps[2 * h].u, ps[2 * h + 1].u);
-                *reinterpret_cast<double2*>(P.v + s0 + 2 * h) = make_double2(ps[2 * h].v, ps[2 * h + 1].v);
-                *reinterpret_cast<double2*>(P.w + s0 + 2 * h) = make_double2(ps[2 * h].w, ps[2 * h + 1].w);
-            }
-        }
-    }
-
-    // stayers' deposit: group lanes by cell, transpose-reduce the 32 node
-    // components, one FP64 atomic per lane and group
-    if (deposit) {
-        unsigned todo = __ballot_sync(0xffffffffu, has_acc);
-        while (todo) {
-            const int leader = __ffs(todo) - 1;
-            const int gcell = __shfl_sync(0xffffffffu, cell, leader);
-            const bool mine = has_acc && cell == gcell;
-            const unsigned grp = __ballot_sync(0xffffffffu, mine);
-            T v[32];
-#pragma unroll
-            for (int l = 0; l < 32; ++l) v[l] = mine ? acc[l] : T(0);
-            const double tot = (double)warp_transpose_sum<T>(v);
-            int gx, gy, gz;
-            cell_coords(g, gcell, gx, gy, gz);
-            node_atomic_add(g, gx, gy, gz, lane, tot);
-            todo &= ~grp;
-        }
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kPushThreads) k_push(Geom g, Pop<T> P, int mode) {
-    push_body<T>(g, P, blockIdx.x, mode);
-}
-
-// ---- particles that waited for a slot --------------------------------------
-// Entries t0, t0 + stride, ... of the pending list.
-template <typename T>
-__device__ __forceinline__ void push_pending_body(const Geom& g, const Pop<T>& P, uint32_t t0, uint32_t stride) {
-    const uint32_t n = *P.pending_in_count;
-    const double q = P.q;
-    for (uint32_t i = t0; i < n; i += stride) {
-        Mover<T> m = P.pending_in[i];
-        PState<T> p = {m.x, m.y, m.z, m.u, m.v, m.w};
-        int cx, cy, cz;
-        cell_coords(g, m.cell, cx, cy, cz);
-        int dest = m.cell;
-        int outcome = step_particle(g, cx, cy, cz, (T)P.qom, p, dest);
-        if (outcome == kDrop) {
-            atomicAdd(&P.ctr->removed, 1u);
-            continue;
-        }
-        if (outcome == kMove) atomicAdd(&P.ctr->migrated, 1u);
-        Mover<T> o = {dest, m.id, p.x, p.y, p.z, p.u, p.v, p.w};
-        uint32_t k = atomicAdd(&P.ctr->outbox, 1u);
-        if (k < P.outbox_cap) {
-            P.outbox[k] = o;
-            register_arrival(P, k, o);
-        } else {
-            atomicAdd(&P.ctr->lost, 1u);
-        }
-        if (g.deposit) deposit_one<T>(g, dest, p, q);
-    }
-}
-
-template <typename T>
-__global__ void k_push_pending(Geom g, const __grid_constant__ PopSet<T> S) {
-    push_pending_body<T>(g, S.p[blockIdx.y], blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 // ---- injection at the x = 0 face (not in the reference) ---------------------

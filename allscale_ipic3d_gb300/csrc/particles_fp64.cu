@@ -1,16 +1,75 @@
-// FP64 particle kernels: absolute positions, the reference's arithmetic
-// order. Built with -fmad=false: no product-sum is fused, as on the
-// reference's x86 build (explicit __fma_rn calls stay fused on purpose).
+// FP64 particle kernels: absolute positions. Built with -fmad=false: the
+// dipole mover, the export test and the element kernel round as the
+// reference's x86 build does; the field mover and the deposit (push64.cuh)
+// fuse their products explicitly (__fma_rn).
+#include <algorithm>
+
 #include "particles_impl.cuh"
+#include "push64.cuh"
 
 namespace ipg {
+
+namespace {
+// How a launch over `slots` slots in `tiles` tiles is cut: particles per
+// work item, tiles per block, blocks per span. About 4 warps per
+// sub-partition (152 SMs x 4) keep the FP64 pipe busy; an item costs its
+// group about 70 FP64 instructions beside 150 per 8 particles, so items are
+// as long as that allows. Spans of 4 tiles leave fewer warps part-filled
+// where there are blocks enough.
+struct Shape64 {
+    int item, span, parts;
+};
+Shape64 shape64(int64_t slots, int64_t tiles) {
+    constexpr int64_t kSms = 152, kGroups = kSms * 4 * 4 * (32 / kGroup64);
+    Shape64 s{256, 1, 1};
+    while (s.item > 16 && slots < s.item * kGroups) s.item /= 2;
+    if (tiles >= kMaxSpan64 * kSms * 6) s.span = kMaxSpan64;
+    const int64_t most = std::max<int64_t>(1, kSlotsPerCta / (s.item * kItems64));
+    s.parts = (int)std::max<int64_t>(1, std::min(most, (4 * kSms + tiles - 1) / std::max<int64_t>(1, tiles)));
+    return s;
+}
+
+Push64Set push64_set(const Geom& g, const PopSet<double>& S) {
+    Push64Set pcs{};
+    for (int i = 0; i < S.n; ++i) pcs.c[i] = push64_const(g, S.p[i]);
+    return pcs;
+}
+}  // namespace
+
+Push64Const push64_const(const Geom& g, const Pop<double>& P) {
+    Push64Const c;
+    c.d = dipole_species(g.mft, P.qom, g.dt, g.inv_pic);
+    c.k1 = P.qom * 0.5 * g.dt;
+    c.field_scale = (g.flags & 2u /*IPIC3D_F_GATHER_DIV_VOL*/) ? 1.0 / g.vol : 1.0;
+    return c;
+}
+
 template <>
 int launch_push<double>(const Geom& g, const PopSet<double>& S, int mode, const PushShape&, cudaStream_t st) {
-    return launch_push_generic<double>(g, S, mode, st);
+    int64_t tiles = 0, most = 0, slots = 0;
+    for (int i = 0; i < S.n; ++i) {
+        const int64_t t = (S.p[i].capacity + kSlotsPerCta - 1) / kSlotsPerCta;
+        tiles += t;
+        most = std::max(most, t);
+        slots += S.p[i].capacity;
+    }
+    if (most <= 0 || (mode != 0 && !g.deposit)) return 0;
+    const Shape64 sh = shape64(slots, tiles);
+    const dim3 grid((unsigned)((most + sh.span - 1) / sh.span), sh.parts, S.n);
+    const Push64Set pcs = push64_set(g, S);
+    auto run = [&](auto k) { k<<<grid, kThreads64, 0, st>>>(g, S, pcs, sh.span, sh.item); };
+    if (mode != 0) run(k_push64<false, false, true>);
+    else if (g.mover == 1 && g.deposit) run(k_push64<true, true, true>);
+    else if (g.mover == 1) run(k_push64<true, true, false>);
+    else if (g.deposit) run(k_push64<true, false, true>);
+    else run(k_push64<true, false, false>);
+    return 1;
 }
 template <>
 int launch_push_pending<double>(const Geom& g, const PopSet<double>& S, cudaStream_t st) {
-    return launch_push_pending_generic<double>(g, S, st);
+    if (S.n <= 0) return 0;
+    k_push_pending64<<<dim3(152, S.n), 128, 0, st>>>(g, S, push64_set(g, S));
+    return 1;
 }
 template int launch_inject<double>(const Geom&, const Pop<double>&, double, const double*, const double*, uint64_t,
                                    const uint64_t*, cudaStream_t);
@@ -21,12 +80,22 @@ template int launch_pending_count<double>(const Pop<double>&, int32_t*, cudaStre
 
 template <>
 int launch_push_batch<double>(const PopJob<double>* jobs, const int2* cta_job, int64_t nctas, int mode,
-                              const Geom&, const PushShape&, cudaStream_t st) {
-    return launch_push_batch_generic<double>(jobs, cta_job, nctas, mode, st);
+                              const Geom& g, const PushShape&, cudaStream_t st) {
+    if (nctas <= 0 || (mode != 0 && !g.deposit)) return 0;
+    const Shape64 sh = shape64(nctas * kSlotsPerCta, nctas);
+    const dim3 grid((unsigned)nctas, sh.parts);
+    auto run = [&](auto k) { k<<<grid, kThreads64, 0, st>>>(jobs, cta_job, sh.span, sh.item); };
+    if (mode != 0) run(k_push64_batch<false, false, true>);
+    else if (g.mover == 1 && g.deposit) run(k_push64_batch<true, true, true>);
+    else if (g.mover == 1) run(k_push64_batch<true, true, false>);
+    else if (g.deposit) run(k_push64_batch<true, false, true>);
+    else run(k_push64_batch<true, false, false>);
+    return 1;
 }
 template <>
 int launch_push_pending_batch<double>(const PopJob<double>* jobs, int njobs, cudaStream_t st) {
-    return launch_push_pending_batch_generic<double>(jobs, njobs, st);
+    k_push_pending64_batch<<<dim3(2, njobs), 128, 0, st>>>(jobs);
+    return 1;
 }
 template int launch_place_batch<double>(const PopJob<double>*, const int2*, int64_t, cudaStream_t);
 template int launch_pending_rotate_batch<double>(const PopJob<double>*, int, cudaStream_t);

@@ -7,27 +7,6 @@
 
 namespace ipg {
 
-// generic versions (the FP64 path); particles_fp32.cu specialises both
-template <typename T>
-int launch_push_generic(const Geom& g, const PopSet<T>& S, int mode, cudaStream_t st) {
-    int n = 0;
-    for (int i = 0; i < S.n; ++i) {
-        const Pop<T>& P = S.p[i];
-        if (P.capacity <= 0) continue;
-        const int64_t blocks = (P.capacity + kSlotsPerCta - 1) / kSlotsPerCta;
-        k_push<T><<<(unsigned)blocks, kPushThreads, 0, st>>>(g, P, mode);
-        ++n;
-    }
-    return n;
-}
-
-template <typename T>
-int launch_push_pending_generic(const Geom& g, const PopSet<T>& S, cudaStream_t st) {
-    if (S.n <= 0) return 0;
-    k_push_pending<T><<<dim3(152, S.n), 128, 0, st>>>(g, S);
-    return 1;
-}
-
 template <typename T>
 int launch_inject(const Geom& g, const Pop<T>& P, double per_cell, const double drift[3], const double vth[3],
                   uint64_t seed, const uint64_t* d_step, cudaStream_t st) {
@@ -82,23 +61,6 @@ int launch_pending_count(const Pop<T>& P, int32_t* per_cell, cudaStream_t st) {
 }
 
 // ---- batched ensemble ------------------------------------------------------
-// cta_job[b] = (job, CTA of the job) for the push, blk_job[b] = (job, first
-// cell) for the placement (8 cells of one job per 256-thread block).
-template <typename T>
-__global__ void __launch_bounds__(kPushThreads) k_push_batch(const PopJob<T>* __restrict__ jobs,
-                                                             const int2* __restrict__ cta_job, int mode) {
-    __shared__ PopJob<T> job;
-    const int2 cj = __ldg(cta_job + blockIdx.x);
-    load_job(job, jobs + cj.x);
-    push_body<T>(job.g, job.P, cj.y, mode);
-}
-
-template <typename T>
-__global__ void k_push_pending_batch(const PopJob<T>* __restrict__ jobs) {
-    const PopJob<T>& J = jobs[blockIdx.y];
-    push_pending_body<T>(J.g, J.P, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-}
-
 // Placement of a batch: blockIdx.y = job, the job's warps stride over its
 // dirty-cell list (cells with holes or arrivals only).
 // Batched dirty lists: block b lists the flagged cells of the 512-cell
@@ -182,22 +144,6 @@ __global__ void k_batch_status(const PopJob<T>* __restrict__ jobs, int njobs, Jo
     s.pending_in = *jobs[j].pend_count;
     s.pad = 0;
     out[j] = s;
-}
-
-template <typename T>
-int launch_push_batch_generic(const PopJob<T>* jobs, const int2* cta_job, int64_t nctas, int mode, cudaStream_t st) {
-    if (nctas <= 0) return 0;
-    k_push_batch<T><<<(unsigned)nctas, kPushThreads, 0, st>>>(jobs, cta_job, mode);
-    return 1;
-}
-
-template <typename T>
-int launch_push_pending_batch(const PopJob<T>* jobs, int njobs, cudaStream_t st);
-
-template <typename T>
-int launch_push_pending_batch_generic(const PopJob<T>* jobs, int njobs, cudaStream_t st) {
-    k_push_pending_batch<T><<<dim3(2, njobs), 128, 0, st>>>(jobs);
-    return 1;
 }
 
 template <typename T>
