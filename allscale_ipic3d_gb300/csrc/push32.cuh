@@ -77,7 +77,7 @@ __device__ __forceinline__ CellInfo cell_info(const Geom& g, const Push32Const& 
     return c;
 }
 
-// The CellInfo of lane `src` (warp-wide).
+// The CellInfo of lane `src` (every lane of the warp its own).
 __device__ __forceinline__ CellInfo shfl_cell_info(const CellInfo& c, int src) {
     CellInfo r;
     r.ox = __shfl_sync(0xffffffffu, c.ox, src);

@@ -534,10 +534,94 @@ __device__ __forceinline__ float run_transpose_sum(const float (&acc)[32], bool 
     return v[0];
 }
 
+// Slot mode's flush where no run of lanes of one cell is longer than 8 (cells
+// of at most 32 slots: the sparse tiles), all runs of the warp together: the
+// lanes at distance 4, then 2, then 1 of each run are added (the order in
+// which run_transpose_sum meets them: the same sums bit for bit), which
+// leaves 16 of the 32 moments in each of a run's first two lanes; these take
+// the corner butterflies in registers and pass the corner sums through shared
+// memory, so that a run still costs one 32-lane atomic. About 350 warp
+// instructions for the 8 or so runs of a warp where a transpose-reduction
+// and butterflies per run take about 150 each.
+constexpr int kShortRun = 8;
+constexpr int kRunRow = 36;                     // 32 corner sums, padded: two lanes write a row
+constexpr int kRunRows = 5;                     // rows of the warp's buffer
+constexpr int kRunBuffer = kRunRow * kRunRows;  // floats; in the stage's coefficient space, unused in slot mode
+static_assert(kSlotWarps * kRunBuffer <= kItemMaxCells * 48 && kRunRow % 4 == 0, "the buffers fit, 16-byte rows");
+
+__device__ __forceinline__ void flush_short_runs(const Geom& g, const Push32Const& pc, float (&acc)[32], int count,
+                                                 int cell, int pos, int run_len, int longest, float* buffer,
+                                                 double q) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    if (longest > 4) {
+        const bool in = pos + 4 < run_len;
+#pragma unroll
+        for (int l = 0; l < 32; ++l) {
+            const float t = __shfl_down_sync(kAll, acc[l], 4);
+            if (in) acc[l] += t;
+        }
+        const int t = __shfl_down_sync(kAll, count, 4);
+        if (in) count += t;
+    }
+    if (longest > 2) {
+        const bool in = pos + 2 < run_len;
+#pragma unroll
+        for (int l = 0; l < 32; ++l) {
+            const float t = __shfl_down_sync(kAll, acc[l], 2);
+            if (in) acc[l] += t;
+        }
+        const int t = __shfl_down_sync(kAll, count, 2);
+        if (in) count += t;
+    }
+    // runs start at even lanes (cells at multiples of 8 slots)
+    const bool odd = (lane & 1) != 0;
+    float v[16];
+#pragma unroll
+    for (int l = 0; l < 16; ++l) {
+        const float send = odd ? acc[l] : acc[l + 16];
+        const float keep = odd ? acc[l + 16] : acc[l];
+        v[l] = keep + __shfl_xor_sync(kAll, send, 1);
+    }
+    count += __shfl_xor_sync(kAll, count, 1);
+    if (odd) v[8] = (float)count;  // moment 24: the stayers
+#pragma unroll
+    for (int o = 0; o < 16; o += 8)
+#pragma unroll
+        for (int bit = 1; bit < 8; bit <<= 1)
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+                if (!(m & bit)) {
+                    const float lo = v[o + m], hi = v[o + (m | bit)];
+                    v[o + m] = fmaf(0.5f, lo, -hi);
+                    v[o + (m | bit)] = fmaf(0.5f, lo, hi);
+                }
+    unsigned runs = __ballot_sync(kAll, pos == 0 && count > 0);
+    const int rank = __popc(runs & ((1u << (lane & ~1)) - 1u));
+    const bool writes = pos < 2 && count > 0;
+    for (int first = 0; runs; first += kRunRows) {
+        __syncwarp();
+        if (writes && rank >= first && rank < first + kRunRows) {
+            float4* row = reinterpret_cast<float4*>(buffer + (rank - first) * kRunRow + (odd ? 16 : 0));
+#pragma unroll
+            for (int k = 0; k < 4; ++k) row[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        }
+        __syncwarp();
+        for (int r = 0; r < kRunRows && runs; ++r) {
+            const int ra = __ffs(runs) - 1;
+            runs &= runs - 1;
+            const float s = buffer[r * kRunRow + lane];
+            const int3 c = cell_xyz(g, pc, __shfl_sync(kAll, cell, ra));
+            if (s != 0.f) corner_atomic_add(g, c.x, c.y, c.z, lane & 7, lane >> 3, (double)s * q);
+        }
+    }
+}
+
 // Slot mode: slice w of the tile (slots [128 w, 128 w + 128)) is pushed by
-// one warp, thread t of the slice the 4 slots from 4 t (one cell:
-// capacities are multiples of 8), in two passes as in item mode (move, then
-// moments of the stayers), and flushed per run of lanes of one cell.
+// one warp in two passes as in item mode: the move, over the slice's
+// occupied slots in rounds of 32; then the moments of the stayers, thread t
+// the 4 slots from 4 t (one cell: capacities are multiples of 8), and flushed per run of lanes of one cell, short
+// runs together.
 template <int kF>
 __device__ __forceinline__ void push_slots(const Geom& g, const Pop<float>& P, const Push32Const& pc,
                                            const Push32Const& sp, PipeStage& st, int base, int2 desc, int slice,
@@ -565,29 +649,47 @@ __device__ __forceinline__ void push_slots(const Geom& g, const Pop<float>& P, c
         const int e = cstart + N[lc] - s0;
         nv = e <= 0 ? 0 : (e >= kPer ? kPer : e);
     }
-    const CellInfo ci = cell_info(g, pc, cell);
     const int sl0 = tid * kPer;
     int nst = nv;  // this thread's stayers
     if (kStep) {
-        const float* coef = g.cellcoef + (size_t)cell * 48;
-        // lane groups start at different slots of their run of 4: the words a
-        // warp reads in one step fall in 32 different banks
-        const int rot = lane >> 3;
+        const CellInfo ci0 = cell_info(g, pc, cell);
+        // the slice's occupied slots, listed (bytes: lane << 2 | slot): rounds
+        // of 32 particles whatever the slots' occupancy, the cell's data
+        // from the lane that owns the slot
+        uint8_t* const list = reinterpret_cast<uint8_t*>(st.coef + slice * kRunBuffer);
+        int upto = nv;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= o) upto += t;
+        }
+        const int total = __shfl_sync(0xffffffffu, upto, 31);
+#pragma unroll
+        for (int j = 0; j < kPer; ++j)
+            if (j < nv) list[upto - nv + j] = (uint8_t)(lane * kPer + j);
+        __syncwarp();
 #pragma unroll 1
-        for (int jj = 0; jj < kPer; ++jj) {
-            const int j = (jj + rot) & (kPer - 1);
-            const int sl = sl0 + j;
-            PState<float> p;
+        for (int k0 = 0; k0 < total; k0 += 32) {
+            const bool has = k0 + lane < total;
+            const int at = has ? list[k0 + lane] : 0;
+            const int owner = at >> 2;
+            const int sl = slice * 128 + at;
+            const int pcell = __shfl_sync(0xffffffffu, cell, owner);
+            const int pstart = __shfl_sync(0xffffffffu, cstart, owner);
+            const CellInfo ci = shfl_cell_info(ci0, owner);
+            PState<float> p = load_slot(st, sl);
             int outcome = -1, dir = 0;
-            if (j < nv) {
-                p = load_slot(st, sl);
-                outcome = step32f<false, (kF & kPipeGather) != 0, (kF & kPipeDipole) != 0>(g, pc, sp, coef, ci, p,
-                                                                                           dir);
+            if (has) {
+                outcome = step32f<false, (kF & kPipeGather) != 0, (kF & kPipeDipole) != 0>(
+                    g, pc, sp, g.cellcoef + (size_t)pcell * 48, ci, p, dir);
                 if (outcome == kStay) store_slot(st, sl, p);
                 else if (kDep) clear_slot(st, sl);
             }
-            if (outcome > 0) --nst;
-            leave_and_hole<false>(g, P, pc, outcome, dir, p, base + sl, cell, cstart, kDep, nmig, nrem);
+            unsigned gone = __ballot_sync(0xffffffffu, outcome > 0);
+            if (!gone) continue;
+            leave_and_hole<false>(g, P, pc, outcome, dir, p, base + sl, pcell, pstart, kDep, nmig, nrem);
+            for (; gone; gone &= gone - 1)
+                nst -= __shfl_sync(0xffffffffu, owner, __ffs(gone) - 1) == lane;
         }
         __syncwarp();
     }
@@ -597,9 +699,19 @@ __device__ __forceinline__ void push_slots(const Geom& g, const Pop<float>& P, c
     for (int l = 0; l < 32; ++l) acc[l] = 0.f;
 #pragma unroll 1
     for (int j = 0; j < nv; ++j) add_moments(acc, load_slot(st, sl0 + j));
-    const unsigned todo = __ballot_sync(0xffffffffu, nst > 0);
     const int prev_cell = __shfl_up_sync(0xffffffffu, cell, 1);
     unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev_cell != cell);
+    const unsigned upto = 0xffffffffu >> (31 - lane);
+    const int head = 31 - __clz(heads & upto);
+    const unsigned after = heads & ~upto;
+    const int run_len = (after ? __ffs(after) - 1 : 32) - head;
+    const int longest = __reduce_max_sync(0xffffffffu, run_len);
+    if (longest <= kShortRun) {
+        // the usual sparse tile: every run at once
+        flush_short_runs(g, pc, acc, nst, cell, lane - head, run_len, longest, st.coef + slice * kRunBuffer, P.q);
+        return;
+    }
+    const unsigned todo = __ballot_sync(0xffffffffu, nst > 0);
     while (heads) {
         const int ra = __ffs(heads) - 1;
         heads &= heads - 1;
@@ -682,9 +794,15 @@ __device__ __forceinline__ bool push_tile_warp(const Geom& g, const Pop<float>& 
     first = __shfl_sync(0xffffffffu, first, 0);
     if (nc > shp.item_cells) {
         if (first && lane == 0) mbar_arrive(td.ready);
-        for (int w = threadIdx.x >> 5; w < kSlotWarps; w += kComputeWarps)
+        // slices are claimed like items: 8 slices for 11 warps, the others
+        // go on to the next stage's
+        for (;;) {
+            int w = 0;
+            if (lane == 0) w = atomicAdd(next_item, 1);
+            w = __shfl_sync(0xffffffffu, w, 0);
+            if (w >= kSlotWarps) return true;
             push_slots<kF>(g, P, pc, sp, st, base, desc, w, nmig, nrem);
-        return true;
+        }
     }
     const int sh = 31 - __clz(shp.item);  // items of 2^sh particles
     if (first) {
