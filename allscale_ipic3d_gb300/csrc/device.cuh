@@ -33,6 +33,7 @@ struct Geom {
     int sx, sy, sz;
     int ncells;
     double w[3], inv_w[3], half_w[3];
+    int exact_inv[3];       // w is a power of two: the product with inv_w is the quotient
     double origin[3];
     double object_center[3];
     double L[3];            // domain length per axis

@@ -507,15 +507,7 @@ int scatter_pops(ipic3d_ctx* ctx, std::vector<PopStore<T>>& pops, const std::vec
         CU(cudaMemsetAsync(P.pending_in_count, 0, sizeof(uint32_t), st));
         CU(cudaMemsetAsync(P.ctr, 0, sizeof(StepCounters), st));
     }
-    UploadGeom g;
-    g.ncells = (int)nc;
-    g.sx = (int)ctx->props.size[0];
-    g.sy = (int)ctx->props.size[1];
-    g.sz = (int)ctx->props.size[2];
-    for (int a = 0; a < 3; ++a) {
-        g.origin[a] = ctx->props.origin[a];
-        g.w[a] = ctx->props.cell_width[a];
-    }
+    const UploadGeom g = upload_geom(ctx->props);
     int nl = launch_scatter<T>(ctx->st_parts, have_ids ? ctx->st_ids : nullptr, ctx->st_sid, ctx->st_off, U, g,
                                ctx->stream);
     (void)n;
@@ -587,15 +579,7 @@ int upload_fast(ipic3d_ctx* ctx, std::vector<PopStore<T>>& pops, const ipic3d_pa
         sp.q[k] = pops[k].q;
         sp.qom[k] = pops[k].qom;
     }
-    UploadGeom g;
-    g.ncells = (int)nc;
-    g.sx = (int)ctx->props.size[0];
-    g.sy = (int)ctx->props.size[1];
-    g.sz = (int)ctx->props.size[2];
-    for (int a = 0; a < 3; ++a) {
-        g.origin[a] = ctx->props.origin[a];
-        g.w[a] = ctx->props.cell_width[a];
-    }
+    const UploadGeom g = upload_geom(ctx->props);
     // chunks of about 16 MB of records, cut at cell boundaries (the last
     // chunk's kernel runs after the last copy: small chunks keep that short)
     const int64_t chunk = on_device ? std::max<int64_t>(1, n)
@@ -944,15 +928,7 @@ int download_device(ipic3d_ctx* ctx, std::vector<PopStore<T>>& pops, ipic3d_part
     }
     P.dst = ctx->st_dst;
     P.positions_only = xyz ? 1 : 0;
-    UploadGeom g;
-    g.ncells = (int)nc;
-    g.sx = (int)ctx->props.size[0];
-    g.sy = (int)ctx->props.size[1];
-    g.sz = (int)ctx->props.size[2];
-    for (int a = 0; a < 3; ++a) {
-        g.origin[a] = ctx->props.origin[a];
-        g.w[a] = ctx->props.cell_width[a];
-    }
+    const UploadGeom g = upload_geom(ctx->props);
     // chunks of about 64 MB of records, cut at cell boundaries: few enough
     // that enqueueing them (a pack kernel, an event and a copy each) costs
     // little host time, which otherwise delays the caller's next upload
@@ -1062,6 +1038,7 @@ void refresh_geom(ipic3d_ctx* ctx) {
     for (int a = 0; a < 3; ++a) {
         g.w[a] = p.cell_width[a];
         g.inv_w[a] = 1.0 / p.cell_width[a];
+        g.exact_inv[a] = soft::power_of_two(p.cell_width[a]);
         g.half_w[a] = p.cell_width[a] / 2.0;
         g.origin[a] = p.origin[a];
         g.object_center[a] = p.object_center[a];

@@ -163,9 +163,9 @@ template <typename T>
 __device__ __forceinline__ void frac_in_cell(const Geom& g, int cx, int cy, int cz, const PState<T>& p, T& rx, T& ry,
                                              T& rz) {
     if constexpr (std::is_same<T, double>::value) {
-        rx = (p.x - (g.origin[0] + (double)cx * g.w[0])) / g.w[0];
-        ry = (p.y - (g.origin[1] + (double)cy * g.w[1])) / g.w[1];
-        rz = (p.z - (g.origin[2] + (double)cz * g.w[2])) / g.w[2];
+        rx = soft::quotient(p.x - (g.origin[0] + (double)cx * g.w[0]), g.w[0], g.inv_w[0], g.exact_inv[0]);
+        ry = soft::quotient(p.y - (g.origin[1] + (double)cy * g.w[1]), g.w[1], g.inv_w[1], g.exact_inv[1]);
+        rz = soft::quotient(p.z - (g.origin[2] + (double)cz * g.w[2]), g.w[2], g.inv_w[2], g.exact_inv[2]);
     } else {
         rx = p.x; ry = p.y; rz = p.z;
     }

@@ -5,6 +5,9 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "../../include/ipic3d_types.h"
+#include "fp64_int.cuh"
+
 namespace ipg {
 
 constexpr int kUploadMaxPops = 16;
@@ -17,7 +20,23 @@ struct SpeciesTable {
 struct UploadGeom {
     int ncells, sx, sy, sz;
     double origin[3], w[3];
+    double inv_w[3];   // 1 / w
+    int exact_inv[3];  // w is a power of two: the product with inv_w is the quotient
 };
+inline UploadGeom upload_geom(const ipic3d_props& p) {
+    UploadGeom g;
+    g.sx = (int)p.size[0];
+    g.sy = (int)p.size[1];
+    g.sz = (int)p.size[2];
+    g.ncells = (int)(p.size[0] * p.size[1] * p.size[2]);
+    for (int a = 0; a < 3; ++a) {
+        g.origin[a] = p.origin[a];
+        g.w[a] = p.cell_width[a];
+        g.inv_w[a] = 1.0 / p.cell_width[a];
+        g.exact_inv[a] = soft::power_of_two(p.cell_width[a]);
+    }
+    return g;
+}
 
 template <typename T>
 struct UploadPops {

@@ -4,7 +4,7 @@
 // by the exact value times 1 + e, e over the instructions' error bounds.
 // Reads quadruples of doubles (a, b, c, err in [-1, 1]) from argv[1] and
 // writes per quadruple: the number of operations that differ from FP64
-// (product, square, triple, sum of magnitudes, quotient), pow25(|a|) and
+// (product, square, triple, sum of magnitudes, quotients), pow25(|a|) and
 // whether it is sure.
 #include <cmath>
 #include <cstdint>
@@ -41,6 +41,10 @@ int main(int argc, char** argv) {
         bad += pack(div(A, divisor(B))) != a / b;
         bad += pack(div(mul(A, C), divisor(add_positive(B, C)))) != (a * c) / (std::fabs(b) + std::fabs(c));
         bad += std::signbit(pack(div(A, divisor(B)))) != std::signbit(a / b);
+        const double w = std::fabs(b) * std::ldexp(1.0, 1023 - exponent_of(b) + (exponent_of(c) % 90));
+        bad += quotient(a, w, 1.0 / w, power_of_two(w)) != a / w;
+        bad += quotient(a, 0.125, 8.0, power_of_two(0.125)) != a / 0.125;
+        bad += std::signbit(quotient(-0.0, w, 1.0 / w, 0)) != std::signbit(-0.0 / w);
         bool sure = false;
         const double p = pack(pow25(unpack(std::fabs(a)), sure));
         const double out[3] = {bad, p, sure ? 1.0 : 0.0};
