@@ -26,6 +26,18 @@ constexpr int kPushThreads = 256;       // threads per CTA of the push kernel
 constexpr int kSlotsPerCta = kVec * kPushThreads;
 constexpr int kSetPops = 4;             // populations per launch of the population-set kernels
 constexpr int kSlotAlign = 8;          // start[] and every cell's capacity are multiples of 8
+constexpr int kPlaceThreads = 128;
+// Cells a warp of the placement looks after: 8, or fewer where that would
+// leave SMs without warps (about 32 per SM).
+__host__ __device__ inline int place_cells_per_warp(int64_t ncells) {
+    return ncells >= 8 * 152 * 32 ? 8 : ncells >= 4 * 152 * 32 ? 4 : ncells >= 2 * 152 * 32 ? 2 : 1;
+}
+constexpr int kPlaceBatchCells = 8;  // batched placement
+// blocks of the placement of `ncells` cells, `cells` per warp
+__host__ __device__ inline int place_blocks(int64_t ncells, int cells) {
+    const int64_t per = (int64_t)cells * (kPlaceThreads / 32);
+    return (int)((ncells + per - 1) / per);
+}
 constexpr int kMaxCellsPerCta = kSlotsPerCta / kSlotAlign + 2;
 
 // Geometry and physics of one universe (UniverseProperties plus the policy).
@@ -56,7 +68,7 @@ struct Geom {
 
 // A particle that leaves its slot (migration) or waits for a slot (pending).
 template <typename T>
-struct Mover {
+struct alignas(sizeof(T) == 4 ? 16 : 8) Mover {  // FP32: two 16-byte accesses
     int32_t cell;           // destination cell (for pending: the cell it is in)
     uint32_t id;
     T x, y, z, u, v, w;
@@ -70,7 +82,6 @@ struct StepCounters {
     uint32_t removed;       // particles removed (planet, open faces)
     uint32_t migrated;      // particles that changed cell
     uint32_t injected;
-    uint32_t dirty;         // cells with holes or arrivals this step (entries of dirty_list)
     uint32_t lost;          // pending list overflow (must stay 0)
     uint32_t timeouts;      // CTAs that gave up a bounded wait (must stay 0)
 };
@@ -86,8 +97,6 @@ struct Pop {
     int32_t* hole_list;     // [capacity] holes of cell c at start[c] + k
     int32_t* arr_cnt;       // [ncells]
     int32_t* arr_list;      // [capacity] arrivals of cell c at start[c] + k (outbox index)
-    int32_t* dirty_flag;    // [ncells] 1 while the cell is on this step's dirty list
-    int32_t* dirty_list;    // [ncells] cells with holes or arrivals (the placement's work list)
     Mover<T>* outbox;
     uint32_t outbox_cap;
     Mover<T>* pending_in;   // pushed this step
@@ -246,29 +255,16 @@ __device__ __forceinline__ int fast_div(int a, int d, float inv_d) {
     return q;
 }
 
-// Flags cell c as touched this step (holes or arrivals): a plain store, no
-// round trip; k_dirty_compact lists the flagged cells for the placement,
-// which clears the flag.
-template <typename T>
-__device__ __forceinline__ void mark_dirty(const Pop<T>& P, int c) {
-    P.dirty_flag[c] = 1;
-}
-
 // Files slot `slot` as a hole of cell c (its slots start at cstart).
 template <typename T>
 __device__ __forceinline__ void file_hole(const Pop<T>& P, int c, int64_t cstart, int64_t slot) {
     const int k = atomicAdd(P.hole_cnt + c, 1);
     P.hole_list[cstart + k] = (int32_t)slot;
-    mark_dirty(P, c);
 }
 
 // t = (a * n1 + b) * n2 + c for t in [0, n0 * n1 * n2): 32-bit divisions
 // when t fits (64-bit division by a runtime divisor is a long software
 // sequence on the GPU).
-// Blocks of the batched placement for a universe of `ncells` cells: one per
-// 512 cells (256 threads, a cell per 8 lanes: 32 cells at a time).
-__host__ __device__ inline int place_blocks(int ncells) { return ncells > 0 ? (ncells + 511) / 512 : 1; }
-
 __device__ __forceinline__ void split3(int64_t t, int n1, int n2, int& a, int& b, int& c) {
     if (t < 0x7fffffff) {
         const unsigned u = (unsigned)t, r = u / (unsigned)n2;

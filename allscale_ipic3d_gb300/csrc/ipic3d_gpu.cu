@@ -73,7 +73,6 @@ struct PopStore {
     int2* cta_cells = nullptr;
     int32_t *count = nullptr, *hole_cnt = nullptr, *arr_cnt = nullptr;
     int32_t *hole_list = nullptr, *arr_list = nullptr, *sort_tmp = nullptr;
-    int32_t *dirty_flag = nullptr, *dirty_list = nullptr;
     Mover<T>*outbox = nullptr, *pending_in = nullptr, *pending_out = nullptr;
     uint32_t* pending_in_count = nullptr;
     StepCounters* ctr = nullptr;
@@ -82,7 +81,7 @@ struct PopStore {
     void release() {
         dfree(x); dfree(y); dfree(z); dfree(u); dfree(v); dfree(w); dfree(id);
         dfree(start); dfree(cta_cells); dfree(count); dfree(hole_cnt); dfree(arr_cnt);
-        dfree(hole_list); dfree(arr_list); dfree(sort_tmp); dfree(dirty_flag); dfree(dirty_list);
+        dfree(hole_list); dfree(arr_list); dfree(sort_tmp);
         dfree(outbox); dfree(pending_in); dfree(pending_out);
         dfree(pending_in_count); dfree(ctr);
         capacity = 0;
@@ -98,8 +97,6 @@ struct PopStore {
         P.hole_list = hole_list;
         P.arr_cnt = arr_cnt;
         P.arr_list = arr_list;
-        P.dirty_flag = dirty_flag;
-        P.dirty_list = dirty_list;
         P.outbox = outbox;
         P.outbox_cap = outbox_cap;
         P.pending_in = pending_in;
@@ -313,9 +310,6 @@ int alloc_pop(ipic3d_ctx* ctx, PopStore<T>& P, const std::vector<uint64_t>& coun
     CU(cudaMalloc(&P.hole_list, cap * sizeof(int32_t)));
     CU(cudaMalloc(&P.arr_list, cap * sizeof(int32_t)));
     CU(cudaMalloc(&P.sort_tmp, cap * sizeof(int32_t)));
-    CU(cudaMalloc(&P.dirty_flag, nc * sizeof(int32_t)));
-    CU(cudaMalloc(&P.dirty_list, nc * sizeof(int32_t)));
-    CU(cudaMemsetAsync(P.dirty_flag, 0, nc * sizeof(int32_t), ctx->stream));
     CU(cudaMalloc(&P.outbox, (size_t)P.outbox_cap * sizeof(Mover<T>)));
     CU(cudaMalloc(&P.pending_in, (size_t)P.pending_cap * sizeof(Mover<T>)));
     CU(cudaMalloc(&P.pending_out, (size_t)P.pending_cap * sizeof(Mover<T>)));
@@ -503,7 +497,6 @@ int scatter_pops(ipic3d_ctx* ctx, std::vector<PopStore<T>>& pops, const std::vec
         cudaStream_t st = ctx->stream;
         CU(cudaMemsetAsync(P.hole_cnt, 0, nc * sizeof(int32_t), st));
         CU(cudaMemsetAsync(P.arr_cnt, 0, nc * sizeof(int32_t), st));
-        CU(cudaMemsetAsync(P.dirty_flag, 0, nc * sizeof(int32_t), st));
         CU(cudaMemsetAsync(P.pending_in_count, 0, sizeof(uint32_t), st));
         CU(cudaMemsetAsync(P.ctr, 0, sizeof(StepCounters), st));
     }
@@ -557,7 +550,6 @@ int upload_fast(ipic3d_ctx* ctx, std::vector<PopStore<T>>& pops, const ipic3d_pa
         U.count[k] = P.count;
         CU(cudaMemsetAsync(P.hole_cnt, 0, nc * sizeof(int32_t), st));
         CU(cudaMemsetAsync(P.arr_cnt, 0, nc * sizeof(int32_t), st));
-        CU(cudaMemsetAsync(P.dirty_flag, 0, nc * sizeof(int32_t), st));
         CU(cudaMemsetAsync(P.pending_in_count, 0, sizeof(uint32_t), st));
         CU(cudaMemsetAsync(P.ctr, 0, sizeof(StepCounters), st));
     }
@@ -2113,7 +2105,7 @@ int batch_tables(ipic3d_batch* b) {
     for (size_t j = 0; j < nj.size(); ++j) {
         const int64_t nb = (nj[j].P.capacity + kSlotsPerCta - 1) / kSlotsPerCta;
         for (int64_t k = 0; k < nb; ++k) cta.push_back(make_int2((int)j, (int)k));
-        const int npb = place_blocks(nj[j].g.ncells);
+        const int npb = place_blocks(nj[j].g.ncells, kPlaceBatchCells);
         for (int k = 0; k < npb; ++k) place.push_back(make_int2((int)j, k));
     }
     for (auto& I : ni) {

@@ -273,7 +273,6 @@ __device__ __forceinline__ void move_slot(const Pop<T>& P, int64_t from, int64_t
 template <typename T>
 __device__ __forceinline__ void register_arrival(const Pop<T>& P, uint32_t o, const Mover<T>& m) {
     int k = atomicAdd(P.arr_cnt + m.cell, 1);
-    mark_dirty(P, m.cell);
     int64_t s = P.start[m.cell];
     if (k < (int)(P.start[m.cell + 1] - s)) {
         P.arr_list[s + k] = (int32_t)o;
@@ -370,27 +369,31 @@ __global__ void k_inject(Geom g, Pop<T> P, InjectParams ip) {
     if (lane == 0 && tot) atomicAdd(&P.ctr->injected, (uint32_t)tot);
 }
 
-// ---- import: one warp per cell ------------------------------------------------
-// Fills the cell's holes (sorted ascending) with its arrivals; surplus
-// arrivals append after the last particle, surplus holes are closed by moving
-// the cell's last particles into them. Arrivals beyond the cell's slots go to
-// the pending list and are pushed and placed again next step.
-// place_body is the work of a group of kG lanes (kG = 8: four cells per warp
-// at once; the kernel waits on memory, so four cells' loads in flight per
-// warp) on cell c (uniform within the group).
+// ---- import ---------------------------------------------------------------------
+// Fills a cell's holes (ascending) with its arrivals; surplus arrivals append
+// after the last particle, surplus holes are closed by moving the cell's last
+// particles into them. Arrivals beyond the cell's slots go to the pending
+// list and are pushed and placed again next step.
+//
+// The kernels wait on memory, and what counts is the number of round trips in
+// a row. A warp looks after up to 8 consecutive cells (place_cells_per_warp:
+// fewer on small grids): one round of loads fetches the hole, arrival and
+// particle counts and the slot ranges of all of them; groups of kPlaceLanes
+// lanes then take the cells that have holes or arrivals, four at a time: the
+// two lists, then the arriving records and the cell's last particles, then
+// the stores. Cells with more than kPlaceLanes holes or arrivals take the
+// whole warp (place_body, whose lists are sorted in memory). Listing the
+// flagged cells in a kernel of its own and placing from the list took 4 + 13
+// us on the headline workload and 4 + 21 us where most cells have arrivals;
+// this takes 10 us on both.
 constexpr int kPlaceLanes = 8;
 
-template <typename T, int kG = kPlaceLanes>
+// The general path, by a warp on cell c.
+template <typename T>
 __device__ __forceinline__ void place_body(const Geom& g, const Pop<T>& P, int32_t* sort_tmp, int c) {
-    static_assert(kG == 8 || kG == 16 || kG == 32, "group of 8, 16 or 32 lanes");
-    const int wl = threadIdx.x & 31, lane = wl & (kG - 1);
-    const unsigned gmask = (kG == 32 ? 0xffffffffu : ((1u << kG) - 1u)) << (wl & ~(kG - 1));
-    if (c >= g.ncells) return;
+    constexpr int kG = 32;
+    const int lane = threadIdx.x & 31;
     const int nh = P.hole_cnt[c], na_all = P.arr_cnt[c];
-    if (nh == 0 && na_all == 0) {  // nothing to place: only the flag to clear
-        if (lane == 0) P.dirty_flag[c] = 0;
-        return;
-    }
     const int64_t s0 = P.start[c];
     const int cap = (int)(P.start[c + 1] - s0);
     const int cnt = P.count[c];
@@ -412,7 +415,7 @@ __device__ __forceinline__ void place_body(const Geom& g, const Pop<T>& P, int32
             for (int j = 0; j < nh; ++j) r += P.hole_list[s0 + j] < h;
             sort_tmp[s0 + r] = h;
         }
-        __syncwarp(gmask);
+        __syncwarp();
     }
     const int32_t* H = (nh > 1 ? sort_tmp : P.hole_list) + s0;
     const int m = nh < np ? nh : np;
@@ -440,8 +443,8 @@ __device__ __forceinline__ void place_body(const Geom& g, const Pop<T>& P, int32
                 }
                 valid = !(a < nh && H[a] == t);
             }
-            const unsigned bal = __ballot_sync(gmask, valid);  // bits of this group's lanes only
-            const int idx = filled + __popc(bal & ((1u << wl) - 1u));
+            const unsigned bal = __ballot_sync(0xffffffffu, valid);
+            const int idx = filled + __popc(bal & ((1u << lane) - 1u));
             if (valid) move_slot(P, t, H[np + idx]);
             filled += __popc(bal);
         }
@@ -450,46 +453,98 @@ __device__ __forceinline__ void place_body(const Geom& g, const Pop<T>& P, int32
         P.count[c] = newcount;
         P.hole_cnt[c] = 0;
         P.arr_cnt[c] = 0;
-        P.dirty_flag[c] = 0;
     }
 }
 
-// Lists the cells flagged this step (holes or arrivals) of cells [c0, c1) of
-// population P on its dirty list (order: warp by warp, ascending within a
-// warp; the placement does not depend on the order). 32 x n threads from
-// thread t0 with stride `stride`.
+// The cells [c0, c0 + cells) of population P, cells <= 8, by one warp.
 template <typename T>
-__device__ __forceinline__ void dirty_compact_body(const Pop<T>& P, int c0, int c1, int64_t t0, int64_t stride) {
-    const int lane = threadIdx.x & 31;
-    for (int64_t base = t0 - lane; base + c0 < c1; base += stride) {
-        const int c = (int)(c0 + base + lane);
-        const bool d = c < c1 && P.dirty_flag[c] != 0;
-        const unsigned b = __ballot_sync(0xffffffffu, d);
-        if (!b) continue;
-        uint32_t o = 0;
-        if (lane == 0) o = atomicAdd(&P.ctr->dirty, (uint32_t)__popc(b));
-        o = __shfl_sync(0xffffffffu, o, 0) + __popc(b & ((1u << lane) - 1u));
-        if (d) P.dirty_list[o] = c;
+__device__ __forceinline__ void place_cells(const Geom& g, const Pop<T>& P, int32_t* sort_tmp, int c0, int cells) {
+    constexpr unsigned kAll = 0xffffffffu;
+    constexpr int kG = kPlaceLanes;
+    const int lane = threadIdx.x & 31, gl = lane & (kG - 1), grp = lane / kG;
+    cells = min(cells, g.ncells - c0);
+    int v = 0;
+    int64_t s = 0;
+    {   // lanes 0-7 the holes, 8-15 the arrivals, 16-23 the particles of a cell each
+        const int32_t* tab = lane < 8 ? P.hole_cnt : lane < 16 ? P.arr_cnt : P.count;
+        if (lane < 24 && (lane & 7) < cells) v = tab[c0 + (lane & 7)];
+        if (lane <= cells) s = P.start[c0 + lane];
+    }
+    const unsigned any = __ballot_sync(kAll, v != 0), many = __ballot_sync(kAll, v > kG);
+    unsigned heavy = (many | (many >> 8)) & 0xffu;
+    unsigned todo = (any | (any >> 8)) & 0xffu & ~heavy;
+    for (; heavy; heavy &= heavy - 1) {
+        __syncwarp();
+        place_body<T>(g, P, sort_tmp, c0 + __ffs(heavy) - 1);
+    }
+    while (todo) {
+        // group k takes the k-th cell left
+        unsigned t = todo;
+        for (int k = 0; k < grp; ++k) t &= t - 1;
+        const bool small = t != 0;
+        const int i = small ? __ffs(t) - 1 : 0;
+#pragma unroll
+        for (int k = 0; k < 32 / kG; ++k) todo &= todo - 1;
+        const int nh = __shfl_sync(kAll, v, i), na_all = __shfl_sync(kAll, v, 8 + i);
+        const int cnt = __shfl_sync(kAll, v, 16 + i);
+        const int64_t s0 = __shfl_sync(kAll, s, i), s1 = __shfl_sync(kAll, s, i + 1);
+        const int cap = (int)(s1 - s0);
+        const int na = small ? min(na_all, cap) : 0, holes = small ? nh : 0;
+        const int np = min(na, cap - (cnt - holes));  // arrivals that find a slot
+        const int newcount = cnt - holes + np;
+        int32_t h = gl < holes ? P.hole_list[s0 + gl] : 0x7fffffff;
+        const int32_t o = gl < na ? P.arr_list[s0 + gl] : 0;
+        // the arriving record and, where holes are left over, the cell's last
+        // particles: issued together
+        Mover<T> m = {};
+        if (gl < na) m = P.outbox[o];
+        const int left = holes - np;  // > 0: holes to close, as many last slots
+        const int64_t tail = s0 + newcount + gl;
+        const bool in_tail = gl < left;
+        Mover<T> last = {};
+        if (in_tail) {
+            last.x = P.x[tail]; last.y = P.y[tail]; last.z = P.z[tail];
+            last.u = P.u[tail]; last.v = P.v[tail]; last.w = P.w[tail];
+            last.id = P.id ? P.id[tail] : 0u;
+        }
+        // the holes in ascending order: bitonic, 8 lanes
+#pragma unroll
+        for (int size = 2; size <= kG; size <<= 1)
+#pragma unroll
+            for (int step = size >> 1; step >= 1; step >>= 1) {
+                const int32_t x = __shfl_xor_sync(kAll, h, step);
+                const bool up = (gl & size) == 0, low = (gl & step) == 0;
+                h = (up == low) ? min(h, x) : max(h, x);
+            }
+        if (gl < na && gl >= np) {  // no slot: waits a step
+            const uint32_t pi = atomicAdd(&P.ctr->pending_out, 1u);
+            if (pi < P.pending_cap) P.pending_out[pi] = m;
+            else atomicAdd(&P.ctr->lost, 1u);
+        }
+        if (gl < np) write_slot(P, gl < holes ? (int64_t)h : s0 + cnt + (gl - holes), m);
+        // is this lane's last slot one of the remaining holes H[np, holes)?
+        bool valid = in_tail;
+#pragma unroll
+        for (int k = 0; k < kG; ++k) {
+            const int32_t x = __shfl_sync(kAll, h, k, kG);
+            valid = valid && !(k >= np && (int64_t)x == tail);
+        }
+        const unsigned moving = (__ballot_sync(kAll, valid) >> (grp * kG)) & 0xffu;
+        const int32_t to = __shfl_sync(kAll, h, max(0, np) + __popc(moving & ((1u << gl) - 1u)), kG);
+        if (valid) write_slot(P, to, last);
+        if (small && gl == 0) {
+            P.count[c0 + i] = newcount;
+            P.hole_cnt[c0 + i] = 0;
+            P.arr_cnt[c0 + i] = 0;
+        }
     }
 }
 
+// Population blockIdx.y of the set, `cells` cells per warp.
 template <typename T>
-__global__ void k_dirty_compact(int ncells, const __grid_constant__ PopSet<T> S) {
-    dirty_compact_body<T>(S.p[blockIdx.y], 0, ncells, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
-                          (int64_t)gridDim.x * blockDim.x);
-}
-
-// The cells of the step's dirty lists (the only ones with holes or
-// arrivals), one group of kPlaceLanes lanes per cell, groups striding over
-// the list of population blockIdx.y.
-template <typename T>
-__global__ void k_place(Geom g, const __grid_constant__ PopSet<T> S) {
-    const Pop<T>& P = S.p[blockIdx.y];
-    int32_t* sort_tmp = S.sort_tmp[blockIdx.y];
-    const uint32_t n = P.ctr->dirty;
-    const uint32_t g0 = (blockIdx.x * blockDim.x + threadIdx.x) / kPlaceLanes,
-                   ng = (gridDim.x * blockDim.x) / kPlaceLanes;
-    for (uint32_t i = g0; i < n; i += ng) place_body<T>(g, P, sort_tmp, P.dirty_list[i]);
+__global__ void __launch_bounds__(kPlaceThreads) k_place(Geom g, const __grid_constant__ PopSet<T> S, int cells) {
+    const int64_t c0 = (blockIdx.x * (int64_t)kPlaceThreads + threadIdx.x) / 32 * cells;
+    if (c0 < g.ncells) place_cells<T>(g, S.p[blockIdx.y], S.sort_tmp[blockIdx.y], (int)c0, cells);
 }
 
 // Moves this step's pending list to the next step's input (thread t0 = 0

@@ -26,15 +26,9 @@ int launch_inject(const Geom& g, const Pop<T>& P, double per_cell, const double 
 template <typename T>
 int launch_place(const Geom& g, const PopSet<T>& S, cudaStream_t st) {
     if (S.n <= 0) return 0;
-    // the flagged cells onto the dirty lists (a thread per cell)
-    int64_t cb = ((int64_t)g.ncells + 255) / 256;
-    if (cb > 152 * 8) cb = 152 * 8;
-    k_dirty_compact<T><<<dim3((unsigned)cb, S.n), 256, 0, st>>>(g.ncells, S);
-    // a group of kPlaceLanes lanes per dirty cell
-    int64_t blocks = ((int64_t)g.ncells + 7) / 8;
-    if (blocks > 152 * 8) blocks = 152 * 8;
-    k_place<T><<<dim3((unsigned)blocks, S.n), 256, 0, st>>>(g, S);
-    return 2;
+    const int cells = place_cells_per_warp((int64_t)g.ncells * S.n);
+    k_place<T><<<dim3((unsigned)place_blocks(g.ncells, cells), S.n), kPlaceThreads, 0, st>>>(g, S, cells);
+    return 1;
 }
 
 template <typename T>
@@ -61,29 +55,15 @@ int launch_pending_count(const Pop<T>& P, int32_t* per_cell, cudaStream_t st) {
 }
 
 // ---- batched ensemble ------------------------------------------------------
-// Placement of a batch: blockIdx.y = job, the job's warps stride over its
-// dirty-cell list (cells with holes or arrivals only).
-// Batched dirty lists: block b lists the flagged cells of the 512-cell
-// range tab[b].y of job tab[b].x.
+// Batched placement: block b is block tab[b].y of the blocks of job
+// tab[b].x, 8 cells per warp.
 template <typename T>
-__global__ void k_dirty_compact_batch(const PopJob<T>* __restrict__ jobs, const int2* __restrict__ tab) {
+__global__ void __launch_bounds__(kPlaceThreads)
+    k_place_batch(const PopJob<T>* __restrict__ jobs, const int2* __restrict__ tab) {
     const int2 e = tab[blockIdx.x];
     const PopJob<T>& J = jobs[e.x];
-    const int c0 = e.y * 512, c1 = c0 + 512 < J.g.ncells ? c0 + 512 : J.g.ncells;
-    dirty_compact_body<T>(J.P, c0, c1, threadIdx.x, blockDim.x);
-}
-
-// Batched placement: block b is block tab[b].y of the place_blocks(ncells)
-// blocks of job tab[b].x (its share grows with the universe), groups of
-// kPlaceLanes lanes striding over the job's dirty list.
-template <typename T>
-__global__ void k_place_batch(const PopJob<T>* __restrict__ jobs, const int2* __restrict__ tab) {
-    const int2 e = tab[blockIdx.x];
-    const PopJob<T>& J = jobs[e.x];
-    const uint32_t n = J.P.ctr->dirty;
-    const uint32_t g0 = ((uint32_t)e.y * blockDim.x + threadIdx.x) / kPlaceLanes,
-                   ng = ((uint32_t)place_blocks(J.g.ncells) * blockDim.x) / kPlaceLanes;
-    for (uint32_t i = g0; i < n; i += ng) place_body<T>(J.g, J.P, J.sort_tmp, J.P.dirty_list[i]);
+    const int c0 = (e.y * kPlaceThreads + (int)threadIdx.x) / 32 * kPlaceBatchCells;
+    if (c0 < J.g.ncells) place_cells<T>(J.g, J.P, J.sort_tmp, c0, kPlaceBatchCells);
 }
 
 template <typename T>
@@ -103,7 +83,7 @@ __global__ void k_batch_begin(const PopJob<T>* __restrict__ jobs, int njobs, con
         for (int64_t j = t0; j < njobs; j += stride) {
             StepCounters* c = jobs[j].P.ctr;
             c->outbox = 0; c->pending_out = 0; c->deferred = 0;
-            c->removed = 0; c->migrated = 0; c->injected = 0; c->dirty = 0;
+            c->removed = 0; c->migrated = 0; c->injected = 0;
         }
         if (t0 == 0) *flagged = 0;
         return;
@@ -149,9 +129,8 @@ __global__ void k_batch_status(const PopJob<T>* __restrict__ jobs, int njobs, Jo
 template <typename T>
 int launch_place_batch(const PopJob<T>* jobs, const int2* tab, int64_t nblocks, cudaStream_t st) {
     if (nblocks <= 0) return 0;
-    k_dirty_compact_batch<T><<<(unsigned)nblocks, 256, 0, st>>>(jobs, tab);
-    k_place_batch<T><<<(unsigned)nblocks, 256, 0, st>>>(jobs, tab);
-    return 2;
+    k_place_batch<T><<<(unsigned)nblocks, kPlaceThreads, 0, st>>>(jobs, tab);
+    return 1;
 }
 
 template <typename T>

@@ -346,8 +346,7 @@ __device__ __forceinline__ void emit_node_sums(const Geom& g, float s, int64_t n
 // arrival list of the destination, cooperative deposit; the old slot is
 // filed as a hole of its cell (leavers and drops). `dir` is the export's
 // move. The round trips (the destination's arrival slot, the outbox slots,
-// the hole slots) are issued together before any result is used, and cells
-// are flagged with plain stores (k_dirty_compact lists them). kOneCell:
+// the hole slots) are issued together before any result is used. kOneCell:
 // every lane's slot is in `cell` (item mode), so the warp files its holes
 // with one aggregated atomic.
 template <bool kOneCell>
@@ -396,7 +395,6 @@ __device__ __forceinline__ void leave_and_hole(const Geom& g, const Pop<float>& 
             m.id = id;
             m.x = p.x; m.y = p.y; m.z = p.z;
             m.u = p.u; m.v = p.v; m.w = p.w;
-            mark_dirty(P, dc);
             // the outbox holds every particle of the population plus the
             // pending and injected ones: o is always below its capacity
             const bool in_box = o < P.outbox_cap;
@@ -415,9 +413,6 @@ __device__ __forceinline__ void leave_and_hole(const Geom& g, const Pop<float>& 
     }
     if (kOneCell) {
         hk = __shfl_sync(0xffffffffu, hk, __ffs(hb) - 1) + __popc(hb & below);
-        if (lane == 0) mark_dirty(P, cell);
-    } else if (hole) {
-        mark_dirty(P, cell);
     }
     if (hole) P.hole_list[cstart + hk] = (int32_t)slot;
     if (outcome == kDrop) ++nrem;
