@@ -136,6 +136,26 @@ std::vector<PopSet<T>> pop_sets(std::vector<PopStore<T>>& pops) {
 }
 // Advances the device step counter (keys the injection generator).
 __global__ void k_step_end(uint64_t* step) { *step += 1; }
+
+// Clears what a step accumulates into: the step counters of every population
+// (not the sticky ones, lost and timeouts) and, with nj > 0, J and rho. One
+// launch: as memsets these were up to 4 nodes in a row before the push,
+// about 2 us each.
+struct CounterSet {
+    StepCounters* c[kMaxPops];
+    int n;
+};
+__global__ void __launch_bounds__(256) k_step_begin(const __grid_constant__ CounterSet s, double* J, int64_t nj,
+                                                    double* rho, int64_t nrho) {
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
+    if (t0 < s.n) {
+        StepCounters* c = s.c[t0];
+        c->outbox = 0; c->pending_out = 0; c->deferred = 0;
+        c->removed = 0; c->migrated = 0; c->injected = 0;
+    }
+    for (int64_t t = t0; t < nj; t += stride) J[t] = 0.0;
+    for (int64_t t = t0; t < nrho; t += stride) rho[t] = 0.0;
+}
 }  // namespace ipg
 
 using namespace ipg;
@@ -163,8 +183,9 @@ struct ipic3d_ctx {
     // step graphs (StepKind): the whole step, or, in a run of steps with a
     // field solver, the first solve alone, then the moves with the next
     // step's solve beside the placement, the last move without it
-    cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
-    uint64_t graph_kernels[4] = {0, 0, 0, 0};  // kernels one replay runs
+    // [0] one step, [1] kUnroll steps of the kind per replay
+    cudaGraphExec_t graph[4][2] = {};
+    uint64_t graph_kernels[4][2] = {};  // kernels one replay runs
     // pending-list watch: per step an async copy of the pending counts into
     // pinned memory, read one step later (ring of two)
     uint32_t* h_pending = nullptr;  // [2][kMaxPops]
@@ -240,10 +261,11 @@ struct ipic3d_ctx {
 namespace {
 
 void drop_graph(ipic3d_ctx* ctx) {
-    for (auto& gr : ctx->graph) {
-        if (gr) cudaGraphExecDestroy(gr);
-        gr = nullptr;
-    }
+    for (auto& kind : ctx->graph)
+        for (auto& gr : kind) {
+            if (gr) cudaGraphExecDestroy(gr);
+            gr = nullptr;
+        }
 }
 
 // What one replay of a step graph does.
@@ -253,6 +275,10 @@ enum StepKind : int {
     kStepMoveSolve = 2,  // the move, the next step's solve beside its placement
     kStepMove = 3,       // the move alone (last step of a run)
 };
+
+// Steps of one replay in long runs: between replays the pending counts come
+// back and the next graph starts, 6 to 15 us in which the GPU waits.
+constexpr int kUnroll = 8;
 
 void release_pops(ipic3d_ctx* ctx) {
     for (auto& p : ctx->p32) p.release();
@@ -1088,6 +1114,19 @@ int ph_collect(ipic3d_ctx* ctx) {
     return IPIC3D_OK;
 }
 
+// Clears the step counters and, with `moments`, J and rho (k_step_begin).
+int step_begin(ipic3d_ctx* ctx, bool counters, bool moments, cudaStream_t st) {
+    CounterSet s{};
+    if (counters) {
+        for (auto& P : ctx->p32) s.c[s.n++] = P.ctr;
+        for (auto& P : ctx->p64) s.c[s.n++] = P.ctr;
+    }
+    const int64_t nrho = moments ? ctx->nnode() : 0;
+    const int64_t blocks = std::min<int64_t>(std::max<int64_t>(1, (3 * nrho + 1023) / 1024), 152 * 8);
+    k_step_begin<<<(unsigned)blocks, 256, 0, st>>>(s, ctx->J, 3 * nrho, ctx->rho, nrho);
+    return 1;
+}
+
 // projectToDensityField over the stored particles (deposit-only pass).
 int project_impl(ipic3d_ctx* ctx) {
     cudaStream_t st = ctx->stream;
@@ -1138,23 +1177,16 @@ int solve_impl(ipic3d_ctx* ctx) {
 // deposit is in; they read and write fields and J only, the move and the
 // placement touch particles, J and interior nodes' reads only). Then the
 // E update reads the raw deposit sums and folds and normalises them itself:
-// no J finalisation, and J and rho are cleared for the next step's deposit
-// once it has read them (`cleared`: a step that starts so skips its own
-// clear). With phase timing on, everything runs on one stream.
+// no J finalisation. With `next_solve`, J, rho and the step counters are
+// cleared for the next step at the end (`cleared`: a step that starts so
+// skips its own clear). With phase timing on, everything runs on one stream.
 int move_impl(ipic3d_ctx* ctx, bool deposit, bool next_solve = false, bool cleared = false) {
     cudaStream_t st = ctx->stream;
     Geom g = ctx->g;
     g.deposit = deposit ? 1 : 0;
     int n = 0;
-    for (auto& P : ctx->p32) CU(cudaMemsetAsync(P.ctr, 0, offsetof(StepCounters, lost), st));
-    for (auto& P : ctx->p64) CU(cudaMemsetAsync(P.ctr, 0, offsetof(StepCounters, lost), st));
-    if (deposit) {
-        ph_begin(ctx, IPIC3D_PHASE_MOMENTS);
-        if (!cleared) {
-            CU(cudaMemsetAsync(ctx->J, 0, ctx->nnode() * 3 * sizeof(double), st));
-            CU(cudaMemsetAsync(ctx->rho, 0, ctx->nnode() * sizeof(double), st));
-        }
-    }
+    if (deposit) ph_begin(ctx, IPIC3D_PHASE_MOMENTS);
+    if (!cleared) n += step_begin(ctx, true, deposit, st);
     const bool fork = !ctx->profiling;
     if (fork && !ctx->aux_stream) {
         // the higher priority: the solver chain on it is the longer branch
@@ -1227,11 +1259,9 @@ int move_impl(ipic3d_ctx* ctx, bool deposit, bool next_solve = false, bool clear
         ++n;
     }
     ph_end(ctx, IPIC3D_PHASE_PLACE);
-    if (raw_j) {  // the E update has read J: clear J and rho for the next step
-        CU(cudaStreamWaitEvent(st, ctx->aux_ev[4], 0));
-        CU(cudaMemsetAsync(ctx->J, 0, ctx->nnode() * 3 * sizeof(double), st));
-        CU(cudaMemsetAsync(ctx->rho, 0, ctx->nnode() * sizeof(double), st));
-    }
+    // once the E update has read J: clear for the next step
+    if (raw_j) CU(cudaStreamWaitEvent(st, ctx->aux_ev[4], 0));
+    if (next_solve) n += step_begin(ctx, true, raw_j, st);
     if (jfork) {
         CU(cudaEventRecord(ctx->aux_ev[3], aux));
         CU(cudaStreamWaitEvent(st, ctx->aux_ev[3], 0));
@@ -1328,24 +1358,24 @@ int enqueue_step(ipic3d_ctx* ctx, int kind = kStepFull) {
         if ((rc = solve_impl(ctx))) return rc;
     }
     if (kind == kStepSolve) {  // a move follows: J and rho cleared for its deposit
-        if (project) {
-            CU(cudaMemsetAsync(ctx->J, 0, ctx->nnode() * 3 * sizeof(double), ctx->stream));
-            CU(cudaMemsetAsync(ctx->rho, 0, ctx->nnode() * sizeof(double), ctx->stream));
-        }
-        return IPIC3D_OK;
+        return check_launch(ctx, step_begin(ctx, true, project, ctx->stream));
     }
     // advances the device step counter
     return move_impl(ctx, project, kind == kStepMoveSolve, kind == kStepMoveSolve || kind == kStepMove);
 }
 
-// Replays step graph `kind`, capturing it first if needed.
-int run_graph(ipic3d_ctx* ctx, int kind) {
-    if (!ctx->graph[kind]) {
+// Replays step graph `kind` (`steps` = 1 or kUnroll times it), capturing it
+// first if needed.
+int run_graph(ipic3d_ctx* ctx, int kind, int steps = 1) {
+    const int u = steps > 1 ? 1 : 0;
+    cudaGraphExec_t& exec = ctx->graph[kind][u];
+    if (!exec) {
         cudaGraph_t graph = nullptr;
         CU(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
         const uint64_t before = ctx->launches;
-        const int rc = enqueue_step(ctx, kind);
-        ctx->graph_kernels[kind] = ctx->launches - before;
+        int rc = IPIC3D_OK;
+        for (int i = 0; i < steps && rc == IPIC3D_OK; ++i) rc = enqueue_step(ctx, kind);
+        ctx->graph_kernels[kind][u] = ctx->launches - before;
         ctx->launches = before;  // capturing runs nothing
         cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
         if (rc) {
@@ -1353,12 +1383,12 @@ int run_graph(ipic3d_ctx* ctx, int kind) {
             return rc;
         }
         if (e != cudaSuccess) return fail(IPIC3D_E_CUDA, "graph capture: %s", cudaGetErrorString(e));
-        e = cudaGraphInstantiate(&ctx->graph[kind], graph, cudaGraphInstantiateFlagUseNodePriority);
+        e = cudaGraphInstantiate(&exec, graph, cudaGraphInstantiateFlagUseNodePriority);
         cudaGraphDestroy(graph);
         if (e != cudaSuccess) return fail(IPIC3D_E_CUDA, "graph instantiate: %s", cudaGetErrorString(e));
     }
-    CU(cudaGraphLaunch(ctx->graph[kind], ctx->stream));
-    ctx->launches += ctx->graph_kernels[kind];
+    CU(cudaGraphLaunch(exec, ctx->stream));
+    ctx->launches += ctx->graph_kernels[kind][u];
     return IPIC3D_OK;
 }
 
@@ -1730,14 +1760,19 @@ int ipic3d_gpu_step(ipic3d_ctx* ctx, uint64_t num_steps) {
     const bool use_graph = (ctx->cfg.flags & IPIC3D_F_USE_GRAPH) != 0 && !ctx->profiling;
     // re-lay out when more than 0.5% of the particles wait for a slot
     const uint64_t pend_limit = std::max<uint64_t>(64, ctx->particles_hint / 200);
-    uint64_t watch_from = 0;  // first step whose pending count is still meaningful
+    uint64_t watch_from = 0;  // first round whose pending count is still meaningful
     tune_prepare(ctx);
     // a run of graph steps with a field solver solves the next step's fields
     // beside the current step's placement: the first solve alone, the last
     // step without a solve after it
     const bool overlap = use_graph && ctx->cfg.solver != IPIC3D_SOLVER_STATIC;
     bool presolved = false;
-    for (uint64_t done = 0; done < num_steps;) {
+    // long runs replay kUnroll steps at a time (the last step apart; capturing
+    // the longer graph pays for itself over a few replays)
+    const bool unroll = use_graph && num_steps >= 3 * kUnroll;
+    uint64_t round = 0;  // replays (or eager steps) so far
+    for (uint64_t done = 0; done < num_steps; ++round) {
+        uint64_t steps = 1;
         if (ctx->tuner.running()) {  // a trial step of the autotuner: outside the graph, push timed
             ctx->tune_timing = true;
             rc = enqueue_step(ctx);
@@ -1748,38 +1783,41 @@ int ipic3d_gpu_step(ipic3d_ctx* ctx, uint64_t num_steps) {
         } else if (overlap && (presolved || done + 1 < num_steps)) {
             if (!presolved && (rc = run_graph(ctx, kStepSolve))) return rc;
             const bool last = done + 1 == num_steps;
-            if ((rc = run_graph(ctx, last ? kStepMove : kStepMoveSolve))) return rc;
+            if (unroll && num_steps - done > kUnroll) steps = kUnroll;
+            if ((rc = run_graph(ctx, last ? kStepMove : kStepMoveSolve, (int)steps))) return rc;
             presolved = !last;
         } else if (use_graph) {  // a lone step (or no field solver): one graph
-            if ((rc = run_graph(ctx, kStepFull))) return rc;
+            if (unroll && !overlap && num_steps - done > kUnroll) steps = kUnroll;
+            if ((rc = run_graph(ctx, kStepFull, (int)steps))) return rc;
         } else {
             if ((rc = enqueue_step(ctx))) return rc;
             if ((rc = ph_collect(ctx))) return rc;
         }
-        // this step's pending count -> pinned slot (done & 1)
-        const int slot = (int)(done & 1);
+        done += steps;
+        ctx->steps += steps;
+        if (done == num_steps) break;
+        // the particles that wait for a slot now -> pinned slot (round & 1)
+        const int slot = (int)(round & 1);
         int k = 0;
         for (auto& P : ctx->p32)
             if (k < kMaxPops)
-                CU(cudaMemcpyAsync(ctx->h_pending + slot * kMaxPops + k++, &P.ctr->pending_out, sizeof(uint32_t),
+                CU(cudaMemcpyAsync(ctx->h_pending + slot * kMaxPops + k++, P.pending_in_count, sizeof(uint32_t),
                                    cudaMemcpyDeviceToHost, ctx->stream));
         for (auto& P : ctx->p64)
             if (k < kMaxPops)
-                CU(cudaMemcpyAsync(ctx->h_pending + slot * kMaxPops + k++, &P.ctr->pending_out, sizeof(uint32_t),
+                CU(cudaMemcpyAsync(ctx->h_pending + slot * kMaxPops + k++, P.pending_in_count, sizeof(uint32_t),
                                    cudaMemcpyDeviceToHost, ctx->stream));
         CU(cudaEventRecord(ctx->pend_ev[slot], ctx->stream));
-        ++done;
-        ++ctx->steps;
-        // the previous step's count (the GPU works on this step meanwhile)
-        if (done >= 2 && done - 2 >= watch_from && done < num_steps) {
-            const int ps = (int)((done - 2) & 1);
+        // the previous round's count (the GPU works on this round meanwhile)
+        if (round >= 1 && round - 1 >= watch_from) {
+            const int ps = (int)((round - 1) & 1);
             CU(cudaEventSynchronize(ctx->pend_ev[ps]));
             uint64_t pend = 0;
             for (int q = 0; q < k; ++q) pend += ctx->h_pending[ps * kMaxPops + q];
             if (pend > pend_limit) {
                 ctx->relayout_steps += 1;
                 if ((rc = after_steps(ctx))) return rc;  // waits, then re-lays out
-                watch_from = done;  // counts recorded before the re-layout are stale
+                watch_from = round + 1;  // counts recorded before the re-layout are stale
             }
         }
     }
