@@ -10,22 +10,32 @@
 namespace ipg {
 
 namespace {
-// How a launch over `slots` slots in `tiles` tiles is cut: particles per
-// work item, tiles per block, blocks per span. About 4 warps per
-// sub-partition (152 SMs x 4) keep the FP64 pipe busy; an item costs its
-// group about 70 FP64 instructions beside 150 per 8 particles, so items are
-// as long as that allows. Spans of 4 tiles leave fewer warps part-filled
-// where there are blocks enough.
+// How a launch over `slots` slots in `tiles` tiles is cut: particles per work
+// item, tiles per block, blocks per span, warps per block.
+//   * About 4 warps per sub-partition (152 SMs x 4) keep the FP64 pipe busy.
+//     An item costs its group about 70 FP64 instructions with the deposit,
+//     beside 150 per 8 particles, so items are as long as that allows;
+//     without the deposit an item costs next to nothing, and 32 particles
+//     leave a short tail.
+//   * Where there are blocks enough, spans of 4 tiles and 4 warps per block:
+//     fewer table scans and part-filled warps. Otherwise one warp per block:
+//     160 blocks of 4 warps put two blocks on 8 of the 152 SMs, and the FP64
+//     pipe of those decides (E x B 8^3: a step of 57 us, single warps with
+//     items of 16 particles 56, of 8 particles 43; .inp 16^3: push 0.207 ms
+//     with 4 warps and items of 64, 0.160 with single warps and 32).
 struct Shape64 {
-    int item, span, parts;
+    int item, span, parts, warps;
 };
-Shape64 shape64(int64_t slots, int64_t tiles) {
-    constexpr int64_t kSms = 152, kGroups = kSms * 4 * 4 * (32 / kGroup64);
-    Shape64 s{256, 1, 1};
-    while (s.item > 16 && slots < s.item * kGroups) s.item /= 2;
-    if (tiles >= kMaxSpan64 * kSms * 6) s.span = kMaxSpan64;
-    const int64_t most = std::max<int64_t>(1, kSlotsPerCta / (s.item * kItems64));
-    s.parts = (int)std::max<int64_t>(1, std::min(most, (4 * kSms + tiles - 1) / std::max<int64_t>(1, tiles)));
+Shape64 shape64(int64_t slots, int64_t tiles, bool deposit) {
+    constexpr int64_t kSms = 152, kGroups = kSms * 4 * 4 * kWarpItems64;
+    Shape64 s{deposit ? 256 : 32, 1, 1, 1};
+    while (s.item > kGroup64 && slots < s.item * kGroups) s.item /= 2;
+    if (tiles >= kMaxSpan64 * kSms * 6) {
+        s.span = kMaxSpan64;
+        s.warps = kMaxWarps64;
+    } else {
+        s.parts = (int)std::max<int64_t>(1, kSlotsPerCta / (s.item * kWarpItems64 * s.warps));
+    }
     return s;
 }
 
@@ -54,10 +64,10 @@ int launch_push<double>(const Geom& g, const PopSet<double>& S, int mode, const 
         slots += S.p[i].capacity;
     }
     if (most <= 0 || (mode != 0 && !g.deposit)) return 0;
-    const Shape64 sh = shape64(slots, tiles);
+    const Shape64 sh = shape64(slots, tiles, g.deposit != 0);
     const dim3 grid((unsigned)((most + sh.span - 1) / sh.span), sh.parts, S.n);
     const Push64Set pcs = push64_set(g, S);
-    auto run = [&](auto k) { k<<<grid, kThreads64, 0, st>>>(g, S, pcs, sh.span, sh.item); };
+    auto run = [&](auto k) { k<<<grid, 32 * sh.warps, push64_smem_bytes(sh.span, sh.warps), st>>>(g, S, pcs, sh.span, sh.item); };
     if (mode != 0) run(k_push64<false, false, true>);
     else if (g.mover == 1 && g.deposit) run(k_push64<true, true, true>);
     else if (g.mover == 1) run(k_push64<true, true, false>);
@@ -82,9 +92,9 @@ template <>
 int launch_push_batch<double>(const PopJob<double>* jobs, const int2* cta_job, int64_t nctas, int mode,
                               const Geom& g, const PushShape&, cudaStream_t st) {
     if (nctas <= 0 || (mode != 0 && !g.deposit)) return 0;
-    const Shape64 sh = shape64(nctas * kSlotsPerCta, nctas);
+    const Shape64 sh = shape64(nctas * kSlotsPerCta, nctas, g.deposit != 0);
     const dim3 grid((unsigned)nctas, sh.parts);
-    auto run = [&](auto k) { k<<<grid, kThreads64, 0, st>>>(jobs, cta_job, sh.span, sh.item); };
+    auto run = [&](auto k) { k<<<grid, 32 * sh.warps, push64_smem_bytes(sh.span, sh.warps), st>>>(jobs, cta_job, sh.span, sh.item); };
     if (mode != 0) run(k_push64_batch<false, false, true>);
     else if (g.mover == 1 && g.deposit) run(k_push64_batch<true, true, true>);
     else if (g.mover == 1) run(k_push64_batch<true, true, false>);

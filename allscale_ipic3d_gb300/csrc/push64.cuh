@@ -20,19 +20,21 @@
 // 541 before. The dipole mover without the gather rounds exactly as the
 // reference does (dipole64.cuh). Measured push per step, before and after:
 // 8.4M particles, gather + dipole + deposit 9.18 -> 2.89 ms (FP64 pipe 86 %
-// busy); 306k particles, two species, gather + deposit 0.593 -> 0.161 ms;
-// 33k particles 0.140 -> 0.033 ms; 1.05M particles, dipole mover 0.489 ->
-// 0.221 ms.
+// busy); 306k particles, two species, gather + deposit 0.593 -> 0.151 ms;
+// 33k particles 0.140 -> 0.028 ms (a warp's serial chain); 1.05M particles,
+// dipole mover, a sixth of them leaving their cells 0.489 -> 0.160 ms (FP64
+// pipe 58 %, integer 42 %). Loading a round's particles a round ahead
+// changed nothing.
 //
 // Work. A work item is up to `item` particles of one cell, pushed by a group
 // of 8 lanes, 8 particles at a time (slots are 8-aligned: full 64-byte
 // segments); four items share a warp. Groups of 8 rather than whole warps
 // keep the lanes busy where cells hold few particles or end unevenly, at the
 // price of a reduction per 8 lanes; a cell of more than `item` particles is
-// cut evenly, so that the items of a warp end together. A block takes the
-// items of `span` consecutive 1024-slot tiles, or of a part of them
-// (gridDim.y parts): cells of up to a tile belong to the span they start in,
-// larger ones are cut at its boundaries.
+// cut evenly, so that the items of a warp end together. A block of 1 to 4
+// warps takes the items of `span` consecutive 1024-slot tiles, or of a part
+// of them (gridDim.y parts): cells of up to a tile belong to the span they
+// start in, larger ones are cut at its boundaries.
 #pragma once
 
 #include "dipole64.cuh"
@@ -40,9 +42,8 @@
 namespace ipg {
 
 constexpr int kGroup64 = 8;
-constexpr int kWarps64 = 4;
-constexpr int kThreads64 = 32 * kWarps64;
-constexpr int kItems64 = kThreads64 / kGroup64;  // work items of a block at a time
+constexpr int kMaxWarps64 = 4;
+constexpr int kWarpItems64 = 32 / kGroup64;  // work items of a warp at a time
 constexpr int kCoefStride64 = 50;  // 48 + 2: the four groups of a warp read different banks
 
 // ---- field --------------------------------------------------------------------
@@ -177,29 +178,41 @@ __device__ __forceinline__ void move_dipole64(const Geom& g, const Push64Const& 
 // ---- export ---------------------------------------------------------------------
 
 // A particle's cell: its coordinates, centre (getCenterOfCell,
-// universe_properties.h:139-142) and whether the planet reaches it.
+// universe_properties.h:139-142), and what the export can leave out.
 struct Cell64 {
     int x, y, z;
     double cen[3];
-    bool near_planet;
+    bool near_planet;  // the planet can reach a particle that stays in the cell
+    bool far_planet;   // it cannot reach one that is at most a cell away
+    bool edge;         // a face of the cell lies on the domain boundary
 };
 
 __device__ __forceinline__ double cell_centre(const Geom& g, int a, int pos) {
     return (g.origin[a] + (double)pos * g.w[a]) + g.half_w[a];
 }
-// Squared distance along axis a from the planet's centre to the cell's box,
-// in FP32; `reach2` below adds the margin.
-__device__ __forceinline__ float planet_gap2(const Geom& g, int a, double cen) {
-    const float d = fmaxf(fabsf((float)(cen - g.object_center[a])) - (float)g.half_w[a], 0.f);
-    return d * d;
+// Distance along axis a from the planet's centre to the cell's box, in FP32;
+// the comparison with planet_reach adds the margin.
+__device__ __forceinline__ float planet_gap(const Geom& g, int a, double cen) {
+    return fabsf((float)(cen - g.object_center[a])) - (float)g.half_w[a];
 }
-// A particle that stays in a cell further than this from the planet's centre
-// is outside the planet whatever the rounding (a 64th of a cell and 10^-5 of
-// the radius of margin).
-__device__ __forceinline__ float planet_reach2(const Geom& g) {
+// A particle further than this from the planet's centre is outside the planet
+// whatever the rounding (a 64th of a cell and 10^-5 of the radius of margin).
+__device__ __forceinline__ float planet_reach(const Geom& g) {
     const float w = fmaxf(fmaxf((float)g.w[0], (float)g.w[1]), (float)g.w[2]);
-    const float r = sqrtf((float)g.planet_r2) * 1.00001f + w * (1.f / 64.f);
-    return r * r;
+    return sqrtf((float)g.planet_r2) * 1.00001f + w * (1.f / 64.f);
+}
+// The flags from the three gaps (NaN and overflow: near, not far).
+__device__ __forceinline__ void planet_flags(const Geom& g, const float (&gap)[3], float reach, Cell64& c) {
+    float in2 = 0.f, out2 = 0.f;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float in = fmaxf(gap[a], 0.f), out = fmaxf(gap[a] - (float)g.w[a], 0.f);
+        in2 += in * in;
+        out2 += out * out;
+    }
+    c.near_planet = !(in2 > reach * reach);
+    c.far_planet = out2 > reach * reach;
+    c.edge = c.x == 0 || c.y == 0 || c.z == 0 || c.x == g.sx - 1 || c.y == g.sy - 1 || c.z == g.sz - 1;
 }
 
 __device__ __forceinline__ uint64_t magnitude_bits(double x) { return soft::bits_of(x) & 0x7fffffffffffffffull; }
@@ -209,6 +222,32 @@ __device__ __forceinline__ bool beyond(double x, double lim) {
     return b > soft::bits_of(lim) && b <= 0x7ff0000000000000ull;
 }
 __device__ __forceinline__ bool is_negative(double x) { return (int64_t)soft::bits_of(x) < 0; }
+
+// The rare parts of the export sit behind calls, so that the FP64
+// instructions of all of them are not issued for every leaver.
+struct Walled {
+    double p;
+    int inverts, drops;
+};
+// The wall rule of one axis (cell.h:1102-1121): reflecting faces shift by half
+// a cell and invert the velocity, open ones drop.
+__device__ __noinline__ Walled wall64(double p, double rel, double half, int pos, int size, int lo, int hi) {
+    Walled r = {p, 0, 0};
+    if (!beyond(rel, half)) return r;
+    const bool low = is_negative(rel);
+    const int bc = low ? (pos == 0 ? lo : 1) : (pos == size - 1 ? hi : 1);
+    r.drops = bc == 2;
+    r.inverts = bc == 0;
+    if (bc == 0) r.p = low ? p + half : p - half;
+    return r;
+}
+__device__ __noinline__ bool inside_planet64(double dx, double dy, double dz, double limit) {
+    double r2 = dx * dx;
+    r2 += dy * dy;
+    r2 += dz * dz;
+    return r2 <= limit;  // cell.h:1123-1128
+}
+__device__ __noinline__ double wrap64(double p, double length, int periodic) { return periodic ? p + length : p; }
 
 // exportParticles (cell.h:1093-1146) for a moved particle: walls, planet,
 // move to a neighbour. rel: the position relative to the cell's centre.
@@ -222,34 +261,32 @@ __device__ __forceinline__ int export64(const Geom& g, const Cell64& c, PState<d
         return kStay;
     const int pos[3] = {c.x, c.y, c.z}, size[3] = {g.sx, g.sy, g.sz};
     double P[3] = {p.x, p.y, p.z};
-    bool invert = false, drop = false;
+    if (c.edge) {
+        int inverts = 0, drops = 0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        if (!beyond(rel[a], g.half_w[a])) continue;
-        const bool low = is_negative(rel[a]);
-        const int bc = low ? (pos[a] == 0 ? g.bc_lo[a] : 1) : (pos[a] == size[a] - 1 ? g.bc_hi[a] : 1);
-        if (bc == 2) drop = true;
-        if (bc == 0) {
-            invert = true;
-            P[a] = low ? P[a] + g.half_w[a] : P[a] - g.half_w[a];
-            rel[a] = P[a] - c.cen[a];
+        for (int a = 0; a < 3; ++a) {
+            const Walled r = wall64(P[a], rel[a], g.half_w[a], pos[a], size[a], g.bc_lo[a], g.bc_hi[a]);
+            P[a] = r.p;
+            inverts |= r.inverts;
+            drops |= r.drops;
         }
+        if (inverts) {
+            p.u = soft::from_bits(soft::bits_of(p.u) ^ 0x8000000000000000ull);
+            p.v = soft::from_bits(soft::bits_of(p.v) ^ 0x8000000000000000ull);
+            p.w = soft::from_bits(soft::bits_of(p.w) ^ 0x8000000000000000ull);
+        }
+        if (drops) return kDrop;
+        rel[0] = P[0] - c.cen[0];
+        rel[1] = P[1] - c.cen[1];
+        rel[2] = P[2] - c.cen[2];
     }
-    if (invert) {
-        p.u = p.u * -1.0;
-        p.v = p.v * -1.0;
-        p.w = p.w * -1.0;
-    }
-    if (drop) return kDrop;
-    // the planet (cell.h:1123-1128): FP32 settles it away from the surface
-    const double dx = P[0] - g.object_center[0], dy = P[1] - g.object_center[1], dz = P[2] - g.object_center[2];
-    const float fx = (float)dx, fy = (float)dy, fz = (float)dz;
-    if (!(fx * fx + fy * fy + fz * fz > (float)g.planet_r2 * 1.00001f)) {
-        double r2 = dx * dx;
-        r2 += dy * dy;
-        r2 += dz * dz;
-        if (r2 <= g.planet_r2) return kDrop;
-    }
+    // the planet: settled by the cell for a particle within a cell width of
+    // its centre
+    if (!(c.far_planet && magnitude_bits(rel[0]) <= soft::bits_of(g.w[0]) &&
+          magnitude_bits(rel[1]) <= soft::bits_of(g.w[1]) && magnitude_bits(rel[2]) <= soft::bits_of(g.w[2])) &&
+        inside_planet64(P[0] - g.object_center[0], P[1] - g.object_center[1], P[2] - g.object_center[2],
+                        g.planet_r2))
+        return kDrop;
     int n[3];
     bool out = false;
 #pragma unroll
@@ -260,10 +297,10 @@ __device__ __forceinline__ int export64(const Geom& g, const Cell64& c, PState<d
             t += is_negative(rel[a]) ? -1 : 1;
             if (t < 0) {
                 t += size[a];
-                if (g.bc_lo[a] == 1) P[a] += (double)size[a] * g.w[a];
+                P[a] = wrap64(P[a], g.L[a], g.bc_lo[a] == 1);
             } else if (t >= size[a]) {
                 t -= size[a];
-                if (g.bc_hi[a] == 1) P[a] -= (double)size[a] * g.w[a];
+                P[a] = wrap64(P[a], -g.L[a], g.bc_hi[a] == 1);
             }
         }
         n[a] = t;
@@ -284,13 +321,13 @@ __device__ __forceinline__ int step_one64(const Geom& g, const Push64Const& pc, 
     Cell64 c;
     cell_coords(g, cell, c.x, c.y, c.z);
     const int pos[3] = {c.x, c.y, c.z};
-    float gap2 = 0.f;
+    float gap[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         c.cen[a] = cell_centre(g, a, pos[a]);
-        gap2 += planet_gap2(g, a, c.cen[a]);
+        gap[a] = planet_gap(g, a, c.cen[a]);
     }
-    c.near_planet = !(gap2 > planet_reach2(g));
+    planet_flags(g, gap, planet_reach(g), c);
     if (g.mover == 1) {
         const double x = (p.x - c.cen[0]) * g.inv_w[0], y = (p.y - c.cen[1]) * g.inv_w[1],
                      z = (p.z - c.cen[2]) * g.inv_w[2];
@@ -323,14 +360,30 @@ __device__ __forceinline__ int step_one64(const Geom& g, const Push64Const& pc, 
 
 // ---- the bulk push ---------------------------------------------------------------
 constexpr int kMaxSpan64 = 4;
-constexpr int kMaxCells64 = kMaxSpan64 * kMaxCellsPerCta;
 
+// A block's dynamic shared memory: the cells of its span, their coefficients
+// per group.
 struct Push64Smem {
-    int64_t start[kMaxCells64 + 1];
-    int count[kMaxCells64];
-    int first[kMaxCells64 + 1];  // items before the cell's
-    alignas(16) double coef[kItems64][kCoefStride64];
+    int64_t* start;  // [cells + 1]
+    double* coef;    // [groups][kCoefStride64]
+    int* count;      // [cells]
+    int* first;      // [cells + 1] items before the cell's
 };
+__host__ __device__ constexpr size_t push64_smem_bytes(int span, int warps) {
+    const int cells = span * kMaxCellsPerCta;
+    return (size_t)(cells + 2) / 2 * 2 * sizeof(int64_t) + (size_t)warps * kWarpItems64 * kCoefStride64 * sizeof(double) +
+           (size_t)(2 * cells + 1) * sizeof(int);
+}
+__device__ __forceinline__ Push64Smem push64_smem(int span, int warps) {
+    extern __shared__ __align__(16) unsigned char push64_raw[];
+    const int cells = span * kMaxCellsPerCta;
+    Push64Smem sm;
+    sm.start = reinterpret_cast<int64_t*>(push64_raw);
+    sm.coef = reinterpret_cast<double*>(sm.start + (cells + 2) / 2 * 2);  // 16-byte aligned
+    sm.count = reinterpret_cast<int*>(sm.coef + warps * kWarpItems64 * kCoefStride64);
+    sm.first = sm.count + cells;
+    return sm;
+}
 
 // Slots [lo, hi) of cell i that belong to the block's span [base, top).
 __device__ __forceinline__ void span_range64(const Push64Smem& sm, int i, int64_t base, int64_t top, int64_t& lo,
@@ -347,47 +400,70 @@ __device__ __forceinline__ void span_range64(const Push64Smem& sm, int i, int64_
     if (hi < lo) hi = lo;
 }
 
-// Bookkeeping of the warp's leavers and drops of one round.
+// Bookkeeping of the warp's leavers and drops of one round: outbox, arrival
+// lists, holes (a group's slots are of one cell: one atomic per group). The
+// round trips -- hole slots, arrival slots, outbox slots -- are issued
+// together before any result is used: in the .inp run every round has
+// leavers.
 __device__ __forceinline__ void leave64(const Geom& g, const Pop<double>& P, int outcome, int cell, int64_t cstart,
                                         int64_t slot, int dest, const PState<double>& p, bool deposit,
                                         uint32_t& nmig, uint32_t& nrem) {
-    const bool leave = outcome == kMove;
-    const uint32_t o = warp_append(&P.ctr->outbox, leave);
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, gl = lane & (kGroup64 - 1);
+    const unsigned below = (1u << lane) - 1u, group = 0xffu << (lane & ~(kGroup64 - 1));
+    const bool leave = outcome == kMove, hole = leave || outcome == kDrop;
+    const unsigned lb = __ballot_sync(kAll, leave), hb = __ballot_sync(kAll, hole) & group;
+    int hk = 0, ak = 0;
+    if (hb && gl == 0) hk = atomicAdd(P.hole_cnt + cell, __popc(hb));
+    uint32_t o = 0, id = 0u;
+    int64_t ds = 0, de = 0;
+    if (leave) {
+        ak = atomicAdd(P.arr_cnt + dest, 1);
+        ds = P.start[dest];
+        de = P.start[dest + 1];
+        if (P.id) id = P.id[slot];
+    }
+    if (lb && lane == 0) o = atomicAdd(&P.ctr->outbox, (uint32_t)__popc(lb));
+    o = __shfl_sync(kAll, o, 0) + __popc(lb & below);
     if (leave) {
         Mover<double> m;
         m.cell = dest;
-        m.id = P.id ? P.id[slot] : 0u;
+        m.id = id;
         m.x = p.x; m.y = p.y; m.z = p.z;
         m.u = p.u; m.v = p.v; m.w = p.w;
-        if (o < P.outbox_cap) {  // sized for one entry per slot: never full
-            P.outbox[o] = m;
-            register_arrival(P, o, m);
-        } else {
-            atomicAdd(&P.ctr->lost, 1u);
+        const bool in_box = o < P.outbox_cap;  // sized for one entry per slot: never full
+        if (in_box) P.outbox[o] = m;
+        else atomicAdd(&P.ctr->lost, 1u);
+        if (ak < (int)(de - ds)) {
+            P.arr_list[ds + ak] = in_box ? (int32_t)o : 0;
+        } else {  // the destination's slots are short: wait a step
+            const uint32_t pi = atomicAdd(&P.ctr->pending_out, 1u);
+            if (pi < P.pending_cap) P.pending_out[pi] = m;
+            else atomicAdd(&P.ctr->lost, 1u);
         }
         ++nmig;
     }
-    if (leave || outcome == kDrop) {
-        file_hole(P, cell, cstart, slot);
-        if (outcome == kDrop) ++nrem;
-    }
-    if (deposit) warp_deposit_leavers<double>(g, leave, dest, p, P.q);
+    hk = __shfl_sync(kAll, hk, 0, kGroup64) + __popc(hb & below);
+    if (hole) P.hole_list[cstart + hk] = (int32_t)slot;
+    if (outcome == kDrop) ++nrem;
+    if (deposit && lb) warp_deposit_leavers<double>(g, leave, dest, p, P.q);
 }
 
 // kStep: mover + export (else the deposit of the particles as they are);
 // kField: field-gather mover (else the dipole mover); kDep: deposit.
 template <bool kStep, bool kField, bool kDep>
 __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P, const Push64Const& pc, int64_t tile,
-                                            int span, int part, int parts, int item, Push64Smem& sm) {
+                                            int span, int part, int parts, int item) {
     constexpr unsigned kAll = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int gl = lane & (kGroup64 - 1), sub = lane / kGroup64;
+    const Push64Smem sm = push64_smem(span, warps);
     // the cells of the span: consecutive tiles' cells follow one another
     const int64_t base = tile * kSlotsPerCta, top = min(base + (int64_t)span * kSlotsPerCta, P.capacity);
     const int2 cc = __ldg(P.cta_cells + tile), ce = __ldg(P.cta_cells + (top - 1) / kSlotsPerCta);
     const int c0 = cc.x, nc = ce.x + ce.y - cc.x;
-    for (int i = threadIdx.x; i <= nc; i += kThreads64) sm.start[i] = P.start[c0 + i];
-    for (int i = threadIdx.x; i < nc; i += kThreads64) sm.count[i] = P.count[c0 + i];
+    for (int i = threadIdx.x; i <= nc; i += blockDim.x) sm.start[i] = P.start[c0 + i];
+    for (int i = threadIdx.x; i < nc; i += blockDim.x) sm.count[i] = P.count[c0 + i];
     __syncthreads();
     if (warp == 0) {  // items before each cell
         int before = 0;
@@ -412,11 +488,11 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
     }
     __syncthreads();
     const int total = sm.first[nc];
-    double* const coef = sm.coef[warp * (32 / kGroup64) + sub];
-    const float reach2 = planet_reach2(g);
+    double* const coef = sm.coef + (warp * kWarpItems64 + sub) * kCoefStride64;
+    const float reach = planet_reach(g);
     uint32_t nmig = 0, nrem = 0;
 
-    for (int j0 = (part * kWarps64 + warp) * (32 / kGroup64); j0 < total; j0 += parts * kItems64) {
+    for (int j0 = (part * warps + warp) * kWarpItems64; j0 < total; j0 += parts * warps * kWarpItems64) {
         const int j = min(j0 + sub, total - 1);
         int i = 0;
         {
@@ -439,14 +515,14 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
         cell_coords(g, cell, c.x, c.y, c.z);
         {   // lane 0, 1, 2 of the group: the axis' centre
             const double cen = gl < 3 ? cell_centre(g, gl, gl == 0 ? c.x : gl == 1 ? c.y : c.z) : 0.0;
-            const float gap2 = gl < 3 ? planet_gap2(g, gl, cen) : 0.f;
-            float gap = 0.f;
+            const float mine = gl < 3 ? planet_gap(g, gl, cen) : 0.f;
+            float gap[3];
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
                 c.cen[b] = __shfl_sync(kAll, cen, b, kGroup64);
-                gap += __shfl_sync(kAll, gap2, b, kGroup64);
+                gap[b] = __shfl_sync(kAll, mine, b, kGroup64);
             }
-            c.near_planet = !(gap > reach2);
+            planet_flags(g, gap, reach, c);
         }
         if (kStep && kField) {  // lane k: corner k, then coefficient k
             const double* f = corner_field(g, c.x, c.y, c.z, gl);
@@ -573,27 +649,25 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
 
 // Block (span, part) of population blockIdx.z of the set.
 template <bool kStep, bool kField, bool kDep>
-__global__ void __launch_bounds__(kThreads64)
+__global__ void __launch_bounds__(32 * kMaxWarps64, kDep ? 3 : 5)
     k_push64(Geom g, const __grid_constant__ PopSet<double> S, const __grid_constant__ Push64Set pcs, int span,
              int item) {
-    __shared__ Push64Smem sm;
     const Pop<double>& P = S.p[blockIdx.z];
     const int64_t tile = (int64_t)blockIdx.x * span;
     if (tile * kSlotsPerCta >= P.capacity) return;
-    push64_body<kStep, kField, kDep>(g, P, pcs.c[blockIdx.z], tile, span, blockIdx.y, gridDim.y, item, sm);
+    push64_body<kStep, kField, kDep>(g, P, pcs.c[blockIdx.z], tile, span, blockIdx.y, gridDim.y, item);
 }
 
 // Batched: cta_job[blockIdx.x] = (job, tile of the job); the span starts at
 // every span-th tile of a job.
 template <bool kStep, bool kField, bool kDep>
-__global__ void __launch_bounds__(kThreads64)
+__global__ void __launch_bounds__(32 * kMaxWarps64, kDep ? 3 : 5)
     k_push64_batch(const PopJob<double>* __restrict__ jobs, const int2* __restrict__ cta_job, int span, int item) {
-    __shared__ Push64Smem sm;
     __shared__ PopJob<double> job;
     const int2 cj = __ldg(cta_job + blockIdx.x);
     if (cj.y % span != 0) return;
     load_job(job, jobs + cj.x);
-    push64_body<kStep, kField, kDep>(job.g, job.P, job.pc, cj.y, span, blockIdx.y, gridDim.y, item, sm);
+    push64_body<kStep, kField, kDep>(job.g, job.P, job.pc, cj.y, span, blockIdx.y, gridDim.y, item);
 }
 
 // ---- particles that waited for a slot ---------------------------------------------
