@@ -202,9 +202,8 @@ int launch_cell_coef(const Geom& g, float* coef, cudaStream_t st) {
     const float scale = (g.flags & 2u) ? (float)(1.0 / g.vol) : 1.0f;
     if (g.node32) {
         const int64_t n = (int64_t)g.sx * g.sy * g.sz;
-        int64_t blocks = (n + 127) / 128;
-        if (blocks > 152 * 16) blocks = 152 * 16;
-        k_cell_coef32<<<(unsigned)blocks, 128, 0, st>>>(g.node32, g.sx, g.sy, g.sz, scale, coef);
+        k_cell_coef32<<<(unsigned)((n + kCoefCells - 1) / kCoefCells), kCoefThreads, 0, st>>>(
+            reinterpret_cast<const float*>(g.node32), g.sx, g.sy, g.sz, scale, coef);
         return 1;
     }
     const int64_t n = (int64_t)g.sx * g.sy * g.sz * 6;
