@@ -203,6 +203,8 @@ struct InstJob {
     int job0, njobs;        // its populations: PopJob entries [job0, job0 + njobs)
     uint32_t pend_limit;    // waiting particles above which it is re-laid out
     int div8;               // J = Js / vol / 8
+    int mul_vol;            // vol is a power of two: the product with inv_vol is the quotient
+    double inv_vol;         // 1 / vol
     int refresh_b;          // leapfrog refreshes node B from Bc
     float* cellcoef;        // FP32 field-gather coefficients (writable view)
     double coef_scale;      // 1 / vol with the gather normalisation, else 1

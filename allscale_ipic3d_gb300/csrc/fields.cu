@@ -47,8 +47,8 @@ __device__ __forceinline__ void ghost_body(double* g, int n, int per, int64_t t0
 struct SolverArgs {
     int s;                // cells per axis (cubic)
     double dt, c;
-    double wx, wy, wz;
-    double iwx, iwy, iwz;  // 1 / w (the multiplying solvers)
+    double w[3];
+    double iw[3];         // 1 / w
     float4* n32;          // FP32 node copy {Ex,Ey,Ez,0},{Bx,By,Bz,0} kept current (FP32 path), or null
     double* field;        // (s+3)^3 x 9
     double* bc;           // (s+2)^3 x 3
@@ -58,100 +58,117 @@ struct SolverArgs {
     // normalised on the read exactly as k_j_finalize (jmode 1: / vol [/ 8])
     // or k_j_finalize_mul (jmode 2: * jinv) would store them
     int jmode, jdiv8;
-    double jvol, jinv;
+    double jvol, jivol;   // vol, 1 / vol
+    double jinv;          // 1 / vol [/ 8]
 };
 
-// J of node m (per axis in [0, s]) as the J finalisation stores it: the sum
-// over the node's images {0, s} on each axis where it lies on the boundary,
-// in the finalisation's order, then normalised.
-__device__ __forceinline__ void final_j(const SolverArgs& A, int mx, int my, int mz, double (&a)[3]) {
+// Component `comp` of J at node m (per axis in [0, s]) as the J finalisation
+// stores it: the sum over the node's images {0, s} on each axis where it lies
+// on the boundary, in the finalisation's order, then normalised.
+__device__ __forceinline__ double final_j(const SolverArgs& A, int mx, int my, int mz, int comp) {
     const int s = A.s, nd = A.s + 1;
     const int x = mx == s ? 0 : mx, y = my == s ? 0 : my, z = mz == s ? 0 : mz;
     const int nxs = x == 0 ? 2 : 1, nys = y == 0 ? 2 : 1, nzs = z == 0 ? 2 : 1;
-    a[0] = a[1] = a[2] = 0.0;
+    double a = soft::plus_zero(A.J[3 * fidx(nd, x, y, z) + comp]);
     for (int i = 0; i < nxs; ++i)
         for (int j = 0; j < nys; ++j)
-            for (int k = 0; k < nzs; ++k) {
-                const double* p = A.J + 3 * fidx(nd, i ? s : x, j ? s : y, k ? s : z);
-                a[0] += p[0]; a[1] += p[1]; a[2] += p[2];
-            }
-    for (int c = 0; c < 3; ++c) {
-        if (A.jmode == 1) {
-            a[c] = a[c] / A.jvol;
-            if (A.jdiv8) a[c] = a[c] / 8.0;
-        } else {
-            a[c] *= A.jinv;
-        }
-    }
-}
-
-__device__ __forceinline__ void read_j(const SolverArgs& A, int mx, int my, int mz, double (&a)[3]) {
-    if (A.jmode == 0) {
-        const double* p = A.J + 3 * fidx(A.s + 1, mx, my, mz);
-        a[0] = p[0]; a[1] = p[1]; a[2] = p[2];
+            for (int k = 0; k < nzs; ++k)
+                if (i + j + k) a += A.J[3 * fidx(nd, i ? s : x, j ? s : y, k ? s : z) + comp];
+    if (A.jmode == 1) {
+        a = soft::quotient(a, A.jvol, A.jivol, 0);
+        if (A.jdiv8) a = a * 0.125;
     } else {
-        final_j(A, mx, my, mz, a);
+        a = a * A.jinv;
     }
+    return a;
 }
 
-// d / w: the reference's division (kMul false) or the product with 1 / w
-// (kMul: equal bit for bit when w is a power of two; the FP32 path's solver
-// otherwise)
+__device__ __forceinline__ double read_j(const SolverArgs& A, int mx, int my, int mz, int comp) {
+    return A.jmode == 0 ? A.J[3 * fidx(A.s + 1, mx, my, mz) + comp] : final_j(A, mx, my, mz, comp);
+}
+
+// d / w of an axis: the reference's division, correctly rounded (kMul false),
+// or the product with 1 / w (kMul: equal bit for bit when w is a power of two;
+// the FP32 path's solver otherwise)
 template <bool kMul>
 __device__ __forceinline__ double over(double d, double w, double iw) {
-    return kMul ? d * iw : d / w;
+    return kMul ? d * iw : soft::quotient(d, w, iw, 0);
 }
 
+// The leapfrog, the node refresh and the J finalisation run a thread per node
+// and component, components fastest: neighbouring lanes read neighbouring
+// doubles, and three times the threads hide the latency of grids that fill
+// the SMs once. A block works on a row (x, y) of the grid, so a thread divides
+// by 3 only (a flat index costs two divisions by the grid size, as much as
+// the update itself). The grids' traffic (72-byte records of which a kernel
+// needs 24) bounds them; taking a third of the FP64 instructions out changed
+// nothing. With the L2 warm, as in a step: 0.336 -> 0.325 ms a step at 48^3,
+// a thread per node before.
+struct NodeComp {
+    int x, y, z, a, b, c;  // (a, b, c): the component and the next two axes, cyclic
+};
+// item r of row (x, y), coordinates from 1
+__device__ __forceinline__ NodeComp node_comp(int x, int y, int r) {
+    NodeComp p;
+    const unsigned z = (unsigned)r / 3u;
+    p.x = x + 1;
+    p.y = y + 1;
+    p.z = (int)z + 1;
+    p.a = r - 3 * (int)z;
+    p.b = p.a == 2 ? 0 : p.a + 1;
+    p.c = p.a == 0 ? 2 : p.a - 1;
+    return p;
+}
+
+__device__ __forceinline__ double pick(int a, const double (&v)[3]) { return a == 0 ? v[0] : a == 1 ? v[1] : v[2]; }
+
 // E at pos in [1, s+2)^3 from Bc(pos), Bc(pos - e_i) and J(pos - 1).
-template <bool kMul = false>
-__device__ __forceinline__ void leapfrog_e_body(SolverArgs A, int64_t t0, int64_t stride) {
-    const int n = A.s + 1;  // nodes per axis in the updated box
-    const int64_t total = (int64_t)n * n * n;
+template <bool kMul>
+__device__ __forceinline__ void leapfrog_e_point(const SolverArgs& A, const NodeComp& p) {
+    const int nb = A.s + 2, nf = A.s + 3;
+    const int64_t sx = 3 * (int64_t)nb * nb, sy = 3 * (int64_t)nb, sz = 3;
+    const double* B0 = A.bc + 3 * fidx(nb, p.x, p.y, p.z);
+    const double* Bb = B0 - (p.b == 0 ? sx : p.b == 1 ? sy : sz);
+    const double* Bc = B0 - (p.c == 0 ? sx : p.c == 1 ? sy : sz);
+    const double wb = pick(p.b, A.w), iwb = pick(p.b, A.iw), wc = pick(p.c, A.w), iwc = pick(p.c, A.iw);
+    const double J = read_j(A, p.x - 1, p.y - 1, p.z - 1, p.a);
+    const int64_t f = fidx(nf, p.x, p.y, p.z);
+    double* E = A.field + 9 * f + p.a;
     const double c2 = A.c * A.c;
-    for (int64_t t = t0; t < total; t += stride) {
-        int x, y, z;
-        split3(t, n, n, x, y, z);
-        ++x; ++y; ++z;
-        const int nb = A.s + 2, nf = A.s + 3;
-        const double* B0 = A.bc + 3 * fidx(nb, x, y, z);
-        const double* Bxm = A.bc + 3 * fidx(nb, x - 1, y, z);
-        const double* Bym = A.bc + 3 * fidx(nb, x, y - 1, z);
-        const double* Bzm = A.bc + 3 * fidx(nb, x, y, z - 1);
-        double J[3];
-        read_j(A, x - 1, y - 1, z - 1, J);
-        double* E = A.field + 9 * fidx(nf, x, y, z);
-        E[0] = E[0] + A.dt * (c2 * (over<kMul>(B0[2] - Bym[2], A.wy, A.iwy) - over<kMul>(B0[1] - Bzm[1], A.wz, A.iwz)) -
-                              J[0]);
-        E[1] = E[1] + A.dt * (c2 * (over<kMul>(B0[0] - Bzm[0], A.wz, A.iwz) - over<kMul>(B0[2] - Bxm[2], A.wx, A.iwx)) -
-                              J[1]);
-        E[2] = E[2] + A.dt * (c2 * (over<kMul>(B0[1] - Bxm[1], A.wx, A.iwx) - over<kMul>(B0[0] - Bym[0], A.wy, A.iwy)) -
-                              J[2]);
-        if (A.n32) A.n32[2 * fidx(nf, x, y, z)] = make_float4((float)E[0], (float)E[1], (float)E[2], 0.f);
-    }
+    const double e =
+        *E + A.dt * (c2 * (over<kMul>(B0[p.c] - Bb[p.c], wb, iwb) - over<kMul>(B0[p.b] - Bc[p.b], wc, iwc)) - J);
+    *E = e;
+    if (A.n32) reinterpret_cast<float*>(A.n32 + 2 * f)[p.a] = (float)e;
 }
 
 // Bc at pos in [1, s+1)^3 from the new E at pos and pos + e_i.
-template <bool kMul = false>
-__device__ __forceinline__ void leapfrog_b_body(SolverArgs A, int64_t t0, int64_t stride) {
-    const int n = A.s;
-    const int64_t total = (int64_t)n * n * n;
-    for (int64_t t = t0; t < total; t += stride) {
-        int x, y, z;
-        split3(t, n, n, x, y, z);
-        ++x; ++y; ++z;
-        const int nb = A.s + 2, nf = A.s + 3;
-        const double* E0 = A.field + 9 * fidx(nf, x, y, z);
-        const double* Ex = A.field + 9 * fidx(nf, x + 1, y, z);
-        const double* Ey = A.field + 9 * fidx(nf, x, y + 1, z);
-        const double* Ez = A.field + 9 * fidx(nf, x, y, z + 1);
-        double* B = A.bc + 3 * fidx(nb, x, y, z);
-        B[0] = B[0] - A.dt * (over<kMul>(Ey[2] - E0[2], A.wy, A.iwy) - over<kMul>(Ez[1] - E0[1], A.wz, A.iwz));
-        B[1] = B[1] - A.dt * (over<kMul>(Ez[0] - E0[0], A.wz, A.iwz) - over<kMul>(Ex[2] - E0[2], A.wx, A.iwx));
-        B[2] = B[2] - A.dt * (over<kMul>(Ex[1] - E0[1], A.wx, A.iwx) - over<kMul>(Ey[0] - E0[0], A.wy, A.iwy));
-    }
+template <bool kMul>
+__device__ __forceinline__ void leapfrog_b_point(const SolverArgs& A, const NodeComp& p) {
+    const int nb = A.s + 2, nf = A.s + 3;
+    const int64_t sx = 9 * (int64_t)nf * nf, sy = 9 * (int64_t)nf, sz = 9;
+    const double* E0 = A.field + 9 * fidx(nf, p.x, p.y, p.z);
+    const double* Eb = E0 + (p.b == 0 ? sx : p.b == 1 ? sy : sz);
+    const double* Ec = E0 + (p.c == 0 ? sx : p.c == 1 ? sy : sz);
+    const double wb = pick(p.b, A.w), iwb = pick(p.b, A.iw), wc = pick(p.c, A.w), iwc = pick(p.c, A.iw);
+    double* B = A.bc + 3 * fidx(nb, p.x, p.y, p.z) + p.a;
+    *B = *B - A.dt * (over<kMul>(Eb[p.c] - E0[p.c], wb, iwb) - over<kMul>(Ec[p.b] - E0[p.b], wc, iwc));
+}
+
+// node B at pos in [1, s+2)^3 = 1/8 sum of Bc at pos - (i,j,k) (interpC2N)
+__device__ __forceinline__ void interp_c2n_point(const SolverArgs& A, const NodeComp& p) {
+    const int64_t nb = A.s + 2;
+    const double* B0 = A.bc + 3 * fidx((int)nb, p.x, p.y, p.z) + p.a;
+    double a = soft::plus_zero(B0[0]);
+#pragma unroll
+    for (int m = 1; m < 8; ++m) a = a + B0[-3 * (((m >> 2) * nb + ((m >> 1) & 1)) * nb + (m & 1))];
+    const double b = .125 * a;
+    const int64_t f = fidx(A.s + 3, p.x, p.y, p.z);
+    A.field[9 * f + 3 + p.a] = b;
+    if (A.n32) reinterpret_cast<float*>(A.n32 + 2 * f + 1)[p.a] = (float)b;
 }
 
 // computeCurlB (field.h:162-193) at node pos from the 8 Bc at pos - (i,j,k).
+template <bool kMul>
 __device__ __forceinline__ void curl_b(const SolverArgs& A, int x, int y, int z, double& cx, double& cy, double& cz) {
     const int nb = A.s + 2;
     double b[2][2][2][3];
@@ -165,18 +182,19 @@ __device__ __forceinline__ void curl_b(const SolverArgs& A, int x, int y, int z,
                 b[i][j][k][0] = p[0]; b[i][j][k][1] = p[1]; b[i][j][k][2] = p[2];
             }
     // d/dy of z: (j=0) - (j=1) over the 4 (i,k); d/dz of y: (k=0) - (k=1); ...
-    double zdy = .25 * (b[0][0][0][2] - b[0][1][0][2] + b[0][0][1][2] - b[0][1][1][2] + b[1][0][0][2] - b[1][1][0][2] + b[1][0][1][2] - b[1][1][1][2]) / A.wy;
-    double ydz = .25 * (b[0][0][0][1] - b[0][0][1][1] + b[1][0][0][1] - b[1][0][1][1] + b[0][1][0][1] - b[0][1][1][1] + b[1][1][0][1] - b[1][1][1][1]) / A.wz;
+    double zdy = over<kMul>(.25 * (b[0][0][0][2] - b[0][1][0][2] + b[0][0][1][2] - b[0][1][1][2] + b[1][0][0][2] - b[1][1][0][2] + b[1][0][1][2] - b[1][1][1][2]), A.w[1], A.iw[1]);
+    double ydz = over<kMul>(.25 * (b[0][0][0][1] - b[0][0][1][1] + b[1][0][0][1] - b[1][0][1][1] + b[0][1][0][1] - b[0][1][1][1] + b[1][1][0][1] - b[1][1][1][1]), A.w[2], A.iw[2]);
     cx = zdy - ydz;
-    double xdz = .25 * (b[0][0][0][0] - b[0][0][1][0] + b[1][0][0][0] - b[1][0][1][0] + b[0][1][0][0] - b[0][1][1][0] + b[1][1][0][0] - b[1][1][1][0]) / A.wz;
-    double zdx = .25 * (b[0][0][0][2] - b[1][0][0][2] + b[0][0][1][2] - b[1][0][1][2] + b[0][1][0][2] - b[1][1][0][2] + b[0][1][1][2] - b[1][1][1][2]) / A.wx;
+    double xdz = over<kMul>(.25 * (b[0][0][0][0] - b[0][0][1][0] + b[1][0][0][0] - b[1][0][1][0] + b[0][1][0][0] - b[0][1][1][0] + b[1][1][0][0] - b[1][1][1][0]), A.w[2], A.iw[2]);
+    double zdx = over<kMul>(.25 * (b[0][0][0][2] - b[1][0][0][2] + b[0][0][1][2] - b[1][0][1][2] + b[0][1][0][2] - b[1][1][0][2] + b[0][1][1][2] - b[1][1][1][2]), A.w[0], A.iw[0]);
     cy = xdz - zdx;
-    double ydx = .25 * (b[0][0][0][1] - b[1][0][0][1] + b[0][0][1][1] - b[1][0][1][1] + b[0][1][0][1] - b[1][1][0][1] + b[0][1][1][1] - b[1][1][1][1]) / A.wx;
-    double xdy = .25 * (b[0][0][0][0] - b[0][1][0][0] + b[0][0][1][0] - b[0][1][1][0] + b[1][0][0][0] - b[1][1][0][0] + b[1][0][1][0] - b[1][1][1][0]) / A.wy;
+    double ydx = over<kMul>(.25 * (b[0][0][0][1] - b[1][0][0][1] + b[0][0][1][1] - b[1][0][1][1] + b[0][1][0][1] - b[1][1][0][1] + b[0][1][1][1] - b[1][1][1][1]), A.w[0], A.iw[0]);
+    double xdy = over<kMul>(.25 * (b[0][0][0][0] - b[0][1][0][0] + b[0][0][1][0] - b[0][1][1][0] + b[1][0][0][0] - b[1][1][0][0] + b[1][0][1][0] - b[1][1][1][0]), A.w[1], A.iw[1]);
     cz = ydx - xdy;
 }
 
 // computeCurlE (field.h:198-229) at centre pos from the 8 node E at pos + (i,j,k).
+template <bool kMul>
 __device__ __forceinline__ void curl_e(const SolverArgs& A, int x, int y, int z, double& cx, double& cy, double& cz) {
     const int nf = A.s + 3;
     double e[2][2][2][3];
@@ -189,17 +207,18 @@ __device__ __forceinline__ void curl_e(const SolverArgs& A, int x, int y, int z,
                 const double* p = A.field + 9 * fidx(nf, x + i, y + j, z + k);
                 e[i][j][k][0] = p[0]; e[i][j][k][1] = p[1]; e[i][j][k][2] = p[2];
             }
-    double zdy = .25 * (e[0][1][0][2] - e[0][0][0][2] + e[0][1][1][2] - e[0][0][1][2] + e[1][1][0][2] - e[1][0][0][2] + e[1][1][1][2] - e[1][0][1][2]) / A.wy;
-    double ydz = .25 * (e[0][0][1][1] - e[0][0][0][1] + e[1][0][1][1] - e[1][0][0][1] + e[0][1][1][1] - e[0][1][0][1] + e[1][1][1][1] - e[1][1][0][1]) / A.wz;
+    double zdy = over<kMul>(.25 * (e[0][1][0][2] - e[0][0][0][2] + e[0][1][1][2] - e[0][0][1][2] + e[1][1][0][2] - e[1][0][0][2] + e[1][1][1][2] - e[1][0][1][2]), A.w[1], A.iw[1]);
+    double ydz = over<kMul>(.25 * (e[0][0][1][1] - e[0][0][0][1] + e[1][0][1][1] - e[1][0][0][1] + e[0][1][1][1] - e[0][1][0][1] + e[1][1][1][1] - e[1][1][0][1]), A.w[2], A.iw[2]);
     cx = zdy - ydz;
-    double xdz = .25 * (e[0][0][1][0] - e[0][0][0][0] + e[1][0][1][0] - e[1][0][0][0] + e[0][1][1][0] - e[0][1][0][0] + e[1][1][1][0] - e[1][1][0][0]) / A.wz;
-    double zdx = .25 * (e[1][0][0][2] - e[0][0][0][2] + e[1][0][1][2] - e[0][0][1][2] + e[1][1][0][2] - e[0][1][0][2] + e[1][1][1][2] - e[0][1][1][2]) / A.wx;
+    double xdz = over<kMul>(.25 * (e[0][0][1][0] - e[0][0][0][0] + e[1][0][1][0] - e[1][0][0][0] + e[0][1][1][0] - e[0][1][0][0] + e[1][1][1][0] - e[1][1][0][0]), A.w[2], A.iw[2]);
+    double zdx = over<kMul>(.25 * (e[1][0][0][2] - e[0][0][0][2] + e[1][0][1][2] - e[0][0][1][2] + e[1][1][0][2] - e[0][1][0][2] + e[1][1][1][2] - e[0][1][1][2]), A.w[0], A.iw[0]);
     cy = xdz - zdx;
-    double ydx = .25 * (e[1][0][0][1] - e[0][0][0][1] + e[1][0][1][1] - e[0][0][1][1] + e[1][1][0][1] - e[0][1][0][1] + e[1][1][1][1] - e[0][1][1][1]) / A.wx;
-    double xdy = .25 * (e[0][1][0][0] - e[0][0][0][0] + e[0][1][1][0] - e[0][0][1][0] + e[1][1][0][0] - e[1][0][0][0] + e[1][1][1][0] - e[1][0][1][0]) / A.wy;
+    double ydx = over<kMul>(.25 * (e[1][0][0][1] - e[0][0][0][1] + e[1][0][1][1] - e[0][0][1][1] + e[1][1][0][1] - e[0][1][0][1] + e[1][1][1][1] - e[0][1][1][1]), A.w[0], A.iw[0]);
+    double xdy = over<kMul>(.25 * (e[0][1][0][0] - e[0][0][0][0] + e[0][1][1][0] - e[0][0][1][0] + e[1][1][0][0] - e[1][0][0][0] + e[1][1][1][0] - e[1][0][1][0]), A.w[1], A.iw[1]);
     cz = ydx - xdy;
 }
 
+template <bool kMul = false>
 __device__ __forceinline__ void forward_e_body(SolverArgs A, int64_t t0, int64_t stride) {
     const int n = A.s + 1;
     const int64_t total = (int64_t)n * n * n;
@@ -208,9 +227,10 @@ __device__ __forceinline__ void forward_e_body(SolverArgs A, int64_t t0, int64_t
         split3(t, n, n, x, y, z);
         ++x; ++y; ++z;
         double cx, cy, cz;
-        curl_b(A, x, y, z, cx, cy, cz);
+        curl_b<kMul>(A, x, y, z, cx, cy, cz);
         double J[3];
-        read_j(A, x - 1, y - 1, z - 1, J);
+#pragma unroll
+        for (int a = 0; a < 3; ++a) J[a] = read_j(A, x - 1, y - 1, z - 1, a);
         double* E = A.field + 9 * fidx(A.s + 3, x, y, z);
         E[0] += (A.c * cx - J[0]) * A.dt;
         E[1] += (A.c * cy - J[1]) * A.dt;
@@ -219,6 +239,7 @@ __device__ __forceinline__ void forward_e_body(SolverArgs A, int64_t t0, int64_t
     }
 }
 
+template <bool kMul = false>
 __device__ __forceinline__ void forward_b_body(SolverArgs A, int64_t t0, int64_t stride) {
     const int n = A.s;
     const int64_t total = (int64_t)n * n * n;
@@ -227,7 +248,7 @@ __device__ __forceinline__ void forward_b_body(SolverArgs A, int64_t t0, int64_t
         split3(t, n, n, x, y, z);
         ++x; ++y; ++z;
         double cx, cy, cz;
-        curl_e(A, x, y, z, cx, cy, cz);
+        curl_e<kMul>(A, x, y, z, cx, cy, cz);
         double* B = A.bc + 3 * fidx(A.s + 2, x, y, z);
         B[0] -= A.c * cx * A.dt;
         B[1] -= A.c * cy * A.dt;
@@ -235,56 +256,48 @@ __device__ __forceinline__ void forward_b_body(SolverArgs A, int64_t t0, int64_t
     }
 }
 
-// node B at pos in [1, s+2)^3 = 1/8 sum of Bc at pos - (i,j,k)
-__device__ __forceinline__ void interp_c2n_body(SolverArgs A, int64_t t0, int64_t stride) {
-    const int n = A.s + 1;
-    const int64_t total = (int64_t)n * n * n;
-    for (int64_t t = t0; t < total; t += stride) {
-        int x, y, z;
-        split3(t, n, n, x, y, z);
-        ++x; ++y; ++z;
-        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-        for (int i = 0; i < 2; i++)
-            for (int j = 0; j < 2; j++)
-                for (int k = 0; k < 2; k++) {
-                    const double* p = A.bc + 3 * fidx(A.s + 2, x - i, y - j, z - k);
-                    a0 = a0 + p[0]; a1 = a1 + p[1]; a2 = a2 + p[2];
-                }
-        double* B = A.field + 9 * fidx(A.s + 3, x, y, z) + 3;
-        B[0] = .125 * a0; B[1] = .125 * a1; B[2] = .125 * a2;
-        if (A.n32) A.n32[2 * fidx(A.s + 3, x, y, z) + 1] = make_float4((float)B[0], (float)B[1], (float)B[2], 0.f);
-    }
-}
-
 // The gather form of the reference adds, at node index 0 and index s of an
 // axis, the same two cells (periodic wrap of the cell index): the final value
 // of a node is the sum of the raw deposits over its image set {0, s} on every
-// axis where it lies on the boundary. Then J = (Js / vol) [/ 8].
-__device__ __forceinline__ void j_finalize_body(int sx, int sy, int sz, double* J, double* rho, double vol, int div8,
-                                                int64_t t0, int64_t stride) {
-    const int64_t total = (int64_t)sx * sy * sz;
+// axis where it lies on the boundary. Then J = (Js / vol) [/ 8], correctly
+// rounded (kMul false), or the product with `inv` = 1 / vol [/ 8] (the FP32
+// path, and wherever vol is a power of two: then the product equals the
+// reference's quotients bit for bit). Item r of row (x, y): node z = r / 4,
+// component r % 4 (rho the last); the images' loads issued together (in
+// loops over the images, one after the other, 8^3 cells took 10 us, now 3.5).
+template <bool kMul>
+__device__ __forceinline__ void j_finalize_point(int sx, int sy, int sz, double* J, double* rho, double vol, double inv,
+                                                 int div8, int x, int y, int r) {
     const int ny = sy + 1, nz = sz + 1;
-    for (int64_t t = t0; t < total; t += stride) {
-        int x, y, z;
-        split3(t, sy, sz, x, y, z);
-        const int nxs = x == 0 ? 2 : 1, nys = y == 0 ? 2 : 1, nzs = z == 0 ? 2 : 1;
-        double a[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int i = 0; i < nxs; ++i)
-            for (int j = 0; j < nys; ++j)
-                for (int k = 0; k < nzs; ++k) {
-                    const int64_t n = ((int64_t)(i ? sx : x) * ny + (j ? sy : y)) * nz + (k ? sz : z);
-                    a[0] += J[3 * n]; a[1] += J[3 * n + 1]; a[2] += J[3 * n + 2]; a[3] += rho[n];
-                }
-        for (int c = 0; c < 4; ++c) {
-            a[c] = a[c] / vol;
-            if (div8) a[c] = a[c] / 8.0;
+    const int comp = r & 3, z = r >> 2;
+    double* const base = comp < 3 ? J + comp : rho;
+    const int64_t pitch = comp < 3 ? 3 : 1;
+    const auto normal = [&](double a) {
+        if (kMul) return a * inv;
+        a = soft::quotient(a, vol, inv, 0);  // inv = 1 / vol
+        return div8 ? a * 0.125 : a;
+    };
+    if (x != 0 && y != 0 && z != 0) {
+        double* p = base + pitch * (((int64_t)x * ny + y) * nz + z);
+        *p = normal(soft::plus_zero(*p));
+    } else {
+        int64_t n[8];
+        double v[8];
+        bool in[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            in[k] = (!(k & 4) || x == 0) && (!(k & 2) || y == 0) && (!(k & 1) || z == 0);
+            n[k] = pitch * (((int64_t)((k & 4) ? sx : x) * ny + ((k & 2) ? sy : y)) * nz + ((k & 1) ? sz : z));
+            if (in[k]) v[k] = base[n[k]];
         }
-        for (int i = 0; i < nxs; ++i)
-            for (int j = 0; j < nys; ++j)
-                for (int k = 0; k < nzs; ++k) {
-                    const int64_t n = ((int64_t)(i ? sx : x) * ny + (j ? sy : y)) * nz + (k ? sz : z);
-                    J[3 * n] = a[0]; J[3 * n + 1] = a[1]; J[3 * n + 2] = a[2]; rho[n] = a[3];
-                }
+        double a = 0.0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (in[k]) a += v[k];
+        a = normal(a);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (in[k]) base[n[k]] = a;
     }
 }
 
@@ -304,12 +317,10 @@ __host__ __device__ inline SolverArgs solver_args(const Geom& g) {
     A.s = g.sx;
     A.dt = g.dt;
     A.c = g.c;
-    A.wx = g.w[0];
-    A.wy = g.w[1];
-    A.wz = g.w[2];
-    A.iwx = 1.0 / g.w[0];
-    A.iwy = 1.0 / g.w[1];
-    A.iwz = 1.0 / g.w[2];
+    for (int a = 0; a < 3; ++a) {
+        A.w[a] = g.w[a];
+        A.iw[a] = g.inv_w[a];
+    }
     A.field = g.field;
     A.bc = g.bcfield;
     A.J = g.J;
@@ -317,6 +328,7 @@ __host__ __device__ inline SolverArgs solver_args(const Geom& g) {
     A.jmode = 0;
     A.jdiv8 = 0;
     A.jvol = g.vol;
+    A.jivol = 1.0;
     A.jinv = 1.0;
     return A;
 }
@@ -332,43 +344,31 @@ __global__ void k_ghost2(double* field, int nf, double* bc, int nb) {
     else
         ghost_body(bc, nb, 3, t - mf, (int64_t)(nb - 2) * (nb - 2) * 3);
 }
+// rows: block (., y, x), items of the row along the threads
+__device__ __forceinline__ int row_item() { return blockIdx.x * blockDim.x + threadIdx.x; }
 template <bool kMul>
-__global__ void k_leapfrog_e(SolverArgs A) { leapfrog_e_body<kMul>(A, grid_t0(), grid_stride()); }
+__global__ void k_leapfrog_e(SolverArgs A) {
+    const int r = row_item();
+    if (r < 3 * (A.s + 1)) leapfrog_e_point<kMul>(A, node_comp(blockIdx.z, blockIdx.y, r));
+}
 template <bool kMul>
-__global__ void k_leapfrog_b(SolverArgs A) { leapfrog_b_body<kMul>(A, grid_t0(), grid_stride()); }
-__global__ void k_forward_e(SolverArgs A) { forward_e_body(A, grid_t0(), grid_stride()); }
-__global__ void k_forward_b(SolverArgs A) { forward_b_body(A, grid_t0(), grid_stride()); }
-__global__ void k_interp_c2n(SolverArgs A) { interp_c2n_body(A, grid_t0(), grid_stride()); }
-__global__ void k_j_finalize(int sx, int sy, int sz, double* J, double* rho, double vol, int div8) {
-    j_finalize_body(sx, sy, sz, J, rho, vol, div8, grid_t0(), grid_stride());
+__global__ void k_leapfrog_b(SolverArgs A) {
+    const int r = row_item();
+    if (r < 3 * A.s) leapfrog_b_point<kMul>(A, node_comp(blockIdx.z, blockIdx.y, r));
 }
-// The same with the normalisation as one multiplication by `inv` (1 / vol
-// [/ 8]): for the FP32 path, and wherever vol is a power of two (then the
-// product equals the reference's quotients bit for bit).
-__global__ void k_j_finalize_mul(int sx, int sy, int sz, double* J, double* rho, double inv) {
-    const int64_t total = (int64_t)sx * sy * sz;
-    const int ny = sy + 1, nz = sz + 1;
-    for (int64_t t = grid_t0(); t < total; t += grid_stride()) {
-        int x, y, z;
-        split3(t, sy, sz, x, y, z);
-        const int nxs = x == 0 ? 2 : 1, nys = y == 0 ? 2 : 1, nzs = z == 0 ? 2 : 1;
-        double a[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int i = 0; i < nxs; ++i)
-            for (int j = 0; j < nys; ++j)
-                for (int k = 0; k < nzs; ++k) {
-                    const int64_t n = ((int64_t)(i ? sx : x) * ny + (j ? sy : y)) * nz + (k ? sz : z);
-                    a[0] += J[3 * n]; a[1] += J[3 * n + 1]; a[2] += J[3 * n + 2]; a[3] += rho[n];
-                }
-        for (int c = 0; c < 4; ++c) a[c] *= inv;
-        for (int i = 0; i < nxs; ++i)
-            for (int j = 0; j < nys; ++j)
-                for (int k = 0; k < nzs; ++k) {
-                    const int64_t n = ((int64_t)(i ? sx : x) * ny + (j ? sy : y)) * nz + (k ? sz : z);
-                    J[3 * n] = a[0]; J[3 * n + 1] = a[1]; J[3 * n + 2] = a[2]; rho[n] = a[3];
-                }
-    }
+__global__ void k_interp_c2n(SolverArgs A) {
+    const int r = row_item();
+    if (r < 3 * (A.s + 1)) interp_c2n_point(A, node_comp(blockIdx.z, blockIdx.y, r));
 }
-
+template <bool kMul>
+__global__ void k_j_finalize(int sx, int sy, int sz, double* J, double* rho, double vol, double inv, int div8) {
+    const int r = row_item();
+    if (r < 4 * sz) j_finalize_point<kMul>(sx, sy, sz, J, rho, vol, inv, div8, blockIdx.z, blockIdx.y, r);
+}
+template <bool kMul>
+__global__ void k_forward_e(SolverArgs A) { forward_e_body<kMul>(A, grid_t0(), grid_stride()); }
+template <bool kMul>
+__global__ void k_forward_b(SolverArgs A) { forward_b_body<kMul>(A, grid_t0(), grid_stride()); }
 // batched kernels: blockIdx.y is the universe, blockIdx.x strides over its
 // items (the grid is sized for the largest universe of the batch)
 __global__ void k_ghost_batch(const InstJob* jobs) {
@@ -376,11 +376,25 @@ __global__ void k_ghost_batch(const InstJob* jobs) {
     ghost_body(g.field, g.sx + 3, 9, grid_t0(), grid_stride());
     ghost_body(g.bcfield, g.sx + 2, 3, grid_t0(), grid_stride());
 }
+// item t of the rows of n x n x len: row (x, y), item r of it
+__device__ __forceinline__ void row_of(int64_t t, int n, int len, int& x, int& y, int& r) { split3(t, n, len, x, y, r); }
 __global__ void k_leapfrog_e_batch(const InstJob* jobs) {
-    leapfrog_e_body(solver_args(jobs[blockIdx.y].g), grid_t0(), grid_stride());
+    const SolverArgs A = solver_args(jobs[blockIdx.y].g);
+    const int n = A.s + 1;
+    for (int64_t t = grid_t0(); t < 3 * (int64_t)n * n * n; t += grid_stride()) {
+        int x, y, r;
+        row_of(t, n, 3 * n, x, y, r);
+        leapfrog_e_point<false>(A, node_comp(x, y, r));
+    }
 }
 __global__ void k_leapfrog_b_batch(const InstJob* jobs) {
-    leapfrog_b_body(solver_args(jobs[blockIdx.y].g), grid_t0(), grid_stride());
+    const SolverArgs A = solver_args(jobs[blockIdx.y].g);
+    const int n = A.s;
+    for (int64_t t = grid_t0(); t < 3 * (int64_t)n * n * n; t += grid_stride()) {
+        int x, y, r;
+        row_of(t, n, 3 * n, x, y, r);
+        leapfrog_b_point<false>(A, node_comp(x, y, r));
+    }
 }
 __global__ void k_forward_e_batch(const InstJob* jobs) {
     forward_e_body(solver_args(jobs[blockIdx.y].g), grid_t0(), grid_stride());
@@ -389,11 +403,26 @@ __global__ void k_forward_b_batch(const InstJob* jobs) {
     forward_b_body(solver_args(jobs[blockIdx.y].g), grid_t0(), grid_stride());
 }
 __global__ void k_interp_c2n_batch(const InstJob* jobs) {
-    interp_c2n_body(solver_args(jobs[blockIdx.y].g), grid_t0(), grid_stride());
+    const SolverArgs A = solver_args(jobs[blockIdx.y].g);
+    const int n = A.s + 1;
+    for (int64_t t = grid_t0(); t < 3 * (int64_t)n * n * n; t += grid_stride()) {
+        int x, y, r;
+        row_of(t, n, 3 * n, x, y, r);
+        interp_c2n_point(A, node_comp(x, y, r));
+    }
 }
 __global__ void k_j_finalize_batch(const InstJob* jobs) {
     const InstJob& b = jobs[blockIdx.y];
-    j_finalize_body(b.g.sx, b.g.sy, b.g.sz, b.g.J, b.g.rho, b.g.vol, b.div8, grid_t0(), grid_stride());
+    const Geom& g = b.g;
+    const double inv = b.div8 && b.mul_vol ? b.inv_vol * 0.125 : b.inv_vol;
+    for (int64_t t = grid_t0(); t < (int64_t)g.sx * g.sy * g.sz; t += grid_stride()) {
+        int x, y, z;
+        split3(t, g.sy, g.sz, x, y, z);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+            if (b.mul_vol) j_finalize_point<true>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol, inv, b.div8, x, y, 4 * z + a);
+            else j_finalize_point<false>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol, inv, b.div8, x, y, 4 * z + a);
+    }
 }
 
 // ---- compensated reductions ----------------------------------------------------
@@ -530,6 +559,18 @@ int launch_ghost(const Geom& g, cudaStream_t st) {
     return 1;
 }
 
+// The launch of a row kernel: nx x ny rows of `items`.
+struct Rows {
+    dim3 grid;
+    unsigned threads;
+};
+static Rows rows(int nx, int ny, int items) {
+    Rows r;
+    r.threads = (unsigned)(items < 256 ? (items + 31) / 32 * 32 : 256);
+    r.grid = dim3((items + r.threads - 1) / r.threads, ny, nx);
+    return r;
+}
+
 static bool pow2(double v) {
     int e = 0;
     return std::frexp(v, &e) == 0.5;
@@ -543,19 +584,15 @@ int launch_leapfrog(const Geom& g, bool refresh_node_b, bool exact, cudaStream_t
                     cudaEvent_t after_e) {
     SolverArgs A = solver_args(g);
     if (raw_j) set_raw_j(A, g, div8, exact);
-    const int64_t ne = (int64_t)(g.sx + 1) * (g.sx + 1) * (g.sx + 1);
     const bool mul = !exact || (pow2(g.w[0]) && pow2(g.w[1]) && pow2(g.w[2]));
-    if (mul) {
-        k_leapfrog_e<true><<<grid_for(ne, 256), 256, 0, st>>>(A);
-        if (after_e) cudaEventRecord(after_e, st);
-        k_leapfrog_b<true><<<grid_for((int64_t)g.sx * g.sx * g.sx, 256), 256, 0, st>>>(A);
-    } else {
-        k_leapfrog_e<false><<<grid_for(ne, 256), 256, 0, st>>>(A);
-        if (after_e) cudaEventRecord(after_e, st);
-        k_leapfrog_b<false><<<grid_for((int64_t)g.sx * g.sx * g.sx, 256), 256, 0, st>>>(A);
-    }
+    const Rows nodes = rows(g.sx + 1, g.sx + 1, 3 * (g.sx + 1)), cells = rows(g.sx, g.sx, 3 * g.sx);
+    if (mul) k_leapfrog_e<true><<<nodes.grid, nodes.threads, 0, st>>>(A);
+    else k_leapfrog_e<false><<<nodes.grid, nodes.threads, 0, st>>>(A);
+    if (after_e) cudaEventRecord(after_e, st);
+    if (mul) k_leapfrog_b<true><<<cells.grid, cells.threads, 0, st>>>(A);
+    else k_leapfrog_b<false><<<cells.grid, cells.threads, 0, st>>>(A);
     if (refresh_node_b) {
-        k_interp_c2n<<<grid_for(ne, 256), 256, 0, st>>>(A);
+        k_interp_c2n<<<nodes.grid, nodes.threads, 0, st>>>(A);
         return 3;
     }
     return 2;
@@ -565,29 +602,34 @@ int launch_forward(const Geom& g, cudaStream_t st, bool raw_j, bool div8, bool e
     SolverArgs A = solver_args(g);
     if (raw_j) set_raw_j(A, g, div8, exact);
     const int64_t ne = (int64_t)(g.sx + 1) * (g.sx + 1) * (g.sx + 1);
-    k_forward_e<<<grid_for(ne, 256), 256, 0, st>>>(A);
+    const int64_t nc = (int64_t)g.sx * g.sx * g.sx;
+    const bool mul = pow2(g.w[0]) && pow2(g.w[1]) && pow2(g.w[2]);  // the products are the quotients
+    if (mul) k_forward_e<true><<<grid_for(ne, 256), 256, 0, st>>>(A);
+    else k_forward_e<false><<<grid_for(ne, 256), 256, 0, st>>>(A);
     if (after_e) cudaEventRecord(after_e, st);
-    k_forward_b<<<grid_for((int64_t)g.sx * g.sx * g.sx, 256), 256, 0, st>>>(A);
-    k_interp_c2n<<<grid_for(ne, 256), 256, 0, st>>>(A);
+    if (mul) k_forward_b<true><<<grid_for(nc, 256), 256, 0, st>>>(A);
+    else k_forward_b<false><<<grid_for(nc, 256), 256, 0, st>>>(A);
+    const Rows nodes = rows(g.sx + 1, g.sx + 1, 3 * (g.sx + 1));
+    k_interp_c2n<<<nodes.grid, nodes.threads, 0, st>>>(A);
     return 3;
 }
 
 static void set_raw_j(SolverArgs& A, const Geom& g, bool div8, bool exact) {
     A.jdiv8 = div8 ? 1 : 0;
     A.jvol = g.vol;
+    A.jivol = 1.0 / g.vol;
     A.jinv = div8 ? 1.0 / g.vol / 8.0 : 1.0 / g.vol;
     A.jmode = exact && !pow2(g.vol) ? 1 : 2;  // launch_j_finalize's choice
 }
 
 int launch_j_finalize(const Geom& g, bool div8, bool exact, cudaStream_t st) {
-    if (exact && !pow2(g.vol)) {  // vol = 2^k: 1 / vol is exact
-        k_j_finalize<<<grid_for((int64_t)g.sx * g.sy * g.sz, 256), 256, 0, st>>>(g.sx, g.sy, g.sz, g.J, g.rho,
-                                                                                 g.vol, div8 ? 1 : 0);
-    } else {
-        const double inv = div8 ? 1.0 / g.vol / 8.0 : 1.0 / g.vol;
-        k_j_finalize_mul<<<grid_for((int64_t)g.sx * g.sy * g.sz, 256), 256, 0, st>>>(g.sx, g.sy, g.sz, g.J, g.rho,
-                                                                                     inv);
-    }
+    const Rows r = rows(g.sx, g.sy, 4 * g.sz);
+    if (exact && !pow2(g.vol))  // vol = 2^k: 1 / vol is exact
+        k_j_finalize<false><<<r.grid, r.threads, 0, st>>>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol, 1.0 / g.vol,
+                                                          div8 ? 1 : 0);
+    else
+        k_j_finalize<true><<<r.grid, r.threads, 0, st>>>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol,
+                                                  div8 ? 1.0 / g.vol / 8.0 : 1.0 / g.vol, div8 ? 1 : 0);
     return 1;
 }
 
@@ -606,7 +648,7 @@ int launch_ghost_batch(const InstJob* jobs, int ninst, int max_s, cudaStream_t s
 
 int launch_leapfrog_batch(const InstJob* jobs, int ninst, int max_s, bool refresh_node_b, cudaStream_t st) {
     const int64_t ne = (int64_t)(max_s + 1) * (max_s + 1) * (max_s + 1);
-    const unsigned gx = grid_for(ne, 256, 64);
+    const unsigned gx = grid_for(3 * ne, 256, 192);
     k_leapfrog_e_batch<<<dim3(gx, ninst), 256, 0, st>>>(jobs);
     k_leapfrog_b_batch<<<dim3(gx, ninst), 256, 0, st>>>(jobs);
     if (!refresh_node_b) return 2;

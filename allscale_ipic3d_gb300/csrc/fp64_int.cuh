@@ -169,6 +169,9 @@ IPG_HD Num add_positive(const Num& a, const Num& b) {
 // w = 2^k within a range where 1 / w is exact and normal
 IPG_HD bool power_of_two(double w) { return regular(w, 900) && w > 0 && (bits_of(w) & 0xfffffffffffffull) == 0; }
 
+// 0.0 + x: x, except that -0 becomes +0
+IPG_HD double plus_zero(double x) { return bits_of(x) == 0x8000000000000000ull ? 0.0 : x; }
+
 IPG_HD double fused(double a, double b, double c) {
 #ifdef __CUDA_ARCH__
     return __fma_rn(a, b, c);

@@ -2117,6 +2117,8 @@ int batch_tables(ipic3d_batch* b) {
         I.njobs = (int)pops_of<T>(c).size();
         I.pend_limit = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(64, c->particles_hint / 200), 0xffffffffu);
         I.div8 = (cfg.flags & IPIC3D_F_J_DIV8) ? 1 : 0;
+        I.mul_vol = soft::power_of_two(c->g.vol);
+        I.inv_vol = 1.0 / c->g.vol;
         I.refresh_b = (cfg.flags & IPIC3D_F_REFRESH_NODE_B) ? 1 : 0;
         I.cellcoef = c->cellcoef;
         I.coef_scale = (cfg.flags & IPIC3D_F_GATHER_DIV_VOL) ? 1.0 / c->g.vol : 1.0;

@@ -45,6 +45,7 @@ int main(int argc, char** argv) {
         bad += quotient(a, w, 1.0 / w, power_of_two(w)) != a / w;
         bad += quotient(a, 0.125, 8.0, power_of_two(0.125)) != a / 0.125;
         bad += std::signbit(quotient(-0.0, w, 1.0 / w, 0)) != std::signbit(-0.0 / w);
+        bad += bits_of(plus_zero(-0.0)) != bits_of(0.0 + -0.0) || plus_zero(a) != a;
         bool sure = false;
         const double p = pack(pow25(unpack(std::fabs(a)), sure));
         const double out[3] = {bad, p, sure ? 1.0 : 0.0};
