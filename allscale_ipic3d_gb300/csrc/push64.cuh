@@ -68,7 +68,7 @@ __device__ __forceinline__ double reciprocal(double d) {
     return __fma_rn(y, __fma_rn(e, e, e), y);
 }
 
-// r2^(-5/2): y = r2^(-1/2) by y (1 + e / 2 + 3 e^2 / 8), e = 1 - r2 y^2, and
+// r2^(-5/2) out of the integer path's range: y = r2^(-1/2) by y (1 + e / 2 + 3 e^2 / 8), e = 1 - r2 y^2, and
 // one correction of y^5 from the residual of y^2
 __device__ __forceinline__ double inverse_pow25(double r2) {
     double y = seed_rsqrt(r2);
@@ -80,26 +80,85 @@ __device__ __forceinline__ double inverse_pow25(double r2) {
     return __fma_rn(f, __dmul_rn(2.5, d), f);
 }
 
-// The trilinear polynomial about the cell centre: coefficients of 1, x, y,
-// xy, z, xz, yz, xyz (index = bits x | y << 1 | z << 2).
-__device__ __forceinline__ double poly64(const double* c, double x, double y, double z) {
-    const double a = __fma_rn(y, c[7], c[5]);
-    double b = __fma_rn(y, c[3], c[1]);
-    b = __fma_rn(z, a, b);
-    const double gz = __fma_rn(z, c[6], c[2]);
-    double r = __fma_rn(y, gz, c[0]);
-    r = __fma_rn(z, c[4], r);
-    return __fma_rn(x, b, r);
-}
+// The field of a cell in 64-bit fixed point. A component's 8 corner values
+// share the largest one's exponent e_max: fixed = value 2^(1081 - e_max), below
+// 2^59, so that one unit is 2^-59 of the largest corner (FP64's own rounding
+// is 2^-53 of it). The trilinear polynomial's coefficients are differences of
+// these integers, exact, and the position in the cell is a 64-bit fraction:
+// a product is the high half of 64 x 64 bits. Seven of them and seven sums per
+// component take about 150 integer-pipe cycles per warp; the seven FP64
+// multiply-adds they replace took 448 of the FP64 pipe, which bounds the
+// push.
 
-// Coefficient k of the polynomial through corner values: per axis the mean
-// (bit clear) or the difference (bit set) of the two ends. The sums first,
-// then the halves of the means, an exact scaling.
-__device__ __forceinline__ double mean_scale(int k) { return k == 7 ? 1.0 : 1.0 / (double)(1 << (3 - __popc(k))); }
+// coefficients of 1, x, y, xy, z, xz, yz, xyz (index = bits x | y << 1 | z << 2)
+__device__ __forceinline__ int64_t scaled(int64_t c, uint64_t r) {  // floor(c r / 2^64)
+    return (int64_t)(__umul64hi((uint64_t)c, r) - (c < 0 ? r : 0));
+}
+__device__ __forceinline__ int64_t poly_fixed(const int64_t* c, uint64_t x, uint64_t y, uint64_t z) {
+    const int64_t xz = c[5] + scaled(c[7], y);
+    const int64_t gx = c[1] + scaled(c[3], y) + scaled(xz, z);
+    const int64_t gy = c[2] + scaled(c[6], z);
+    return c[0] + scaled(c[4], z) + scaled(gy, y) + scaled(gx, x);
+}
+// v with exponent e as fixed point for e_max >= e
+__device__ __forceinline__ int64_t to_fixed(double v, int e_max) {
+    const soft::Num n = soft::unpack(v);
+    const int d = e_max - n.e;
+    const int64_t t = n.e == 0 || d > 59 ? 0 : (int64_t)((n.m << 6) >> d);
+    return n.sign ? -t : t;
+}
+__device__ __forceinline__ double from_fixed(int64_t v, int e_max) {
+    if (v == 0) return 0.0;
+    const uint64_t a = v < 0 ? (uint64_t)-v : (uint64_t)v;
+    const int n = __clzll((long long)a);
+    const uint64_t m = a << n;
+    soft::Num r;
+    r.m = (m >> 11) + ((m >> 10) & 1);
+    r.e = e_max - n + 5;
+    r.sign = v < 0 ? 0x80000000u : 0u;
+    return soft::pack(r);
+}
+// e_max a component may have (0: all corners are zero); others take FP64
+__device__ __forceinline__ bool fixed_range(int e_max) { return e_max == 0 || (uint32_t)(e_max - 200) <= 1600u; }
+
+// A coordinate s about the cell's centre, in cell widths, as the fraction
+// (1/2 + s) 2^64; only for |s| <= 1/2.
+__device__ __forceinline__ bool in_cell(double s) {
+    return (soft::bits_of(s) & 0x7fffffffffffffffull) <= 0x3fe0000000000000ull;
+}
+__device__ __forceinline__ uint64_t fraction(double s) {
+    const soft::Num n = soft::unpack(s);
+    const int sh = 1022 - n.e;
+    const uint64_t t = n.e == 0 || sh > 63 ? 0 : (n.m << 11) >> sh;
+    constexpr uint64_t kHalf = 1ull << 63;
+    if (n.sign) return kHalf - t;
+    return t == kHalf ? ~0ull : kHalf + t;  // 1/2 + 1/2: one unit below 1
+}
 
 // The corner node k = x | y << 1 | z << 2 of a cell: its E, B.
 __device__ __forceinline__ const double* corner_field(const Geom& g, int cx, int cy, int cz, int k) {
     return g.field + 9 * field_index(g, cx + 1 + (k & 1), cy + 1 + ((k >> 1) & 1), cz + 1 + (k >> 2));
+}
+
+// A node value with the gather's normalisation (none: no FP64 instruction).
+__device__ __forceinline__ double field_value(const Push64Const& pc, double v) {
+    return soft::bits_of(pc.field_scale) == 0x3ff0000000000000ull ? v : v * pc.field_scale;
+}
+
+// E, B at (x, y, z) about the centre of a cell, by one thread in FP64: the
+// positions outside the cell (a particle that crossed more than a cell) and
+// the values out of the fixed-point range.
+__device__ __noinline__ void gather_fp64(const Geom& g, int cx, int cy, int cz, double scale, double x, double y,
+                                         double z, double* F) {
+    for (int q = 0; q < 6; ++q) {
+        double f = 0.0;
+        for (int k = 0; k < 8; ++k) {
+            const double w = ((k & 1) ? 0.5 + x : 0.5 - x) * ((k & 2) ? 0.5 + y : 0.5 - y) *
+                             ((k & 4) ? 0.5 + z : 0.5 - z);
+            f = __fma_rn(corner_field(g, cx, cy, cz, k)[q], w, f);
+        }
+        F[q] = f * scale;
+    }
 }
 
 // ---- mover ----------------------------------------------------------------------
@@ -130,7 +189,14 @@ __device__ __forceinline__ void move_field64(const Geom& g, const Push64Const& p
                                              PState<double>& p) {
     if (g.flags & 4u /*IPIC3D_F_DIPOLE_IN_GATHER*/) {
         const double r2 = __fma_rn(p.x, p.x, __fma_rn(p.y, p.y, __dmul_rn(p.z, p.z)));
-        const double f = __dmul_rn(g.mft, inverse_pow25(r2));
+        // mft / r2^2.5 on the integer pipe
+        double f;
+        if (pc.d.usable && soft::regular(r2, 200)) {
+            bool sure;  // either neighbour will do where it is not
+            f = soft::pack(soft::div(pc.d.mft, soft::divisor(soft::pow25(soft::unpack(r2), sure))));
+        } else {
+            f = __dmul_rn(g.mft, inverse_pow25(r2));
+        }
         const double z3 = __dmul_rn(3.0, p.z), zf = __dmul_rn(z3, f);
         F[3] = __fma_rn(p.x, zf, F[3]);
         F[4] = __fma_rn(p.y, zf, F[4]);
@@ -332,23 +398,38 @@ __device__ __forceinline__ int step_one64(const Geom& g, const Push64Const& pc, 
         const double x = (p.x - c.cen[0]) * g.inv_w[0], y = (p.y - c.cen[1]) * g.inv_w[1],
                      z = (p.z - c.cen[2]) * g.inv_w[2];
         double F[6];
+        bool fixed = in_cell(x) && in_cell(y) && in_cell(z);
+        int e_max[6];
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
-            double v[8];
+            int e = 0;
+            bool zero = true;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = __ldg(corner_field(g, c.x, c.y, c.z, k) + q);
+            for (int k = 0; k < 8; ++k) {
+                const double v = field_value(pc, __ldg(corner_field(g, c.x, c.y, c.z, k) + q));
+                e = max(e, soft::exponent_of(v));
+                zero = zero && (soft::bits_of(v) << 1) == 0;
+            }
+            e_max[q] = e;
+            fixed = fixed && fixed_range(e) && (e != 0 || zero);
+        }
+        if (fixed) {
+            const uint64_t rx = fraction(x), ry = fraction(y), rz = fraction(z);
 #pragma unroll
-            for (int bit = 1; bit < 8; bit <<= 1)
+            for (int q = 0; q < 6; ++q) {
+                int64_t v[8];
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    if (!(k & bit)) {
-                        const double lo = v[k], hi = v[k | bit];
-                        v[k] = hi + lo;
-                        v[k | bit] = hi - lo;
-                    }
+                    v[k] = to_fixed(field_value(pc, __ldg(corner_field(g, c.x, c.y, c.z, k) + q)), e_max[q]);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = v[k] * (mean_scale(k) * pc.field_scale);
-            F[q] = poly64(v, x, y, z);
+                for (int bit = 1; bit < 8; bit <<= 1)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k)
+                        if (k & bit) v[k] -= v[k ^ bit];
+                F[q] = from_fixed(poly_fixed(v, rx, ry, rz), e_max[q]);
+            }
+        } else {
+            gather_fp64(g, c.x, c.y, c.z, pc.field_scale, x, y, z, F);
         }
         move_field64(g, pc, qom, F, p);
     } else {
@@ -365,7 +446,7 @@ constexpr int kMaxSpan64 = 4;
 // per group.
 struct Push64Smem {
     int64_t* start;  // [cells + 1]
-    double* coef;    // [groups][kCoefStride64]
+    int64_t* coef;   // [groups][kCoefStride64]
     int* count;      // [cells]
     int* first;      // [cells + 1] items before the cell's
 };
@@ -379,7 +460,7 @@ __device__ __forceinline__ Push64Smem push64_smem(int span, int warps) {
     const int cells = span * kMaxCellsPerCta;
     Push64Smem sm;
     sm.start = reinterpret_cast<int64_t*>(push64_raw);
-    sm.coef = reinterpret_cast<double*>(sm.start + (cells + 2) / 2 * 2);  // 16-byte aligned
+    sm.coef = sm.start + (cells + 2) / 2 * 2;  // 16-byte aligned
     sm.count = reinterpret_cast<int*>(sm.coef + warps * kWarpItems64 * kCoefStride64);
     sm.first = sm.count + cells;
     return sm;
@@ -488,7 +569,7 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
     }
     __syncthreads();
     const int total = sm.first[nc];
-    double* const coef = sm.coef + (warp * kWarpItems64 + sub) * kCoefStride64;
+    int64_t* const coef = sm.coef + (warp * kWarpItems64 + sub) * kCoefStride64;
     const float reach = planet_reach(g);
     uint32_t nmig = 0, nrem = 0;
 
@@ -524,21 +605,31 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
             }
             planet_flags(g, gap, reach, c);
         }
-        if (kStep && kField) {  // lane k: corner k, then coefficient k
+        // lane k: corner k, then coefficient k; the components' exponents in
+        // pairs (every lane of the group has them)
+        uint32_t exps[3] = {0u, 0u, 0u};
+        bool fixed = true;
+        if (kStep && kField) {
             const double* f = corner_field(g, c.x, c.y, c.z, gl);
-            const double scale = mean_scale(gl) * pc.field_scale;
             __syncwarp();
 #pragma unroll
             for (int q = 0; q < 6; ++q) {
-                double v = __ldg(f + q);
+                const double v = field_value(pc, __ldg(f + q));
+                int e = soft::exponent_of(v);
+                bool zero = (soft::bits_of(v) << 1) == 0;
+#pragma unroll
+                for (int bit = 1; bit < 8; bit <<= 1) e = max(e, __shfl_xor_sync(kAll, e, bit));
+                fixed = fixed && fixed_range(e) && (e != 0 || zero);
+                int64_t n = to_fixed(v, e);
 #pragma unroll
                 for (int bit = 1; bit < 8; bit <<= 1) {
-                    const double o = __shfl_xor_sync(kAll, v, bit);
-                    // hi + lo at the lower lane, hi - lo at the upper
-                    v = v + soft::from_bits(soft::bits_of(o) ^ ((gl & bit) ? 0x8000000000000000ull : 0ull));
+                    const int64_t o = __shfl_xor_sync(kAll, n, bit);
+                    if (gl & bit) n -= o;
                 }
-                coef[q * 8 + gl] = v * scale;
+                coef[q * 8 + gl] = n;
+                exps[q >> 1] |= (uint32_t)e << (16 * (q & 1));
             }
+            fixed = (__ballot_sync(kAll, fixed) >> (sub * kGroup64) & 0xffu) == 0xffu;
             __syncwarp();
         }
         double acc[kDep ? 32 : 1];
@@ -562,8 +653,18 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
                     const double x = (p.x - c.cen[0]) * g.inv_w[0], y = (p.y - c.cen[1]) * g.inv_w[1],
                                  z = (p.z - c.cen[2]) * g.inv_w[2];
                     double F[6];
+                    if (fixed && in_cell(x) && in_cell(y) && in_cell(z)) {
+                        const uint64_t rx = fraction(x), ry = fraction(y), rz = fraction(z);
 #pragma unroll
-                    for (int q = 0; q < 6; ++q) F[q] = poly64(coef + 8 * q, x, y, z);
+                        for (int q = 0; q < 6; ++q)
+                            F[q] = from_fixed(poly_fixed(coef + 8 * q, rx, ry, rz),
+                                              (int)(exps[q >> 1] >> (16 * (q & 1)) & 0xffffu));
+                    } else {
+                        double T[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+                        if (has) gather_fp64(g, c.x, c.y, c.z, pc.field_scale, x, y, z, T);
+#pragma unroll
+                        for (int q = 0; q < 6; ++q) F[q] = T[q];
+                    }
                     move_field64(g, pc, P.qom, F, p);
                 } else if (has) {
                     move_dipole64(g, pc, P.qom, p);
