@@ -43,9 +43,14 @@ struct Num {
     uint32_t sign;
 };
 
+// A double's bits. The move hides them from the compiler, which turns masks
+// and zero tests of bits that it knows to be a double's back into FP64
+// instructions (absolute value: an addition; x == 0: a comparison).
 IPG_HD uint64_t bits_of(double x) {
 #ifdef __CUDA_ARCH__
-    return (uint64_t)__double_as_longlong(x);
+    uint64_t b;
+    asm("mov.b64 %0, %1;" : "=l"(b) : "d"(x));
+    return b;
 #else
     uint64_t b;
     std::memcpy(&b, &x, 8);

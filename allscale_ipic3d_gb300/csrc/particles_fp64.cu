@@ -11,31 +11,36 @@ namespace ipg {
 
 namespace {
 // How a launch over `slots` slots in `tiles` tiles is cut: particles per work
-// item, tiles per block, blocks per span, warps per block.
-//   * About 4 warps per sub-partition (152 SMs x 4) keep the FP64 pipe busy.
-//     An item costs its group about 70 FP64 instructions with the deposit,
-//     beside 150 per 8 particles, so items are as long as that allows;
-//     without the deposit an item costs next to nothing, and 32 particles
-//     leave a short tail.
-//   * Where there are blocks enough, spans of 4 tiles and 4 warps per block:
-//     fewer table scans and part-filled warps. Otherwise one warp per block:
-//     160 blocks of 4 warps put two blocks on 8 of the 152 SMs, and the FP64
-//     pipe of those decides (E x B 8^3: a step of 57 us, single warps with
-//     items of 16 particles 56, of 8 particles 43; .inp 16^3: push 0.207 ms
-//     with 4 warps and items of 64, 0.160 with single warps and 32).
+// item, tiles per span, one-warp blocks per span.
+//   * Items are as long as leaves about six warps per sub-partition (152 SMs
+//     x 4): an item costs a quarter of a round or more, shorter ones leave
+//     a shorter tail and end more evenly. Gather + dipole + deposit, 256
+//     particles a cell, ms per push with items of 256 / 64 / 32 / 16: 32^3
+//     cells 1.25 / 1.45 / 1.55 / 1.67, 20^3 0.45 / 0.38 / 0.39 / 0.42, 14^3
+//     0.40 / 0.162 / 0.145 / 0.150, 10^3 0.39 / 0.127 / 0.074 / 0.063; 24^3 of
+//     32 a cell and species 0.283 / 0.199 / 0.227 / 0.215. Items of 128 cut
+//     every other cell of 128 in two, and such items leave half a warp idle
+//     (32^3 1.50, 20^3 0.43): not used. Without the deposit an item costs
+//     next to nothing: 32 (32^3, dipole mover: 64 1.56, 32 1.31).
+//   * Spans of 4 tiles leave fewer part-filled warps than single tiles
+//     (32^3 1.25 against 1.47, 14^3 0.145 against 0.148, 306k particles 0.081
+//     against 0.083); small universes keep a tile per span, whose table is
+//     sooner scanned (E x B 8^3: 0.021 against 0.029).
+//   * One warp a block: its registers are free as soon as it ends (blocks of
+//     4 warps: 32^3 1.39).
+//   * A block takes one round of items, where there is no deposit and the
+//     launch is large four (32^3, dipole mover: 1.31 -> 1.22).
 struct Shape64 {
-    int item, span, parts, warps;
+    int item, span, parts;
 };
 Shape64 shape64(int64_t slots, int64_t tiles, bool deposit) {
-    constexpr int64_t kSms = 152, kGroups = kSms * 4 * 4 * kWarpItems64;
-    Shape64 s{deposit ? 256 : 32, 1, 1, 1};
+    constexpr int64_t kSms = 152, kGroups = 6 * kSms * 4 * kWarpItems64;
+    Shape64 s{32, 1, 1};
+    if (deposit) s.item = slots >= kMaxItem64 * kGroups ? kMaxItem64 : 64;
     while (s.item > kGroup64 && slots < s.item * kGroups) s.item /= 2;
-    if (tiles >= kMaxSpan64 * kSms * 6) {
-        s.span = kMaxSpan64;
-        s.warps = kMaxWarps64;
-    } else {
-        s.parts = (int)std::max<int64_t>(1, kSlotsPerCta / (s.item * kWarpItems64 * s.warps));
-    }
+    if (tiles >= 2 * kSms) s.span = kMaxSpan64;
+    s.parts = s.span * kSlotsPerCta / (s.item * kWarpItems64);
+    if (!deposit && tiles >= 6 * kMaxSpan64 * kSms) s.parts /= 4;
     return s;
 }
 
@@ -67,7 +72,7 @@ int launch_push<double>(const Geom& g, const PopSet<double>& S, int mode, const 
     const Shape64 sh = shape64(slots, tiles, g.deposit != 0);
     const dim3 grid((unsigned)((most + sh.span - 1) / sh.span), sh.parts, S.n);
     const Push64Set pcs = push64_set(g, S);
-    auto run = [&](auto k) { k<<<grid, 32 * sh.warps, push64_smem_bytes(sh.span, sh.warps), st>>>(g, S, pcs, sh.span, sh.item); };
+    auto run = [&](auto k) { k<<<grid, 32, push64_smem_bytes(sh.span), st>>>(g, S, pcs, sh.span, sh.item); };
     if (mode != 0) run(k_push64<false, false, true>);
     else if (g.mover == 1 && g.deposit) run(k_push64<true, true, true>);
     else if (g.mover == 1) run(k_push64<true, true, false>);
@@ -94,7 +99,7 @@ int launch_push_batch<double>(const PopJob<double>* jobs, const int2* cta_job, i
     if (nctas <= 0 || (mode != 0 && !g.deposit)) return 0;
     const Shape64 sh = shape64(nctas * kSlotsPerCta, nctas, g.deposit != 0);
     const dim3 grid((unsigned)nctas, sh.parts);
-    auto run = [&](auto k) { k<<<grid, 32 * sh.warps, push64_smem_bytes(sh.span, sh.warps), st>>>(jobs, cta_job, sh.span, sh.item); };
+    auto run = [&](auto k) { k<<<grid, 32, push64_smem_bytes(sh.span), st>>>(jobs, cta_job, sh.span, sh.item); };
     if (mode != 0) run(k_push64_batch<false, false, true>);
     else if (g.mover == 1 && g.deposit) run(k_push64_batch<true, true, true>);
     else if (g.mover == 1) run(k_push64_batch<true, true, false>);

@@ -3,38 +3,43 @@
 //
 // GB300's FP64 pipe bounds it (one warp instruction per 64 to 76 cycles and
 // SM sub-partition), so what counts is the number of FP64 instructions a
-// warp issues -- idle lanes cost as much as busy ones -- and how many warps
-// share the work of a small universe. Per 32 particles of a step with field
-// gather, dipole and deposit:
-//   * the field is the cell's trilinear polynomial about its centre, built
-//     once per work item from the 8 corners: 42 fused multiply-adds (the sum
-//     over corners: about 130 multiplications and additions);
-//   * the dipole's |r|^-5, the rotation's 2 / (1 + |t|^2) and the deposit's
-//     weights are fused forms without divisions (the export test keeps the
+// warp issues -- idle lanes cost as much as busy ones -- then how many warps
+// there are to fill the gaps, and the size of the loop (five warps a
+// sub-partition, each elsewhere in it, share the instruction cache). Per 32
+// particles of a step with field gather, dipole and deposit:
+//   * the field is the cell's trilinear polynomial, built once per work item
+//     from the 8 corners, and the deposit the moments of the work item's
+//     particles: both in 64-bit fixed point on the integer pipe (poly_fixed,
+//     Moments64);
+//   * the dipole's |r|^-5 on the integer pipe (fp64_int.cuh), the rotation's
+//     2 / (1 + |t|^2) without a division (the export test keeps the
 //     reference's own differences from the cell centre);
 //   * comparisons run on the doubles' bit patterns in the integer pipe;
-//   * the deposit sums the centred monomial moments as the FP32 push does
-//     (push32_pipe.cuh): 35 operations, and 40 per work item for the
-//     reduction over its lanes and the corner sums.
-// 183 FP64 instructions (items' shares and idle lanes included) in place of
-// 541 before. The dipole mover without the gather rounds exactly as the
-// reference does (dipole64.cuh). Measured push per step, before and after:
-// 8.4M particles, gather + dipole + deposit 9.18 -> 2.89 ms (FP64 pipe 86 %
-// busy); 306k particles, two species, gather + deposit 0.593 -> 0.151 ms;
-// 33k particles 0.140 -> 0.028 ms (a warp's serial chain); 1.05M particles,
-// dipole mover, a sixth of them leaving their cells 0.489 -> 0.160 ms (FP64
-// pipe 58 %, integer 42 %). Loading a round's particles a round ahead
-// changed nothing.
+//   * rare parts (walls, planet, sub-cycles, positions outside the cell) are
+//     calls: predicated off they would still take the FP64 pipe.
+// 62 FP64 instructions (items' shares and idle lanes included) and 2,600
+// others in place of 541 FP64 ones before. The dipole mover without the
+// gather rounds exactly as the reference does (dipole64.cuh). Measured push
+// per step, before and after: 8.4M particles, gather + dipole + deposit
+// 9.18 -> 1.30 ms (FP64 pipe 67 % busy, issue slots 47 %); 306k particles,
+// two species, gather + deposit 0.593 -> 0.081 ms; 33k particles 0.140 ->
+// 0.021 ms (a warp's serial chain); 1.05M particles, dipole mover, a sixth of
+// them leaving their cells 0.489 -> 0.150 ms (FP64 pipe 58 %, integer 42 %).
+// Loading a round's particles a round ahead changed nothing.
 //
 // Work. A work item is up to `item` particles of one cell, pushed by a group
 // of 8 lanes, 8 particles at a time (slots are 8-aligned: full 64-byte
 // segments); four items share a warp. Groups of 8 rather than whole warps
 // keep the lanes busy where cells hold few particles or end unevenly, at the
 // price of a reduction per 8 lanes; a cell of more than `item` particles is
-// cut evenly, so that the items of a warp end together. A block of 1 to 4
-// warps takes the items of `span` consecutive 1024-slot tiles, or of a part
-// of them (gridDim.y parts): cells of up to a tile belong to the span they
-// start in, larger ones are cut at its boundaries.
+// cut evenly, so that the items of a warp end together. The push and the
+// moments are two passes over an item: their registers are not live together,
+// and the second knows the components' exponents (one pass: 168 registers,
+// 12 warps per SM; two: 128 and 16, 2.02 -> 1.87 ms, the particles' second
+// read from L1 and L2). A block is one warp, which takes the items of `span`
+// consecutive 1024-slot tiles, or every gridDim.y-th four of them: cells of
+// up to a tile belong to the span they start in, larger ones are cut at its
+// boundaries.
 #pragma once
 
 #include "dipole64.cuh"
@@ -42,7 +47,6 @@
 namespace ipg {
 
 constexpr int kGroup64 = 8;
-constexpr int kMaxWarps64 = 4;
 constexpr int kWarpItems64 = 32 / kGroup64;  // work items of a warp at a time
 constexpr int kCoefStride64 = 50;  // 48 + 2: the four groups of a warp read different banks
 
@@ -118,19 +122,41 @@ __device__ __forceinline__ double from_fixed(int64_t v, int e_max) {
     r.sign = v < 0 ? 0x80000000u : 0u;
     return soft::pack(r);
 }
+// q times the same, rounded once
+__device__ __forceinline__ double times_fixed(double q, int64_t v, int e_max) {
+    const soft::Num c = soft::unpack(q);
+    const uint64_t a = v < 0 ? (uint64_t)-v : (uint64_t)v;
+    int n = __clzll((long long)a);
+    uint64_t p = __umul64hi(a << (n & 63), c.m << 11);
+    if ((int64_t)p >= 0) {
+        p <<= 1;
+        ++n;
+    }
+    soft::Num r;
+    r.m = (p >> 11) + ((p >> 10) & 1);
+    r.e = e_max + c.e - 1017 - n;
+    r.sign = (v < 0 ? 0x80000000u : 0u) ^ c.sign;
+    if (v == 0 || c.e == 0 || c.e == 2047 || r.e < 1 || r.e > 2045) return q * from_fixed(v, e_max);
+    return soft::pack(r);
+}
 // e_max a component may have (0: all corners are zero); others take FP64
 __device__ __forceinline__ bool fixed_range(int e_max) { return e_max == 0 || (uint32_t)(e_max - 200) <= 1600u; }
 
-// A coordinate s about the cell's centre, in cell widths, as the fraction
-// (1/2 + s) 2^64; only for |s| <= 1/2.
-__device__ __forceinline__ bool in_cell(double s) {
-    return (soft::bits_of(s) & 0x7fffffffffffffffull) <= 0x3fe0000000000000ull;
+// A coordinate about the cell's centre as the fraction (1/2 + rel / w) 2^64
+// of the cell, inv = 1 / w; only where |rel| <= w / 2 (in_cell).
+__device__ __forceinline__ uint64_t magnitude_bits(double x) { return soft::bits_of(x) & 0x7fffffffffffffffull; }
+__device__ __forceinline__ bool in_cell(const Geom& g, const double (&rel)[3]) {
+    return magnitude_bits(rel[0]) <= soft::bits_of(g.half_w[0]) &&
+           magnitude_bits(rel[1]) <= soft::bits_of(g.half_w[1]) &&
+           magnitude_bits(rel[2]) <= soft::bits_of(g.half_w[2]);
 }
-__device__ __forceinline__ uint64_t fraction(double s) {
-    const soft::Num n = soft::unpack(s);
-    const int sh = 1022 - n.e;
-    const uint64_t t = n.e == 0 || sh > 63 ? 0 : (n.m << 11) >> sh;
+__device__ __forceinline__ uint64_t fraction(double rel, double inv) {
+    const soft::Num n = soft::unpack(rel), w = soft::unpack(inv);
+    const uint64_t p = __umul64hi(n.m << 11, w.m << 11);
+    const int sh = 2044 - n.e - w.e;  // |rel| / w 2^64 = p 2^-sh, sh >= -1
     constexpr uint64_t kHalf = 1ull << 63;
+    uint64_t t = n.e == 0 || sh > 63 ? 0 : sh >= 0 ? p >> sh : p << 1;
+    t = min(t, kHalf);  // (the rounding of 1 / w)
     if (n.sign) return kHalf - t;
     return t == kHalf ? ~0ull : kHalf + t;  // 1/2 + 1/2: one unit below 1
 }
@@ -145,43 +171,61 @@ __device__ __forceinline__ double field_value(const Push64Const& pc, double v) {
     return soft::bits_of(pc.field_scale) == 0x3ff0000000000000ull ? v : v * pc.field_scale;
 }
 
-// E, B at (x, y, z) about the centre of a cell, by one thread in FP64: the
-// positions outside the cell (a particle that crossed more than a cell) and
-// the values out of the fixed-point range.
-__device__ __noinline__ void gather_fp64(const Geom& g, int cx, int cy, int cz, double scale, double x, double y,
-                                         double z, double* F) {
-    for (int q = 0; q < 6; ++q) {
-        double f = 0.0;
-        for (int k = 0; k < 8; ++k) {
-            const double w = ((k & 1) ? 0.5 + x : 0.5 - x) * ((k & 2) ? 0.5 + y : 0.5 - y) *
-                             ((k & 4) ? 0.5 + z : 0.5 - z);
-            f = __fma_rn(corner_field(g, cx, cy, cz, k)[q], w, f);
-        }
-        F[q] = f * scale;
+// Component q of E, B at (rx, ry, rz) from the centre of a cell, by one
+// thread in FP64: the positions outside the cell (a particle that crossed
+// more than a cell) and the values out of the fixed-point range.
+__device__ __noinline__ double gather_fp64(const Geom& g, int cx, int cy, int cz, double scale, double rx, double ry,
+                                           double rz, int q) {
+    const double x = rx * g.inv_w[0], y = ry * g.inv_w[1], z = rz * g.inv_w[2];
+    double f = 0.0;
+    for (int k = 0; k < 8; ++k) {
+        const double w = ((k & 1) ? 0.5 + x : 0.5 - x) * ((k & 2) ? 0.5 + y : 0.5 - y) *
+                         ((k & 4) ? 0.5 + z : 0.5 - z);
+        f = __fma_rn(corner_field(g, cx, cy, cz, k)[q], w, f);
     }
+    return f * scale;
 }
 
 // ---- mover ----------------------------------------------------------------------
 
 // Boris rotations and positions (particle.h:24-49), fused: ns sub-cycles of
-// dts, k = q/m dts / 2.
+// dts, k = q/m dts / 2. The rotation v- + (v- + v- x t) x s, s = t f, is
+// taken as v- + f (w + w x t), w = v- x t: three roundings of the velocity's
+// size per sub-cycle and no s.
 __device__ __forceinline__ void boris64(const double (&F)[6], double k, double dts, int ns, PState<double>& p) {
     const double tx = __dmul_rn(k, F[3]), ty = __dmul_rn(k, F[4]), tz = __dmul_rn(k, F[5]);
     const double den = __fma_rn(tx, tx, __fma_rn(ty, ty, __fma_rn(tz, tz, 1.0)));
     const double y = reciprocal(den), f = __dadd_rn(y, y);
-    const double sx = __dmul_rn(tx, f), sy = __dmul_rn(ty, f), sz = __dmul_rn(tz, f);
+#pragma unroll 1
     for (int s = 0; s < ns; ++s) {
         const double mx = __fma_rn(k, F[0], p.u), my = __fma_rn(k, F[1], p.v), mz = __fma_rn(k, F[2], p.w);
-        const double px = __fma_rn(my, tz, __fma_rn(-mz, ty, mx));
-        const double py = __fma_rn(mz, tx, __fma_rn(-mx, tz, my));
-        const double pz = __fma_rn(mx, ty, __fma_rn(-my, tx, mz));
-        p.u = __fma_rn(k, F[0], __fma_rn(py, sz, __fma_rn(-pz, sy, mx)));
-        p.v = __fma_rn(k, F[1], __fma_rn(pz, sx, __fma_rn(-px, sz, my)));
-        p.w = __fma_rn(k, F[2], __fma_rn(px, sy, __fma_rn(-py, sx, mz)));
+        const double wx = __fma_rn(my, tz, -__dmul_rn(mz, ty));
+        const double wy = __fma_rn(mz, tx, -__dmul_rn(mx, tz));
+        const double wz = __fma_rn(mx, ty, -__dmul_rn(my, tx));
+        const double qx = __fma_rn(wy, tz, __fma_rn(-wz, ty, wx));
+        const double qy = __fma_rn(wz, tx, __fma_rn(-wx, tz, wy));
+        const double qz = __fma_rn(wx, ty, __fma_rn(-wy, tx, wz));
+        p.u = __fma_rn(k, F[0], __fma_rn(f, qx, mx));
+        p.v = __fma_rn(k, F[1], __fma_rn(f, qy, my));
+        p.w = __fma_rn(k, F[2], __fma_rn(f, qz, mz));
         p.x = __fma_rn(p.u, dts, p.x);
         p.y = __fma_rn(p.v, dts, p.y);
         p.z = __fma_rn(p.w, dts, p.z);
     }
+}
+
+struct SubCycles64 {
+    double dts, k;
+    int n;
+};
+// (a call: its divisions would sit in every particle's instruction stream)
+__device__ __noinline__ SubCycles64 sub_cycles64(double dt, double c, double inv_pic, double qom, double bx, double by,
+                                                 double bz) {
+    SubCycles64 s;
+    const double bmag = (bx * bx + by * by) + bz * bz;
+    s.n = sub_cycles_dt(dt, c, inv_pic, qom, bmag, s.dts);
+    s.k = qom * 0.5 * s.dts;
+    return s;
 }
 
 // The field mover's step from the gathered E, B in F.
@@ -204,14 +248,9 @@ __device__ __forceinline__ void move_field64(const Geom& g, const Push64Const& p
     }
     // one sub-cycle is sure below an exponent; else the reference's rule
     const int e = max(max(soft::exponent_of(F[3]), soft::exponent_of(F[4])), soft::exponent_of(F[5]));
-    if (e <= pc.d.e_max) {
-        boris64(F, pc.k1, g.dt, 1, p);
-    } else {
-        double dts;
-        const double bmag = (F[3] * F[3] + F[4] * F[4]) + F[5] * F[5];
-        const int ns = sub_cycles_dt(g.dt, g.c, g.inv_pic, qom, bmag, dts);
-        boris64(F, qom * 0.5 * dts, dts, ns, p);
-    }
+    SubCycles64 s = {g.dt, pc.k1, 1};
+    if (e > pc.d.e_max) s = sub_cycles64(g.dt, g.c, g.inv_pic, qom, F[3], F[4], F[5]);
+    boris64(F, s.k, s.dts, s.n, p);
 }
 
 // The dipole mover's step (cell.h:939-960), rounded as the reference's.
@@ -256,6 +295,11 @@ struct Cell64 {
 __device__ __forceinline__ double cell_centre(const Geom& g, int a, int pos) {
     return (g.origin[a] + (double)pos * g.w[a]) + g.half_w[a];
 }
+// The same rounded once, for the weights of gather and deposit (the three
+// roundings above show in both on widths that are no powers of two).
+__device__ __forceinline__ double cell_middle(const Geom& g, int a, int pos) {
+    return __fma_rn((double)pos + 0.5, g.w[a], g.origin[a]);
+}
 // Distance along axis a from the planet's centre to the cell's box, in FP32;
 // the comparison with planet_reach adds the margin.
 __device__ __forceinline__ float planet_gap(const Geom& g, int a, double cen) {
@@ -281,7 +325,6 @@ __device__ __forceinline__ void planet_flags(const Geom& g, const float (&gap)[3
     c.edge = c.x == 0 || c.y == 0 || c.z == 0 || c.x == g.sx - 1 || c.y == g.sy - 1 || c.z == g.sz - 1;
 }
 
-__device__ __forceinline__ uint64_t magnitude_bits(double x) { return soft::bits_of(x) & 0x7fffffffffffffffull; }
 // |x| > lim (lim >= 0); false for NaN, as the FP64 comparison
 __device__ __forceinline__ bool beyond(double x, double lim) {
     const uint64_t b = magnitude_bits(x);
@@ -322,9 +365,7 @@ __device__ __forceinline__ int export64(const Geom& g, const Cell64& c, PState<d
     rel[0] = p.x - c.cen[0];
     rel[1] = p.y - c.cen[1];
     rel[2] = p.z - c.cen[2];
-    if (!c.near_planet && magnitude_bits(rel[0]) <= soft::bits_of(g.half_w[0]) &&
-        magnitude_bits(rel[1]) <= soft::bits_of(g.half_w[1]) && magnitude_bits(rel[2]) <= soft::bits_of(g.half_w[2]))
-        return kStay;
+    if (!c.near_planet && in_cell(g, rel)) return kStay;
     const int pos[3] = {c.x, c.y, c.z}, size[3] = {g.sx, g.sy, g.sz};
     double P[3] = {p.x, p.y, p.z};
     if (c.edge) {
@@ -395,10 +436,10 @@ __device__ __forceinline__ int step_one64(const Geom& g, const Push64Const& pc, 
     }
     planet_flags(g, gap, planet_reach(g), c);
     if (g.mover == 1) {
-        const double x = (p.x - c.cen[0]) * g.inv_w[0], y = (p.y - c.cen[1]) * g.inv_w[1],
-                     z = (p.z - c.cen[2]) * g.inv_w[2];
+        const double at[3] = {p.x - cell_middle(g, 0, c.x), p.y - cell_middle(g, 1, c.y),
+                              p.z - cell_middle(g, 2, c.z)};
         double F[6];
-        bool fixed = in_cell(x) && in_cell(y) && in_cell(z);
+        bool fixed = in_cell(g, at);
         int e_max[6];
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
@@ -414,7 +455,8 @@ __device__ __forceinline__ int step_one64(const Geom& g, const Push64Const& pc, 
             fixed = fixed && fixed_range(e) && (e != 0 || zero);
         }
         if (fixed) {
-            const uint64_t rx = fraction(x), ry = fraction(y), rz = fraction(z);
+            const uint64_t rx = fraction(at[0], g.inv_w[0]), ry = fraction(at[1], g.inv_w[1]),
+                           rz = fraction(at[2], g.inv_w[2]);
 #pragma unroll
             for (int q = 0; q < 6; ++q) {
                 int64_t v[8];
@@ -429,7 +471,9 @@ __device__ __forceinline__ int step_one64(const Geom& g, const Push64Const& pc, 
                 F[q] = from_fixed(poly_fixed(v, rx, ry, rz), e_max[q]);
             }
         } else {
-            gather_fp64(g, c.x, c.y, c.z, pc.field_scale, x, y, z, F);
+#pragma unroll
+            for (int q = 0; q < 6; ++q)
+                F[q] = gather_fp64(g, c.x, c.y, c.z, pc.field_scale, at[0], at[1], at[2], q);
         }
         move_field64(g, pc, qom, F, p);
     } else {
@@ -441,6 +485,9 @@ __device__ __forceinline__ int step_one64(const Geom& g, const Push64Const& pc, 
 
 // ---- the bulk push ---------------------------------------------------------------
 constexpr int kMaxSpan64 = 4;
+constexpr int kMaxItem64 = 32 * kGroup64;  // a lane's rounds fit a word
+// warps per SM: 128 registers with the deposit (96 spill), 96 without
+constexpr int kDepWarps64 = 16, kMoveWarps64 = 20;
 
 // A block's dynamic shared memory: the cells of its span, their coefficients
 // per group.
@@ -450,18 +497,18 @@ struct Push64Smem {
     int* count;      // [cells]
     int* first;      // [cells + 1] items before the cell's
 };
-__host__ __device__ constexpr size_t push64_smem_bytes(int span, int warps) {
+__host__ __device__ constexpr size_t push64_smem_bytes(int span) {
     const int cells = span * kMaxCellsPerCta;
-    return (size_t)(cells + 2) / 2 * 2 * sizeof(int64_t) + (size_t)warps * kWarpItems64 * kCoefStride64 * sizeof(double) +
+    return (size_t)(cells + 2) / 2 * 2 * sizeof(int64_t) + (size_t)kWarpItems64 * kCoefStride64 * sizeof(double) +
            (size_t)(2 * cells + 1) * sizeof(int);
 }
-__device__ __forceinline__ Push64Smem push64_smem(int span, int warps) {
+__device__ __forceinline__ Push64Smem push64_smem(int span) {
     extern __shared__ __align__(16) unsigned char push64_raw[];
     const int cells = span * kMaxCellsPerCta;
     Push64Smem sm;
     sm.start = reinterpret_cast<int64_t*>(push64_raw);
     sm.coef = sm.start + (cells + 2) / 2 * 2;  // 16-byte aligned
-    sm.count = reinterpret_cast<int*>(sm.coef + warps * kWarpItems64 * kCoefStride64);
+    sm.count = reinterpret_cast<int*>(sm.coef + kWarpItems64 * kCoefStride64);
     sm.first = sm.count + cells;
     return sm;
 }
@@ -530,23 +577,175 @@ __device__ __forceinline__ void leave64(const Geom& g, const Pop<double>& P, int
     if (deposit && lb) warp_deposit_leavers<double>(g, leave, dest, p, P.q);
 }
 
+// The cloud-in-cell moments of a lane's particles in 64-bit fixed point: the
+// sums of Q m for Q in {u, v, w, 1} and m in {1, x, y, xy, z, xz, yz, xyz}
+// of the position in the cell, a 64-bit fraction. The values of a component
+// share the exponent `top` of the largest in the group of 8 lanes; with
+// `room` = log2 of the rounds, they keep 63 - room bits below it, offset by
+// 2^(63 - room) so that the products are unsigned and add without overflow:
+// the sum of the offsets is known from the sums of m and taken off at the end.
+//
+// Precision. A unit is 2^-(63 - room) of the power of two above the largest
+// value, 2^-58 for items of 256 particles; each term is off by less than 2
+// units, and nothing rounds until the node's FP64 addition, where each FP64
+// addition here rounded the partial sum by up to 2^-53 of it. (A spread of
+// magnitudes costs what it costs in FP64: what lies below the last place of
+// the largest is lost.) J's error against 113-bit sums, before and after: 33k
+// particles 1.8e-16 -> 1.4e-16 of its size, 4.8M of 600 a cell 2.7e-16 ->
+// 1.6e-16.
+//
+// Cost. 25 high products of 64 x 64 bits and 32 sums per particle, about 600
+// cycles of a warp on the integer pipe; in FP64 35 instructions, 2400
+// cycles of the FP64 pipe, and 40 per work item for the reduction (8.4M
+// particles: the deposit alone 0.70 -> 0.35 ms, the push 2.10 -> 1.82).
+struct Moments64 {
+    uint64_t a[32];  // Q, moment: 8 Q + m; a[24] unused (the particle count)
+
+    __device__ __forceinline__ static int headroom(int item) {
+        const int rounds = (item + kGroup64 - 1) / kGroup64;
+        return rounds > 1 ? 32 - __clz(rounds - 1) : 0;
+    }
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int l = 0; l < 32; ++l) a[l] = 0;
+    }
+    // the lane's particle, if `in`
+    __device__ __forceinline__ void add(const Geom& g, int room, bool in, const double (&rel)[3],
+                                        const double (&v)[3], const int (&top)[3]) {
+        uint64_t M[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (in) {
+            M[1] = fraction(rel[0], g.inv_w[0]);
+            M[2] = fraction(rel[1], g.inv_w[1]);
+            M[4] = fraction(rel[2], g.inv_w[2]);
+        }
+        M[3] = __umul64hi(M[1], M[2]);
+        M[5] = __umul64hi(M[1], M[4]);
+        M[6] = __umul64hi(M[2], M[4]);
+        M[7] = __umul64hi(M[3], M[4]);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const soft::Num x = soft::unpack(v[q]);
+            const int sh = room + 1 + top[q] - x.e;
+            const uint64_t f = x.e == 0 || sh > 63 ? 0 : (x.m << 11) >> sh;
+            const uint64_t Q = in ? (1ull << (63 - room)) + (x.sign ? 0 - f : f) : 0;
+            a[8 * q] += Q;
+#pragma unroll
+            for (int m = 1; m < 8; ++m) a[8 * q + m] += __umul64hi(Q, M[m]);
+        }
+#pragma unroll
+        for (int m = 1; m < 8; ++m) a[24 + m] += M[m] >> (room + 1);
+    }
+    // The moments turned into the corners' sums of weights (1 - r, r). n: the
+    // lane's particles.
+    __device__ __forceinline__ void corners(int room, int n) {
+        a[24] = (uint64_t)n << (63 - room);
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            // Products and shifts round down, by half a unit on average: what
+            // is left of that (a bias grows with n) is made up for. x, y, z
+            // shift without a remainder: a coordinate is a multiple of 2^-58
+            // cell widths unless within 1/64 of one from zero.
+            const bool exact = m == 1 || m == 2 || m == 4;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) a[8 * q + m] += (exact ? n >> 1 : 0) - a[24 + m];
+            if (m && !exact) a[24 + m] += n >> 1;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int bit = 1; bit < 8; bit <<= 1)
+#pragma unroll
+                for (int m = 0; m < 8; ++m)
+                    if (!(m & bit)) a[8 * q + m] -= a[8 * q + (m | bit)];
+    }
+    // The velocity sums' shift that lets those of 32 lanes add without
+    // overflow: 0 for most (velocities of both signs), up to 6.
+    __device__ __forceinline__ int spare_bits() const {
+        uint32_t mag = 0;
+#pragma unroll
+        for (int l = 0; l < 24; ++l) mag |= (uint32_t)(((uint64_t)((int64_t)a[l] >> 63) ^ a[l]) >> 32);
+        return max(0, 6 - __clz(__reduce_or_sync(0xffffffffu, mag)));
+    }
+    // Over the group's 8 lanes: lane m is left with corner m's sums in a[0],
+    // a[8], a[16] (in units 2^shift as large) and a[24] (2^kRhoShift).
+    __device__ __forceinline__ void reduce(int shift) {
+        constexpr unsigned kAll = 0xffffffffu;
+        const int gl = threadIdx.x & (kGroup64 - 1);
+        const int64_t half = shift ? 1ll << (shift - 1) : 0;
+#pragma unroll
+        for (int l = 0; l < 32; ++l)
+            a[l] = l < 24 ? (uint64_t)(((int64_t)a[l] + half) >> shift)
+                          : (a[l] + (1u << (kRhoShift - 1))) >> kRhoShift;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int off = 4; off >= 1; off >>= 1) {
+                const bool up = (gl & off) != 0;
+#pragma unroll
+                for (int m = 0; m < off; ++m) {
+                    const uint64_t send = up ? a[8 * q + m] : a[8 * q + m + off];
+                    const uint64_t keep = up ? a[8 * q + m + off] : a[8 * q + m];
+                    a[8 * q + m] = keep + __shfl_xor_sync(kAll, send, off);
+                }
+            }
+    }
+    // The groups of one cell: the first is left with their sums (the others
+    // with parts of them). Returns the sum of n likewise.
+    __device__ __forceinline__ int join(int n, bool next, bool after) {
+        constexpr unsigned kAll = 0xffffffffu;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            uint64_t o = __shfl_down_sync(kAll, a[8 * q], kGroup64);
+            if (next) a[8 * q] += o;
+            o = __shfl_down_sync(kAll, a[8 * q], 2 * kGroup64);
+            if (after) a[8 * q] += o;
+        }
+        int o = __shfl_down_sync(kAll, n, kGroup64);
+        if (next) n += o;
+        o = __shfl_down_sync(kAll, n, 2 * kGroup64);
+        if (after) n += o;
+        return n;
+    }
+    static constexpr int kRhoShift = 6;  // 32 lanes of at most 2^63
+    // charge times component q's sum at the lane's corner (shift: as given to
+    // reduce; top = 0: every value is zero, what is left the offsets' rounding)
+    __device__ __forceinline__ double velocity(int q, double charge, int top, int room, int shift) const {
+        return top ? times_fixed(charge, (int64_t)a[8 * q], top + room + shift - 4) : 0.0;
+    }
+    __device__ __forceinline__ double density(double charge, int room) const {
+        return times_fixed(charge, (int64_t)a[24], 1018 + room + kRhoShift);
+    }
+};
+// a velocity component the moments take: zero, or of an exponent in fixed_range
+__device__ __forceinline__ bool moment_range(double v) {
+    const int e = soft::exponent_of(v);
+    return fixed_range(e) && (e != 0 || (soft::bits_of(v) << 1) == 0);
+}
+// A particle outside its cell, or whose velocity is out of the fixed-point
+// range (or no number).
+__device__ __noinline__ void deposit_fp64(const Geom& g, int cell, double x, double y, double z, double u, double v,
+                                          double w, double q) {
+    const PState<double> p = {x, y, z, u, v, w};
+    deposit_one<double>(g, cell, p, q);
+}
+
 // kStep: mover + export (else the deposit of the particles as they are);
 // kField: field-gather mover (else the dipole mover); kDep: deposit.
 template <bool kStep, bool kField, bool kDep>
 __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P, const Push64Const& pc, int64_t tile,
                                             int span, int part, int parts, int item) {
     constexpr unsigned kAll = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int lane = threadIdx.x;
     const int gl = lane & (kGroup64 - 1), sub = lane / kGroup64;
-    const Push64Smem sm = push64_smem(span, warps);
+    const Push64Smem sm = push64_smem(span);
     // the cells of the span: consecutive tiles' cells follow one another
     const int64_t base = tile * kSlotsPerCta, top = min(base + (int64_t)span * kSlotsPerCta, P.capacity);
     const int2 cc = __ldg(P.cta_cells + tile), ce = __ldg(P.cta_cells + (top - 1) / kSlotsPerCta);
     const int c0 = cc.x, nc = ce.x + ce.y - cc.x;
-    for (int i = threadIdx.x; i <= nc; i += blockDim.x) sm.start[i] = P.start[c0 + i];
-    for (int i = threadIdx.x; i < nc; i += blockDim.x) sm.count[i] = P.count[c0 + i];
-    __syncthreads();
-    if (warp == 0) {  // items before each cell
+    for (int i = lane; i <= nc; i += 32) sm.start[i] = P.start[c0 + i];
+    for (int i = lane; i < nc; i += 32) sm.count[i] = P.count[c0 + i];
+    __syncwarp();
+    {  // items before each cell
         int before = 0;
         for (int b = 0; b < nc; b += 32) {
             const int i = b + lane;
@@ -567,13 +766,14 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
         }
         if (lane == 0) sm.first[nc] = before;
     }
-    __syncthreads();
+    __syncwarp();
     const int total = sm.first[nc];
-    int64_t* const coef = sm.coef + (warp * kWarpItems64 + sub) * kCoefStride64;
+    int64_t* const coef = sm.coef + sub * kCoefStride64;
     const float reach = planet_reach(g);
+    const int headroom = Moments64::headroom(item);
     uint32_t nmig = 0, nrem = 0;
 
-    for (int j0 = (part * warps + warp) * kWarpItems64; j0 < total; j0 += parts * warps * kWarpItems64) {
+    for (int j0 = part * kWarpItems64; j0 < total; j0 += parts * kWarpItems64) {
         const int j = min(j0 + sub, total - 1);
         int i = 0;
         {
@@ -594,13 +794,17 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
         const int64_t cstart = sm.start[i];
         Cell64 c;
         cell_coords(g, cell, c.x, c.y, c.z);
+        double mid[3];
         {   // lane 0, 1, 2 of the group: the axis' centre
-            const double cen = gl < 3 ? cell_centre(g, gl, gl == 0 ? c.x : gl == 1 ? c.y : c.z) : 0.0;
+            const int pos = gl == 0 ? c.x : gl == 1 ? c.y : c.z;
+            const double cen = gl < 3 ? cell_centre(g, gl, pos) : 0.0;
+            const double middle = gl < 3 ? cell_middle(g, gl, pos) : 0.0;
             const float mine = gl < 3 ? planet_gap(g, gl, cen) : 0.f;
             float gap[3];
 #pragma unroll
             for (int b = 0; b < 3; ++b) {
                 c.cen[b] = __shfl_sync(kAll, cen, b, kGroup64);
+                mid[b] = __shfl_sync(kAll, middle, b, kGroup64);
                 gap[b] = __shfl_sync(kAll, mine, b, kGroup64);
             }
             planet_flags(g, gap, reach, c);
@@ -632,38 +836,41 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
             fixed = (__ballot_sync(kAll, fixed) >> (sub * kGroup64) & 0xffu) == 0xffu;
             __syncwarp();
         }
-        double acc[kDep ? 32 : 1];
-        if (kDep) {
-#pragma unroll
-            for (int l = 0; l < 32; ++l) acc[l] = 0.0;
-        }
-        int stay = 0;
+        uint32_t adds = 0;            // bit r: the lane's particle of round r adds to the moments
+        int top[3] = {0, 0, 0};       // the components' largest exponents among them
         const int rounds = __reduce_max_sync(kAll, (len + kGroup64 - 1) / kGroup64);
         for (int r = 0; r < rounds; ++r) {
             const int k = r * kGroup64 + gl;
             const bool has = k < len;
             const int64_t slot = a + k;
-            // lanes without a particle: the cell's centre at rest, which adds
-            // nothing to the moments but the count, taken apart
+            // lanes without a particle: the cell's centre at rest
             PState<double> p = {c.cen[0], c.cen[1], c.cen[2], 0.0, 0.0, 0.0};
             if (has) p = {P.x[slot], P.y[slot], P.z[slot], P.u[slot], P.v[slot], P.w[slot]};
             double rel[3];
+            bool stays;
             if (kStep) {
                 if (kField) {
-                    const double x = (p.x - c.cen[0]) * g.inv_w[0], y = (p.y - c.cen[1]) * g.inv_w[1],
-                                 z = (p.z - c.cen[2]) * g.inv_w[2];
+                    const double at[3] = {p.x - mid[0], p.y - mid[1], p.z - mid[2]};
                     double F[6];
-                    if (fixed && in_cell(x) && in_cell(y) && in_cell(z)) {
-                        const uint64_t rx = fraction(x), ry = fraction(y), rz = fraction(z);
+                    if (fixed && in_cell(g, at)) {
+                        const uint64_t rx = fraction(at[0], g.inv_w[0]), ry = fraction(at[1], g.inv_w[1]),
+                                       rz = fraction(at[2], g.inv_w[2]);
+                        // a loop, the results passing through F: unrolled, the
+                        // gather alone was a third of the instruction stream
+                        // (push 1.60 -> 1.43 ms)
+#pragma unroll 1
+                        for (int q = 0; q < 6; ++q) {
+                            const uint32_t e = q < 2 ? exps[0] : q < 4 ? exps[1] : exps[2];
+                            const double f = from_fixed(poly_fixed(coef + 8 * q, rx, ry, rz),
+                                                        (int)(e >> (16 * (q & 1)) & 0xffffu));
+#pragma unroll
+                            for (int k = 0; k < 5; ++k) F[k] = F[k + 1];
+                            F[5] = f;
+                        }
+                    } else {
 #pragma unroll
                         for (int q = 0; q < 6; ++q)
-                            F[q] = from_fixed(poly_fixed(coef + 8 * q, rx, ry, rz),
-                                              (int)(exps[q >> 1] >> (16 * (q & 1)) & 0xffffu));
-                    } else {
-                        double T[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-                        if (has) gather_fp64(g, c.x, c.y, c.z, pc.field_scale, x, y, z, T);
-#pragma unroll
-                        for (int q = 0; q < 6; ++q) F[q] = T[q];
+                            F[q] = has ? gather_fp64(g, c.x, c.y, c.z, pc.field_scale, at[0], at[1], at[2], q) : 0.0;
                     }
                     move_field64(g, pc, P.qom, F, p);
                 } else if (has) {
@@ -677,64 +884,72 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
                 }
                 if (__any_sync(kAll, outcome > kStay))
                     leave64(g, P, outcome, cell, cstart, slot, dest, p, kDep, nmig, nrem);
-                if (kDep) {
-                    stay += outcome == kStay;
-                    if (outcome != kStay) {
-                        rel[0] = rel[1] = rel[2] = 0.0;
-                        p.u = p.v = p.w = 0.0;
-                    }
-                }
+                stays = outcome == kStay;
             } else {
                 rel[0] = p.x - c.cen[0];
                 rel[1] = p.y - c.cen[1];
                 rel[2] = p.z - c.cen[2];
-                stay += has;
+                stays = has;
             }
-            if (kDep) {
-                const double x = rel[0] * g.inv_w[0], y = rel[1] * g.inv_w[1], z = rel[2] * g.inv_w[2];
-                const double xy = x * y, xz = x * z, yz = y * z;
-                const double M[8] = {1.0, x, y, xy, z, xz, yz, xy * z};
-                const double Q[3] = {p.u, p.v, p.w};
+            if (kDep && stays) {
+                const int e[3] = {soft::exponent_of(p.u), soft::exponent_of(p.v), soft::exponent_of(p.w)};
+                if (in_cell(g, rel) && moment_range(p.u) && moment_range(p.v) && moment_range(p.w)) {
+                    adds |= 1u << r;
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    acc[8 * q] = acc[8 * q] + Q[q];
-#pragma unroll
-                    for (int m = 1; m < 8; ++m) acc[8 * q + m] = __fma_rn(Q[q], M[m], acc[8 * q + m]);
+                    for (int q = 0; q < 3; ++q) top[q] = max(top[q], e[q]);
+                } else {
+                    deposit_fp64(g, cell, p.x, p.y, p.z, p.u, p.v, p.w, P.q);
                 }
-#pragma unroll
-                for (int m = 1; m < 8; ++m) acc[24 + m] = acc[24 + m] + M[m];
             }
         }
-        if (kDep) {
-            // over the group's lanes: lane m is left with moment m of each Q
+        if (kDep && __any_sync(kAll, adds != 0)) {
+            Moments64 sums;
+            sums.clear();
+            // groups with items of the same cell (they follow one another) add up
+            // before the FP64 atomics, which round: next: the following
+            // group's cell is this one's, after: the one after it too
+            const int c1 = __shfl_down_sync(kAll, cell, kGroup64), c2 = __shfl_down_sync(kAll, cell, 2 * kGroup64);
+            const int before = __shfl_up_sync(kAll, cell, kGroup64);
+            const bool next = sub < kWarpItems64 - 1 && c1 == cell, after = sub < kWarpItems64 - 2 && c2 == cell;
+            const bool first = sub == 0 || before != cell;
+            const bool shared = __any_sync(kAll, next);
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
+            for (int q = 0; q < 3; ++q) top[q] = __reduce_max_sync(0xffu << (sub * kGroup64), top[q]);
+            if (shared) {
+                int t[3] = {top[0], top[1], top[2]};
 #pragma unroll
-                for (int off = 4; off >= 1; off >>= 1) {
-                    const bool up = (gl & off) != 0;
+                for (int k = 1; k < kWarpItems64; ++k) {
+                    const bool same = __shfl_xor_sync(kAll, cell, k * kGroup64) == cell;
 #pragma unroll
-                    for (int m = 0; m < off; ++m) {
-                        const double send = up ? acc[8 * q + m] : acc[8 * q + m + off];
-                        const double keep = up ? acc[8 * q + m + off] : acc[8 * q + m];
-                        acc[8 * q + m] = keep + __shfl_xor_sync(kAll, send, off);
+                    for (int q = 0; q < 3; ++q) {
+                        const int o = __shfl_xor_sync(kAll, t[q], k * kGroup64);
+                        if (same) top[q] = max(top[q], o);
                     }
                 }
-            stay = __reduce_add_sync(0xffu << (sub * kGroup64), stay);
-            if (gl == 0) acc[24] = (double)stay;
-            // moments -> corner sums (weights 1/2 -+ s), one axis at a time
-#pragma unroll
-            for (int bit = 1; bit < 8; bit <<= 1)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const double o = __shfl_xor_sync(kAll, acc[8 * q], bit);
-                    acc[8 * q] = (gl & bit) ? __fma_rn(0.5, o, acc[8 * q]) : __fma_rn(0.5, acc[8 * q], -o);
+            }
+            for (int r = 0; r < rounds; ++r) {
+                const int64_t slot = a + r * kGroup64 + gl;
+                const bool in = (adds >> r & 1u) != 0;
+                double rel[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
+                if (in) {
+                    rel[0] = P.x[slot] - mid[0];
+                    rel[1] = P.y[slot] - mid[1];
+                    rel[2] = P.z[slot] - mid[2];
+                    v[0] = P.u[slot]; v[1] = P.v[slot]; v[2] = P.w[slot];
                 }
-            if (stay > 0) {
-                const int64_t n =
-                    node_index(g, c.x + (gl & 1), c.y + ((gl >> 1) & 1), c.z + (gl >> 2));
+                sums.add(g, headroom, in, rel, v, top);
+            }
+            int n = __reduce_add_sync(0xffu << (sub * kGroup64), __popc(adds));
+            sums.corners(headroom, __popc(adds));
+            const int shift = sums.spare_bits();
+            sums.reduce(shift);
+            if (shared) n = sums.join(n, next, after);
+            if (first && n > 0) {
+                const int64_t node = node_index(g, c.x + (gl & 1), c.y + ((gl >> 1) & 1), c.z + (gl >> 2));
 #pragma unroll
-                for (int q = 0; q < 3; ++q) atomicAdd(g.J + 3 * n + q, P.q * acc[8 * q]);
-                atomicAdd(g.rho + n, P.q * acc[24]);
+                for (int q = 0; q < 3; ++q)
+                    atomicAdd(g.J + 3 * node + q, sums.velocity(q, P.q, top[q], headroom, shift));
+                atomicAdd(g.rho + node, sums.density(P.q, headroom));
             }
         }
     }
@@ -750,7 +965,7 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
 
 // Block (span, part) of population blockIdx.z of the set.
 template <bool kStep, bool kField, bool kDep>
-__global__ void __launch_bounds__(32 * kMaxWarps64, kDep ? 3 : 5)
+__global__ void __launch_bounds__(32, kDep ? kDepWarps64 : kMoveWarps64)
     k_push64(Geom g, const __grid_constant__ PopSet<double> S, const __grid_constant__ Push64Set pcs, int span,
              int item) {
     const Pop<double>& P = S.p[blockIdx.z];
@@ -762,7 +977,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps64, kDep ? 3 : 5)
 // Batched: cta_job[blockIdx.x] = (job, tile of the job); the span starts at
 // every span-th tile of a job.
 template <bool kStep, bool kField, bool kDep>
-__global__ void __launch_bounds__(32 * kMaxWarps64, kDep ? 3 : 5)
+__global__ void __launch_bounds__(32, kDep ? kDepWarps64 : kMoveWarps64)
     k_push64_batch(const PopJob<double>* __restrict__ jobs, const int2* __restrict__ cta_job, int span, int item) {
     __shared__ PopJob<double> job;
     const int2 cj = __ldg(cta_job + blockIdx.x);
