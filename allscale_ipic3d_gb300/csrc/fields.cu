@@ -15,6 +15,7 @@
 // The reference's per-node solver updates E and then Bc in one in-place pass
 // whose result depends on the visiting order; here E is updated everywhere
 // first and Bc afterwards (the order-independent two-phase reading).
+#include <algorithm>
 #include <cmath>
 
 #include "launch.h"
@@ -363,7 +364,11 @@ __global__ void k_interp_c2n(SolverArgs A) {
 template <bool kMul>
 __global__ void k_j_finalize(int sx, int sy, int sz, double* J, double* rho, double vol, double inv, int div8) {
     const int r = row_item();
-    if (r < 4 * sz) j_finalize_point<kMul>(sx, sy, sz, J, rho, vol, inv, div8, blockIdx.z, blockIdx.y, r);
+    if (r >= 4 * sz) return;
+    // grids need not be cubes: more rows than a launch has are taken in turns
+    for (int x = blockIdx.z; x < sx; x += gridDim.z)
+        for (int y = blockIdx.y; y < sy; y += gridDim.y)
+            j_finalize_point<kMul>(sx, sy, sz, J, rho, vol, inv, div8, x, y, r);
 }
 template <bool kMul>
 __global__ void k_forward_e(SolverArgs A) { forward_e_body<kMul>(A, grid_t0(), grid_stride()); }
@@ -559,7 +564,8 @@ int launch_ghost(const Geom& g, cudaStream_t st) {
     return 1;
 }
 
-// The launch of a row kernel: nx x ny rows of `items`.
+// The launch of a row kernel: nx x ny rows of `items`, up to 65535 each way
+// (the solvers' grids are cubes, which stay far below).
 struct Rows {
     dim3 grid;
     unsigned threads;
@@ -567,7 +573,7 @@ struct Rows {
 static Rows rows(int nx, int ny, int items) {
     Rows r;
     r.threads = (unsigned)(items < 256 ? (items + 31) / 32 * 32 : 256);
-    r.grid = dim3((items + r.threads - 1) / r.threads, ny, nx);
+    r.grid = dim3((items + r.threads - 1) / r.threads, std::min(ny, 65535), std::min(nx, 65535));
     return r;
 }
 
