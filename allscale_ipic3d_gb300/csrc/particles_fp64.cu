@@ -98,8 +98,8 @@ int launch_push_batch<double>(const PopJob<double>* jobs, const int2* cta_job, i
                               const Geom& g, const PushShape&, cudaStream_t st) {
     if (nctas <= 0 || (mode != 0 && !g.deposit)) return 0;
     const Shape64 sh = shape64(nctas * kSlotsPerCta, nctas, g.deposit != 0);
-    const dim3 grid((unsigned)nctas, sh.parts);
-    auto run = [&](auto k) { k<<<grid, 32, push64_smem_bytes(sh.span), st>>>(jobs, cta_job, sh.span, sh.item); };
+    const unsigned grid = (unsigned)(nctas * sh.parts);
+    auto run = [&](auto k) { k<<<grid, 32, push64_smem_bytes(sh.span), st>>>(jobs, cta_job, sh.span, sh.item, sh.parts); };
     if (mode != 0) run(k_push64_batch<false, false, true>);
     else if (g.mover == 1 && g.deposit) run(k_push64_batch<true, true, true>);
     else if (g.mover == 1) run(k_push64_batch<true, true, false>);

@@ -974,16 +974,21 @@ __global__ void __launch_bounds__(32, kDep ? kDepWarps64 : kMoveWarps64)
     push64_body<kStep, kField, kDep>(g, P, pcs.c[blockIdx.z], tile, span, blockIdx.y, gridDim.y, item);
 }
 
-// Batched: cta_job[blockIdx.x] = (job, tile of the job); the span starts at
-// every span-th tile of a job.
+// Batched: block b is part b % parts of cta_job[b / parts] = (job, tile of the
+// job); the span starts at every span-th tile of a job, the other tiles'
+// blocks end at once. The parts of a tile are consecutive blocks: with the
+// tiles along x, every fourth block had work, and the SMs, which hand
+// one-warp blocks to their four sub-partitions in turn, ran it all on one
+// (64 universes of 34M particles: 15.3 ms a step, now 7.0).
 template <bool kStep, bool kField, bool kDep>
 __global__ void __launch_bounds__(32, kDep ? kDepWarps64 : kMoveWarps64)
-    k_push64_batch(const PopJob<double>* __restrict__ jobs, const int2* __restrict__ cta_job, int span, int item) {
+    k_push64_batch(const PopJob<double>* __restrict__ jobs, const int2* __restrict__ cta_job, int span, int item, int parts) {
     __shared__ PopJob<double> job;
-    const int2 cj = __ldg(cta_job + blockIdx.x);
+    const unsigned tile = blockIdx.x / (unsigned)parts;
+    const int2 cj = __ldg(cta_job + tile);
     if (cj.y % span != 0) return;
     load_job(job, jobs + cj.x);
-    push64_body<kStep, kField, kDep>(job.g, job.P, job.pc, cj.y, span, blockIdx.y, gridDim.y, item);
+    push64_body<kStep, kField, kDep>(job.g, job.P, job.pc, cj.y, span, (int)(blockIdx.x - tile * parts), parts, item);
 }
 
 // ---- particles that waited for a slot ---------------------------------------------
