@@ -155,10 +155,10 @@ def measured_peak():
 
 # DRAM bytes (read + write) per push launch on the headline workload, from
 # one ncu capture of each kernel (k_push32_pipe with the push shape 256, 32,
-# 2; k_push<double>); a citation of that capture, not a measurement of this
-# run. FP32: one launch for both species; FP64: one launch per species.
+# 2; k_push64); a citation of that capture, not a measurement of this run.
+# One launch for both species.
 PUSH_TRAFFIC = {"fp32": (436869120, "ncu capture of k_push32_pipe<3, 2, 15> on this workload (cited, not of this run)"),
-                "fp64": (369767168, "ncu capture of k_push<double> on this workload (cited, not of this run)")}
+                "fp64": (821560000, "ncu capture of k_push64<1, 1, 1> on this workload (cited, not of this run)")}
 
 
 def combine_ranks(ms, psteps, dist, device):
@@ -229,9 +229,8 @@ class _Null:
 def push_roofline(sim, precision, nsteps, props, pops, headline=True):
     """Live CUDA-event times of the push phase over `nsteps` eager steps; the
     push kernel's algorithmic bytes per launch over its average launch
-    duration. The FP32 push is one launch per step for all `pops` species
-    populations; the FP64 push one launch per population (`pops` launches of
-    equal size). Algorithmic bytes per population: the particles' state read
+    duration: one launch per step for all `pops` species populations.
+    Algorithmic bytes per population: the particles' state read
     and written once (12 x 4 B FP32, 12 x 8 B FP64), the per-cell field
     coefficients read once (FP32: 48 floats per cell) or the node E, B read
     once (FP64: 48 B per node), and the 4 FP64 node moments written once
@@ -242,16 +241,15 @@ def push_roofline(sim, precision, nsteps, props, pops, headline=True):
     prof = sim.profile_read(reset=True)
     sim.profile(False)
     push = prof["push"]
-    per_launch_pops = pops if precision == "fp32" else 1
-    launches_per_step = 1 if precision == "fp32" else pops
-    ms_per = push["ms"] / max(push["launches"], 1) / launches_per_step
-    parts = push["particles"] / max(push["launches"], 1) / launches_per_step
+    launches_per_step = 1
+    ms_per = push["ms"] / max(push["launches"], 1)
+    parts = push["particles"] / max(push["launches"], 1)
     elem = 4 if precision == "fp32" else 8
     nodes = (props.size[0] + 1) * (props.size[1] + 1) * (props.size[2] + 1)
     if precision == "fp32":
-        bytes_per = parts * 12 * elem + per_launch_pops * (props.ncells * 48 * 4 + nodes * 32)
+        bytes_per = parts * 12 * elem + pops * (props.ncells * 48 * 4 + nodes * 32)
     else:
-        bytes_per = parts * 12 * elem + nodes * (48 + 32)
+        bytes_per = parts * 12 * elem + pops * nodes * (48 + 32)
     peak, src = measured_peak()
     achieved = bytes_per / (ms_per * 1e-3) / 1e9
     phases = {k: round(v["ms"] / max(v["launches"], 1), 5) for k, v in prof.items() if v["launches"]}
@@ -259,7 +257,7 @@ def push_roofline(sim, precision, nsteps, props, pops, headline=True):
             "traffic": PUSH_TRAFFIC[precision][0] if headline else None,
             "traffic_source": PUSH_TRAFFIC[precision][1] if headline else None,
             "kernel": ("ipg::k_push32_pipe<3, 2, 15>" if headline else "ipg::k_push32_pipe") if elem == 4
-            else "ipg::k_push<double>",
+            else "ipg::k_push64",
             "bytes_per_launch": bytes_per, "ms_per_launch": ms_per, "launches_per_step": launches_per_step,
             "peak_source": src + ", burst copy", "phase_ms_per_step": phases}
 
