@@ -676,6 +676,13 @@ struct Moments64 {
         for (int l = 0; l < 24; ++l) mag |= (uint32_t)(((uint64_t)((int64_t)a[l] >> 63) ^ a[l]) >> 32);
         return max(0, 6 - __clz(__reduce_or_sync(0xffffffffu, mag)));
     }
+    // A lane's sum of weights at a corner, up to 2^63 (all particles in the
+    // corner): where every particle is within 2^-49 of the opposite face, the
+    // sums' roundings can leave it below zero, by up to 1.5 units a particle,
+    // which as an unsigned number would be 2^64 less that: zero then.
+    __device__ __forceinline__ static uint64_t density_sum(uint64_t v) {
+        return (uint32_t)(v >> 32) >= 0xc0000000u ? 0 : v;
+    }
     // Over the group's 8 lanes: lane m is left with corner m's sums in a[0],
     // a[8], a[16] (in units 2^shift as large) and a[24] (2^kRhoShift).
     __device__ __forceinline__ void reduce(int shift) {
@@ -685,7 +692,7 @@ struct Moments64 {
 #pragma unroll
         for (int l = 0; l < 32; ++l)
             a[l] = l < 24 ? (uint64_t)(((int64_t)a[l] + half) >> shift)
-                          : (a[l] + (1u << (kRhoShift - 1))) >> kRhoShift;
+                          : (density_sum(a[l]) + (1u << (kRhoShift - 1))) >> kRhoShift;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
