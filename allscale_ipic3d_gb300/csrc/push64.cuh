@@ -596,13 +596,23 @@ __device__ __forceinline__ void leave64(const Geom& g, const Pop<double>& P, int
 // the sum of the offsets is known from the sums of m and taken off at the end.
 //
 // Precision. A unit is 2^-(63 - room) of the power of two above the largest
-// value, 2^-58 for items of 256 particles; each term is off by less than 2
-// units, and nothing rounds until the node's FP64 addition, where each FP64
-// addition here rounded the partial sum by up to 2^-53 of it. (A spread of
-// magnitudes costs what it costs in FP64: what lies below the last place of
-// the largest is lost.) J's error against 113-bit sums, before and after: 33k
-// particles 1.8e-16 -> 1.4e-16 of its size, 4.8M of 600 a cell 2.7e-16 ->
-// 1.6e-16.
+// value (of one charge, for the density), room going by the particles of the
+// cell that a lane adds up, not by the launch's items: 2^-63 for up to 8
+// particles of a cell, 2^-58 for 256. Before the lanes' sums are added they
+// are cut by the bits that the sum of all takes (sum_shift: 1 for a single
+// particle, 6 for a warp of 1024), and nothing else rounds until the node's
+// FP64 addition. RMS error over the cell's largest corner, FP64 sums before
+// and this, 1 / 8 / 64 particles a cell, long items: J 3.3e-17 / 6.1e-17 /
+// 8.3e-17 -> 2.0e-17 / 2.4e-17 / 2.7e-17, rho 2.7e-17 / 5.0e-17 / 6.4e-17 ->
+// 2.0e-17 / 2.9e-17 / 4.0e-17 (with the unit and the cut of the longest items
+// for all: rho 1.5e-16 / 1.1e-16 / 4.5e-17). Whole universes, error over the
+// size of J: 33k particles 1.9e-16 -> 1.5e-16, 4.8M of 600 a cell 2.7e-16 ->
+// 1.6e-16; of rho: 0.90e-16 -> 0.95e-16 and 1.62e-16 -> 0.95e-16 (short items
+// add to a node more often).
+// What is fine is the sum's size, not every node's share of it: a slow
+// particle beside a fast one of its cell, and a node that little of the cell
+// reaches, keep less than 53 bits. One particle at (0.01, 0.02, 0.03) of its
+// cell: 4e-14 of the far node's share, where FP64 products have 3e-16.
 //
 // Cost. 25 high products of 64 x 64 bits and 32 sums per particle, about 600
 // cycles of a warp on the integer pipe; in FP64 35 instructions, 2400
@@ -611,10 +621,12 @@ __device__ __forceinline__ void leave64(const Geom& g, const Pop<double>& P, int
 struct Moments64 {
     uint64_t a[32];  // Q, moment: 8 Q + m; a[24] unused (the particle count)
 
-    __device__ __forceinline__ static int headroom(int item) {
-        const int rounds = (item + kGroup64 - 1) / kGroup64;
-        return rounds > 1 ? 32 - __clz(rounds - 1) : 0;
-    }
+    __device__ __forceinline__ static int log2_up(int n) { return n > 1 ? 32 - __clz(n - 1) : 0; }
+    // log2 of a lane's rounds, for items of `len` particles
+    __device__ __forceinline__ static int headroom(int len) { return log2_up((len + kGroup64 - 1) / kGroup64); }
+    // The shift that lets the sums of `n` particles in all, in units of
+    // `room`, add up to 2^62 at most.
+    __device__ __forceinline__ static int sum_shift(int n, int room) { return max(0, log2_up(n) + 1 - room); }
     __device__ __forceinline__ void clear() {
 #pragma unroll
         for (int l = 0; l < 32; ++l) a[l] = 0;
@@ -668,8 +680,8 @@ struct Moments64 {
                 for (int m = 0; m < 8; ++m)
                     if (!(m & bit)) a[8 * q + m] -= a[8 * q + (m | bit)];
     }
-    // The velocity sums' shift that lets those of 32 lanes add without
-    // overflow: 0 for most (velocities of both signs), up to 6.
+    // The shift that lets the velocity sums of 32 lanes add without overflow:
+    // 0 for most (velocities of both signs), up to 6.
     __device__ __forceinline__ int spare_bits() const {
         uint32_t mag = 0;
 #pragma unroll
@@ -684,15 +696,14 @@ struct Moments64 {
         return (uint32_t)(v >> 32) >= 0xc0000000u ? 0 : v;
     }
     // Over the group's 8 lanes: lane m is left with corner m's sums in a[0],
-    // a[8], a[16] (in units 2^shift as large) and a[24] (2^kRhoShift).
-    __device__ __forceinline__ void reduce(int shift) {
+    // a[8], a[16] (in units 2^shift as large) and a[24] (2^rho_shift).
+    __device__ __forceinline__ void reduce(int shift, int rho_shift) {
         constexpr unsigned kAll = 0xffffffffu;
         const int gl = threadIdx.x & (kGroup64 - 1);
-        const int64_t half = shift ? 1ll << (shift - 1) : 0;
+        const uint32_t half = (1u << shift) >> 1, rho_half = (1u << rho_shift) >> 1;
 #pragma unroll
         for (int l = 0; l < 32; ++l)
-            a[l] = l < 24 ? (uint64_t)(((int64_t)a[l] + half) >> shift)
-                          : (density_sum(a[l]) + (1u << (kRhoShift - 1))) >> kRhoShift;
+            a[l] = l < 24 ? (uint64_t)((int64_t)(a[l] + half) >> shift) : (density_sum(a[l]) + rho_half) >> rho_shift;
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
@@ -707,8 +718,8 @@ struct Moments64 {
             }
     }
     // The groups of one cell: the first is left with their sums (the others
-    // with parts of them). Returns the sum of n likewise.
-    __device__ __forceinline__ int join(int n, bool next, bool after) {
+    // with parts of them).
+    __device__ __forceinline__ void join(bool next, bool after) {
         constexpr unsigned kAll = 0xffffffffu;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -717,20 +728,14 @@ struct Moments64 {
             o = __shfl_down_sync(kAll, a[8 * q], 2 * kGroup64);
             if (after) a[8 * q] += o;
         }
-        int o = __shfl_down_sync(kAll, n, kGroup64);
-        if (next) n += o;
-        o = __shfl_down_sync(kAll, n, 2 * kGroup64);
-        if (after) n += o;
-        return n;
     }
-    static constexpr int kRhoShift = 6;  // 32 lanes of at most 2^63
     // charge times component q's sum at the lane's corner (shift: as given to
     // reduce; top = 0: every value is zero, what is left the offsets' rounding)
     __device__ __forceinline__ double velocity(int q, double charge, int top, int room, int shift) const {
         return top ? times_fixed(charge, (int64_t)a[8 * q], top + room + shift - 4) : 0.0;
     }
-    __device__ __forceinline__ double density(double charge, int room) const {
-        return times_fixed(charge, (int64_t)a[24], 1018 + room + kRhoShift);
+    __device__ __forceinline__ double density(double charge, int room, int rho_shift) const {
+        return times_fixed(charge, (int64_t)a[24], 1018 + room + rho_shift);
     }
 };
 // a velocity component the moments take: zero, or of an exponent in fixed_range
@@ -756,7 +761,7 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
     const int gl = lane & (kGroup64 - 1), sub = lane / kGroup64;
     const Push64Smem sm = push64_smem(span);
     // the cells of the span: consecutive tiles' cells follow one another
-    const int64_t base = tile * kSlotsPerCta, top = min(base + (int64_t)span * kSlotsPerCta, P.capacity);
+    const int base = (int)tile * kSlotsPerCta, top = (int)min(base + (int64_t)span * kSlotsPerCta, P.capacity);
     const int2 cc = __ldg(P.cta_cells + tile), ce = __ldg(P.cta_cells + (top - 1) / kSlotsPerCta);
     const int c0 = cc.x, nc = ce.x + ce.y - cc.x;
     for (int i = lane; i <= nc; i += 32) sm.start[i] = P.start[c0 + i];
@@ -787,7 +792,6 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
     const int total = sm.first[nc];
     int64_t* const coef = sm.coef + sub * kCoefStride64;
     const float reach = planet_reach(g);
-    const int headroom = Moments64::headroom(item);
     uint32_t nmig = 0, nrem = 0;
 
     for (int j0 = part * kWarpItems64; j0 < total; j0 += parts * kWarpItems64) {
@@ -804,8 +808,8 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
         span_range64(sm, i, base, top, lo, end);
         const int pieces = sm.first[i + 1] - sm.first[i];
         const int piece = ((int)(end - lo) + pieces * kGroup64 - 1) / (pieces * kGroup64) * kGroup64;
-        const int64_t a = lo + (int64_t)(j - sm.first[i]) * piece;
-        int len = max(0, (int)min((int64_t)piece, end - a));
+        const int a = (int)lo + (j - sm.first[i]) * piece;
+        int len = max(0, min(piece, (int)end - a));
         if (j0 + sub >= total) len = 0;
         const int cell = c0 + i;
         const int64_t cstart = sm.start[i];
@@ -859,7 +863,7 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
         for (int r = 0; r < rounds; ++r) {
             const int k = r * kGroup64 + gl;
             const bool has = k < len;
-            const int64_t slot = a + k;
+            const int slot = a + k;
             // lanes without a particle: the cell's centre at rest
             PState<double> p = {c.cen[0], c.cen[1], c.cen[2], 0.0, 0.0, 0.0};
             if (has) p = {P.x[slot], P.y[slot], P.z[slot], P.u[slot], P.v[slot], P.w[slot]};
@@ -944,8 +948,12 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
                     }
                 }
             }
+            // at most so many of the cell's particles in an item, in the warp
+            // (the same in all groups of the cell)
+            const int in_item = min(item, sm.count[cell - c0]), in_warp = min(kWarpItems64 * item, sm.count[cell - c0]);
+            const int room = Moments64::headroom(in_item);
             for (int r = 0; r < rounds; ++r) {
-                const int64_t slot = a + r * kGroup64 + gl;
+                const int slot = a + r * kGroup64 + gl;
                 const bool in = (adds >> r & 1u) != 0;
                 double rel[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
                 if (in) {
@@ -954,19 +962,18 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
                     rel[2] = P.z[slot] - mid[2];
                     v[0] = P.u[slot]; v[1] = P.v[slot]; v[2] = P.w[slot];
                 }
-                sums.add(g, headroom, in, rel, v, top);
+                sums.add(g, room, in, rel, v, top);
             }
-            int n = __reduce_add_sync(0xffu << (sub * kGroup64), __popc(adds));
-            sums.corners(headroom, __popc(adds));
-            const int shift = sums.spare_bits();
-            sums.reduce(shift);
-            if (shared) n = sums.join(n, next, after);
-            if (first && n > 0) {
+            sums.corners(room, __popc(adds));
+            const int rho_shift = Moments64::sum_shift(in_warp, room), shift = min(sums.spare_bits(), rho_shift);
+            sums.reduce(shift, rho_shift);
+            if (shared) sums.join(next, after);
+            if (first) {
                 const int64_t node = node_index(g, c.x + (gl & 1), c.y + ((gl >> 1) & 1), c.z + (gl >> 2));
 #pragma unroll
                 for (int q = 0; q < 3; ++q)
-                    atomicAdd(g.J + 3 * node + q, sums.velocity(q, P.q, top[q], headroom, shift));
-                atomicAdd(g.rho + node, sums.density(P.q, headroom));
+                    atomicAdd(g.J + 3 * node + q, sums.velocity(q, P.q, top[q], room, shift));
+                atomicAdd(g.rho + node, sums.density(P.q, room, rho_shift));
             }
         }
     }

@@ -76,3 +76,51 @@ def test_empty_corners_of_cells_with_all_particles_on_an_edge(long_items):
         for k, w in zip(corners(), exact_weights(c, width, x[0])):
             got = float(rho[tuple(c + k)]) * float(np.prod(width))
             assert abs(Fraction(got) - Fraction(Q) * w * n) <= abs(Q) * n * (n / 8 + 32) * 2.0 ** -53, (n, c, k)
+
+
+# Tolerance of the sums of N particles of a cell, V the largest velocity
+# component among them (1 for the density), on widths that are powers of two
+# and positions whose difference from the cell's middle is exact. With items
+# of I particles a lane adds up to r = ceil(min(N, I) / 8) of them in units of
+# 2^(room - 63) of the power of two above V, room = ceil(log2 r): at most 32
+# units a particle over the eight corners' sums (products, weights and shifts
+# round down, by less than 4 units a moment). The lanes' sums are then shifted
+# by at most 2 + log2(N) - room bits, half a unit each: 2 N 2^-63 for each of
+# min(N, 32) lanes. Last, each of A = ceil(N / I) items rounds its product with
+# the charge and its addition to the node by 2^-53 of a sum below S = sum |Q v
+# w|, and the finalisation by nothing (the volume is a power of two):
+# 2 V N (32 2^room + 2 min(N, 32)) 2^-63 |Q| + 2 A 2^-53 S.
+SPARSE = [1, 2, 3, 4, 7, 8, 9, 16, 40, 255, 256, 600]
+
+
+@pytest.mark.parametrize("kind", ["plain", "far", "faces"])
+@pytest.mark.parametrize("long_items", [False, True])
+def test_sums_keep_their_last_places(long_items, kind):
+    """However long the launch's work items are, the sums of a cell with few
+    particles are as fine as their number allows."""
+    width = np.array([0.5, 1.0, 2.0])
+    size, filler, item = ((17, 17, 17), 800, 256) if long_items else ((8, 8, 8), 0, 8)
+    rng = np.random.default_rng(["plain", "far", "faces"].index(kind))
+    places = []
+    for i, n in enumerate(SPARSE):
+        c = np.array([1 + 2 * (i % 3), 1 + 2 * (i // 3 % 2), 1 + 2 * (i // 6)])
+        r = rng.integers(1, 2 ** 20, (n, 3)) / 2.0 ** 20
+        if kind == "far":
+            r = r / 64.0  # the far node gets 2^-18 or less of a particle
+        elif kind == "faces":
+            r = rng.choice([0.0, 0.25, 1.0, 2.0 ** -20, 1.0 - 2.0 ** -30], (n, 3))
+        places.append((c, (c + r) * width, rng.normal(0.0, 1.5, (n, 3))))
+    J, rho = project(size, width, filler, places)
+    for c, x, v in places:
+        n = len(x)
+        rounds = -(-min(n, item) // 8)
+        fine = 2.0 * n * (32 * 2 ** (rounds - 1).bit_length() + 2 * min(n, 32)) * 2.0 ** -63
+        weights = [exact_weights(c, width, t) for t in x]
+        comps = [[Fraction(float(t)) for t in v[:, a]] for a in range(3)] + [[Fraction(1)] * n]
+        for i, k in enumerate(corners()):
+            got = [float(t) for t in J[tuple(c + k)]] + [float(rho[tuple(c + k)])]
+            for a, q in enumerate(comps):
+                terms = [t * w[i] for t, w in zip(q, weights)]
+                top, total = max(abs(t) for t in q), sum(abs(t) for t in terms)
+                tol = abs(Q) * (Fraction(fine) * top + 2 * -(-n // item) * total / 2 ** 53)
+                assert abs(Fraction(got[a]) - Fraction(Q) * sum(terms)) <= tol, (n, k, a, got[a], float(tol))
