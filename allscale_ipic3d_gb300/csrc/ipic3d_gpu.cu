@@ -1114,6 +1114,11 @@ int ph_collect(ipic3d_ctx* ctx) {
     return IPIC3D_OK;
 }
 
+bool injects(const ipic3d_ctx* ctx) {
+    return (ctx->cfg.flags & IPIC3D_F_INJECT_LOW_X) && ctx->cfg.bc_low[0] == IPIC3D_BC_OPEN &&
+           ctx->cfg.inject_per_cell > 0;
+}
+
 // Clears the step counters and, with `moments`, J and rho (k_step_begin).
 int step_begin(ipic3d_ctx* ctx, bool counters, bool moments, cudaStream_t st) {
     CounterSet s{};
@@ -1218,9 +1223,7 @@ int move_impl(ipic3d_ctx* ctx, bool deposit, bool next_solve = false, bool clear
     for (auto& S : s32) n += launch_push_pending<float>(g, S, aux);
     for (auto& S : s64) n += launch_push_pending<double>(g, S, aux);
     ph_end(ctx, IPIC3D_PHASE_PENDING);
-    const bool inject = (ctx->cfg.flags & IPIC3D_F_INJECT_LOW_X) && ctx->cfg.bc_low[0] == IPIC3D_BC_OPEN &&
-                        ctx->cfg.inject_per_cell > 0;
-    if (inject) {
+    if (injects(ctx)) {
         ph_begin(ctx, IPIC3D_PHASE_INJECT);
         if (ctx->fp32)
             n += launch_inject<float>(g, ctx->p32[0].view(), ctx->cfg.inject_per_cell, ctx->cfg.inject_drift,
@@ -1768,8 +1771,14 @@ int ipic3d_gpu_step(ipic3d_ctx* ctx, uint64_t num_steps) {
     const bool overlap = use_graph && ctx->cfg.solver != IPIC3D_SOLVER_STATIC;
     bool presolved = false;
     // long runs replay kUnroll steps at a time (the last step apart; capturing
-    // the longer graph pays for itself over a few replays)
-    const bool unroll = use_graph && num_steps >= 3 * kUnroll;
+    // the longer graph pays for itself over a few replays). A re-layout then
+    // comes up to two replays after its limit is passed, which no run has been
+    // seen to suffer from (converging flows of 0.3M and 1M particles, 30 to
+    // 200 steps: as fast or faster, with half the re-layouts). Injection is
+    // another matter: the pending list is sized for the particles of the last
+    // layout, and holds the injected ones too only if the universe is laid out
+    // anew within two steps
+    const bool unroll = use_graph && num_steps >= 3 * kUnroll && !injects(ctx);
     uint64_t round = 0;  // replays (or eager steps) so far
     for (uint64_t done = 0; done < num_steps; ++round) {
         uint64_t steps = 1;
