@@ -36,7 +36,7 @@ def load(size, mean, seed):
     return props, p, counts.astype(np.uint64)
 
 
-# slots of about 0.4, 1.2 and 4.4 million: items of 16 or 32, 64, 256
+# 0.35, 0.97 and 3.8 million slots: items of 16, 64 (32 without deposit), 256 (32)
 @pytest.mark.parametrize("size,mean", [((11, 10, 10), 270), ((13, 14, 14), 350), ((20, 19, 21), 440)])
 @pytest.mark.parametrize("mover,project,flags", [
     (abi.MOVER_FIELD, abi.PROJECT_CIC, abi.F_GATHER_DIV_VOL),
