@@ -75,6 +75,28 @@ IPG_HD bool regular(double x, int range) {
     return (uint32_t)(exponent_of(x) - (1023 - range)) <= (uint32_t)(2 * range);
 }
 
+// An integer that orders doubles by their high words as their values do
+// (negative ones below positive ones, NaN outside every finite value).
+IPG_HD int32_t order_key_hi(double x) {
+    const int32_t h = (int32_t)(uint32_t)(bits_of(x) >> 32);
+    return h ^ ((h >> 31) & 0x7fffffff);
+}
+
+// The keys strictly between those of low and high, both finite: doubles of
+// such a key lie within [low, high]. The keys of one box can be more than 2^31
+// apart (any box around +-2): the differences are unsigned.
+struct KeyBox {
+    uint32_t first, count;
+};
+IPG_HD KeyBox key_box(double low, double high) {
+    KeyBox b;
+    const int64_t first = (int64_t)order_key_hi(low) + 1, count = order_key_hi(high) - first;
+    b.first = (uint32_t)first;
+    b.count = count > 0 ? (uint32_t)count : 0u;
+    return b;
+}
+IPG_HD bool in_key_box(double x, const KeyBox& b) { return (uint32_t)order_key_hi(x) - b.first < b.count; }
+
 IPG_HD Num unpack(double x) {
     const uint64_t b = bits_of(x);
     const uint32_t h = (uint32_t)(b >> 32);

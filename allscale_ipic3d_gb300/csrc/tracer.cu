@@ -34,9 +34,8 @@ struct TraceArgs {
     double w[3];             // cell width (getCellCoordinates)
     double center[3];        // objectCenter
     int quick_planet;        // objectCenter == 0 and R^2 finite: the planet test's r^2 is the next step's field r^2
-    int quick_box;           // the box is finite: order_key_hi - key_in < key_span lies strictly inside it
-    int32_t key_in[3];
-    uint32_t key_span[3];
+    int quick_box;           // the box is finite: in_key_box settles most positions
+    soft::KeyBox box[3];
     double r2max;            // planetRadius^2
     double mft;              // -Bext.z * pow(planetRadius, 3), host libm
     double dt, c;
@@ -48,13 +47,6 @@ struct TraceArgs {
     uint64_t n;
     uint32_t* counts;
 };
-
-// An integer that orders doubles by their high words as their values do
-// (negative ones below positive ones, NaN outside every finite value).
-__host__ __device__ __forceinline__ int32_t order_key_hi(double x) {
-    const int32_t h = (int32_t)(soft::bits_of(x) >> 32);
-    return h ^ ((h >> 31) & 0x7fffffff);
-}
 
 __device__ __forceinline__ double sum_sq(double a, double b, double c) {
     double r = a * a;  // allscale::utils::sumOfSquares: 0 + a^2 + b^2 + c^2 (0 + a^2 == a^2)
@@ -124,12 +116,11 @@ __global__ void __launch_bounds__(kTraceThreads) k_trace(const TraceArgs A) {
             }
         }
         // periodic wrap (pic_tracer.cxx:129-133). The high words settle that
-        // a position lies strictly inside the box; only the others compare
-        // and add in FP64 (a call, so that no FP64 instruction is issued,
+        // a position lies inside the box; only the others compare and add in
+        // FP64 (a call, so that no FP64 instruction is issued,
         // predicated off, for every particle: 11 of 56 a step were)
-        const bool inside = A.quick_box && (uint32_t)(order_key_hi(P[0]) - A.key_in[0]) < A.key_span[0] &&
-                            (uint32_t)(order_key_hi(P[1]) - A.key_in[1]) < A.key_span[1] &&
-                            (uint32_t)(order_key_hi(P[2]) - A.key_in[2]) < A.key_span[2];
+        const bool inside = A.quick_box && soft::in_key_box(P[0], A.box[0]) && soft::in_key_box(P[1], A.box[1]) &&
+                            soft::in_key_box(P[2], A.box[2]);
         if (!inside) {
             P[0] = wrapped(P[0], A.low[0], A.high[0], A.extent[0]);
             P[1] = wrapped(P[1], A.low[1], A.high[1], A.extent[1]);
@@ -188,9 +179,7 @@ int trace_args(const ipic3d_props* props, uint64_t n, int32_t steps, int32_t fra
     A.quick_box = 1;
     for (int a = 0; a < 3; ++a) {
         if (!std::isfinite(A.low[a]) || !std::isfinite(A.high[a])) A.quick_box = 0;
-        A.key_in[a] = order_key_hi(A.low[a]) + 1;
-        const int64_t span = (int64_t)order_key_hi(A.high[a]) - A.key_in[a];
-        A.key_span[a] = span > 0 ? (uint32_t)span : 0u;
+        A.box[a] = soft::key_box(A.low[a], A.high[a]);
     }
     A.mft = -props->external_b[2] * std::pow(props->planet_radius, 3);
     A.dt = props->dt;
