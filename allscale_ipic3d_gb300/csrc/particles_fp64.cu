@@ -55,6 +55,8 @@ Push64Const push64_const(const Geom& g, const Pop<double>& P) {
     Push64Const c;
     c.d = dipole_species(g.mft, P.qom, g.dt, g.inv_pic);
     c.k1 = P.qom * 0.5 * g.dt;
+    // rotations too large for the fast form take the sub-cycle branch
+    c.d.e_max = std::min(c.d.e_max, kLargeRotation + 1023 - soft::exponent_of(c.k1));
     c.no_field = g.mft == 0.0 && soft::regular(g.dt, 100) && std::isfinite(c.k1) && std::isfinite(P.qom) &&
                  std::isfinite(4.0 * P.qom * g.dt) && std::isfinite(g.inv_pic);
     c.field_scale = (g.flags & 2u /*IPIC3D_F_GATHER_DIV_VOL*/) ? 1.0 / g.vol : 1.0;

@@ -228,6 +228,20 @@ __device__ __noinline__ SubCycles64 sub_cycles64(double dt, double c, double inv
     return s;
 }
 
+// Exponent of a rotation t = k B above which 1 + |t|^2 or |t|^2 v may overflow
+// in boris64, where the reference's operations stay finite.
+constexpr int kLargeRotation = 1023 + 100;
+__device__ __noinline__ PState<double> boris_large64(double ex, double ey, double ez, double bx, double by, double bz,
+                                                     double qom, double dts, int ns, PState<double> p) {
+    for (int s = 0; s < ns; ++s) {
+        boris<double>(p.u, p.v, p.w, ex, ey, ez, bx, by, bz, qom, dts);
+        p.x = p.x + p.u * dts;
+        p.y = p.y + p.v * dts;
+        p.z = p.z + p.w * dts;
+    }
+    return p;
+}
+
 // The field mover's step from the gathered E, B in F.
 __device__ __forceinline__ void move_field64(const Geom& g, const Push64Const& pc, double qom, double (&F)[6],
                                              PState<double>& p) {
@@ -249,7 +263,13 @@ __device__ __forceinline__ void move_field64(const Geom& g, const Push64Const& p
     // one sub-cycle is sure below an exponent; else the reference's rule
     const int e = max(max(soft::exponent_of(F[3]), soft::exponent_of(F[4])), soft::exponent_of(F[5]));
     SubCycles64 s = {g.dt, pc.k1, 1};
-    if (e > pc.d.e_max) s = sub_cycles64(g.dt, g.c, g.inv_pic, qom, F[3], F[4], F[5]);
+    if (e > pc.d.e_max) {
+        s = sub_cycles64(g.dt, g.c, g.inv_pic, qom, F[3], F[4], F[5]);
+        if (soft::exponent_of(s.k) + e > 1023 + kLargeRotation) {
+            p = boris_large64(F[0], F[1], F[2], F[3], F[4], F[5], qom, s.dts, s.n, p);
+            return;
+        }
+    }
     boris64(F, s.k, s.dts, s.n, p);
 }
 
