@@ -215,7 +215,10 @@ IPG_HD double fused(double a, double b, double c) {
 // the range.
 IPG_HD double quotient(double a, double w, double inv, int exact) {
     if (exact) return a * inv;
-    if (!regular(a, 900) || !regular(w, 100)) return a / w;
+    if (!regular(a, 900) || !regular(w, 100)) {
+        if ((bits_of(a) << 1) == 0 && regular(w, 100)) return a * inv;  // a zero of a's and w's signs
+        return a / w;
+    }
     double q = a * inv;
     q = fused(fused(-w, q, a), inv, q);
     return fused(fused(-w, q, a), inv, q);
