@@ -96,8 +96,8 @@ __device__ __forceinline__ double over(double d, double w, double iw) {
     return kMul ? d * iw : soft::quotient(d, w, iw, 0);
 }
 
-// The leapfrog, the node refresh and the J finalisation run a thread per node
-// and component, components fastest: neighbouring lanes read neighbouring
+// The leapfrog, the node refresh and the J finalisation of smaller grids run a
+// thread per node and component, components fastest: neighbouring lanes read neighbouring
 // doubles, and three times the threads hide the latency of grids that fill
 // the SMs once. A block works on a row (x, y) of the grid, so a thread divides
 // by 3 only (a flat index costs two divisions by the grid size, as much as
@@ -257,6 +257,15 @@ __device__ __forceinline__ void forward_b_body(SolverArgs A, int64_t t0, int64_t
     }
 }
 
+// A node's sum over vol [/ 8], correctly rounded with inv = 1 / vol (kMul
+// false), or its product with inv.
+template <bool kMul>
+__device__ __forceinline__ double j_normal(double a, double vol, double inv, int div8) {
+    if (kMul) return a * inv;
+    a = soft::quotient(a, vol, inv, 0);
+    return div8 ? a * 0.125 : a;
+}
+
 // The gather form of the reference adds, at node index 0 and index s of an
 // axis, the same two cells (periodic wrap of the cell index): the final value
 // of a node is the sum of the raw deposits over its image set {0, s} on every
@@ -273,11 +282,7 @@ __device__ __forceinline__ void j_finalize_point(int sx, int sy, int sz, double*
     const int comp = r & 3, z = r >> 2;
     double* const base = comp < 3 ? J + comp : rho;
     const int64_t pitch = comp < 3 ? 3 : 1;
-    const auto normal = [&](double a) {
-        if (kMul) return a * inv;
-        a = soft::quotient(a, vol, inv, 0);  // inv = 1 / vol
-        return div8 ? a * 0.125 : a;
-    };
+    const auto normal = [&](double a) { return j_normal<kMul>(a, vol, inv, div8); };
     if (x != 0 && y != 0 && z != 0) {
         double* p = base + pitch * (((int64_t)x * ny + y) * nz + z);
         *p = normal(soft::plus_zero(*p));
@@ -300,6 +305,29 @@ __device__ __forceinline__ void j_finalize_point(int sx, int sy, int sz, double*
         for (int k = 0; k < 8; ++k)
             if (in[k]) base[n[k]] = a;
     }
+}
+
+// The same by a thread per node (larger grids, launch_j_finalize; batches).
+template <bool kMul>
+__device__ __forceinline__ void j_finalize_node(int sx, int sy, int sz, double* J, double* rho, double vol, double inv,
+                                                int div8, int x, int y, int z) {
+    const int ny = sy + 1, nz = sz + 1;
+    const int nxs = x == 0 ? 2 : 1, nys = y == 0 ? 2 : 1, nzs = z == 0 ? 2 : 1;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = 0; i < nxs; ++i)
+        for (int j = 0; j < nys; ++j)
+            for (int k = 0; k < nzs; ++k) {
+                const int64_t n = ((int64_t)(i ? sx : x) * ny + (j ? sy : y)) * nz + (k ? sz : z);
+                a[0] += J[3 * n]; a[1] += J[3 * n + 1]; a[2] += J[3 * n + 2]; a[3] += rho[n];
+            }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) a[c] = j_normal<kMul>(a[c], vol, inv, div8);
+    for (int i = 0; i < nxs; ++i)
+        for (int j = 0; j < nys; ++j)
+            for (int k = 0; k < nzs; ++k) {
+                const int64_t n = ((int64_t)(i ? sx : x) * ny + (j ? sy : y)) * nz + (k ? sz : z);
+                J[3 * n] = a[0]; J[3 * n + 1] = a[1]; J[3 * n + 2] = a[2]; rho[n] = a[3];
+            }
 }
 
 __global__ void k_node32(const double* field, float4* node32, int64_t nodes) {
@@ -364,11 +392,16 @@ __global__ void k_interp_c2n(SolverArgs A) {
 template <bool kMul>
 __global__ void k_j_finalize(int sx, int sy, int sz, double* J, double* rho, double vol, double inv, int div8) {
     const int r = row_item();
-    if (r >= 4 * sz) return;
-    // grids need not be cubes: more rows than a launch has are taken in turns
-    for (int x = blockIdx.z; x < sx; x += gridDim.z)
-        for (int y = blockIdx.y; y < sy; y += gridDim.y)
-            j_finalize_point<kMul>(sx, sy, sz, J, rho, vol, inv, div8, x, y, r);
+    if (r < 4 * sz) j_finalize_point<kMul>(sx, sy, sz, J, rho, vol, inv, div8, blockIdx.z, blockIdx.y, r);
+}
+template <bool kMul>
+__global__ void __launch_bounds__(256)
+    k_j_finalize_flat(int sx, int sy, int sz, double* J, double* rho, double vol, double inv, int div8) {
+    for (int64_t t = grid_t0(); t < (int64_t)sx * sy * sz; t += grid_stride()) {
+        int x, y, z;
+        split3(t, sy, sz, x, y, z);
+        j_finalize_node<kMul>(sx, sy, sz, J, rho, vol, inv, div8, x, y, z);
+    }
 }
 template <bool kMul>
 __global__ void k_forward_e(SolverArgs A) { forward_e_body<kMul>(A, grid_t0(), grid_stride()); }
@@ -423,10 +456,8 @@ __global__ void k_j_finalize_batch(const InstJob* jobs) {
     for (int64_t t = grid_t0(); t < (int64_t)g.sx * g.sy * g.sz; t += grid_stride()) {
         int x, y, z;
         split3(t, g.sy, g.sz, x, y, z);
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-            if (b.mul_vol) j_finalize_point<true>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol, inv, b.div8, x, y, 4 * z + a);
-            else j_finalize_point<false>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol, inv, b.div8, x, y, 4 * z + a);
+        if (b.mul_vol) j_finalize_node<true>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol, inv, b.div8, x, y, z);
+        else j_finalize_node<false>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol, inv, b.div8, x, y, z);
     }
 }
 
@@ -564,8 +595,8 @@ int launch_ghost(const Geom& g, cudaStream_t st) {
     return 1;
 }
 
-// The launch of a row kernel: nx x ny rows of `items`, up to 65535 each way
-// (the solvers' grids are cubes, which stay far below).
+// The launch of a row kernel: nx x ny rows of `items`, at most 65535 each way
+// (the solvers' grids are cubes, the J finalisation takes few rows this way).
 struct Rows {
     dim3 grid;
     unsigned threads;
@@ -573,7 +604,7 @@ struct Rows {
 static Rows rows(int nx, int ny, int items) {
     Rows r;
     r.threads = (unsigned)(items < 256 ? (items + 31) / 32 * 32 : 256);
-    r.grid = dim3((items + r.threads - 1) / r.threads, std::min(ny, 65535), std::min(nx, 65535));
+    r.grid = dim3((items + r.threads - 1) / r.threads, ny, nx);
     return r;
 }
 
@@ -629,13 +660,25 @@ static void set_raw_j(SolverArgs& A, const Geom& g, bool div8, bool exact) {
 }
 
 int launch_j_finalize(const Geom& g, bool div8, bool exact, cudaStream_t st) {
+    const bool mul = !exact || pow2(g.vol);  // vol = 2^k: 1 / vol is exact
+    const double inv = mul && div8 ? 1.0 / g.vol / 8.0 : 1.0 / g.vol;
+    const int64_t nodes = (int64_t)g.sx * g.sy * g.sz;
+    // Above 160,000 nodes or 16,384 rows a thread per node is faster, below a
+    // row's items side by side, whose blocks are then too many and too small.
+    // us, rows / nodes (in brackets with the exact quotient): 32^3 4.6 / 10
+    // (6.3 / 10.5), 48^3 8.2 / 11.5 (13.3 / 13.0), 59^3 11.6 / 10.9 (23 /
+    // 19), 128^3 61 / 47 (125 / 120), 70 x 70 x 16 7.4 / 11.6 (12 / 13), 256 x
+    // 256 x 4 43 / 13 (83 / 22), 1024 x 1024 x 1, 4 items a row, 579 / 31
+    // (895 / 66).
+    const bool flat = nodes > 160000 || (int64_t)g.sx * g.sy > 16384;
     const Rows r = rows(g.sx, g.sy, 4 * g.sz);
-    if (exact && !pow2(g.vol))  // vol = 2^k: 1 / vol is exact
-        k_j_finalize<false><<<r.grid, r.threads, 0, st>>>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol, 1.0 / g.vol,
-                                                          div8 ? 1 : 0);
-    else
-        k_j_finalize<true><<<r.grid, r.threads, 0, st>>>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol,
-                                                  div8 ? 1.0 / g.vol / 8.0 : 1.0 / g.vol, div8 ? 1 : 0);
+    const auto run = [&](auto k, dim3 grid, unsigned threads) {
+        k<<<grid, threads, 0, st>>>(g.sx, g.sy, g.sz, g.J, g.rho, g.vol, inv, div8 ? 1 : 0);
+    };
+    if (flat && mul) run(k_j_finalize_flat<true>, grid_for(nodes, 256), 256);
+    else if (flat) run(k_j_finalize_flat<false>, grid_for(nodes, 256), 256);
+    else if (mul) run(k_j_finalize<true>, r.grid, r.threads);
+    else run(k_j_finalize<false>, r.grid, r.threads);
     return 1;
 }
 
