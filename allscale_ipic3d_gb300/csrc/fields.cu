@@ -47,7 +47,7 @@ __device__ __forceinline__ void ghost_body(double* g, int n, int per, int64_t t0
 
 struct SolverArgs {
     int s;                // cells per axis (cubic)
-    double dt, c;
+    double dt, c, c2;     // c2 = c^2
     double w[3];
     double iw[3];         // 1 / w
     float4* n32;          // FP32 node copy {Ex,Ey,Ez,0},{Bx,By,Bz,0} kept current (FP32 path), or null
@@ -135,9 +135,8 @@ __device__ __forceinline__ void leapfrog_e_point(const SolverArgs& A, const Node
     const double J = read_j(A, p.x - 1, p.y - 1, p.z - 1, p.a);
     const int64_t f = fidx(nf, p.x, p.y, p.z);
     double* E = A.field + 9 * f + p.a;
-    const double c2 = A.c * A.c;
     const double e =
-        *E + A.dt * (c2 * (over<kMul>(B0[p.c] - Bb[p.c], wb, iwb) - over<kMul>(B0[p.b] - Bc[p.b], wc, iwc)) - J);
+        *E + A.dt * (A.c2 * (over<kMul>(B0[p.c] - Bb[p.c], wb, iwb) - over<kMul>(B0[p.b] - Bc[p.b], wc, iwc)) - J);
     *E = e;
     if (A.n32) reinterpret_cast<float*>(A.n32 + 2 * f)[p.a] = (float)e;
 }
@@ -346,6 +345,7 @@ __host__ __device__ inline SolverArgs solver_args(const Geom& g) {
     A.s = g.sx;
     A.dt = g.dt;
     A.c = g.c;
+    A.c2 = g.c * g.c;
     for (int a = 0; a < 3; ++a) {
         A.w[a] = g.w[a];
         A.iw[a] = g.inv_w[a];
@@ -603,8 +603,10 @@ struct Rows {
 };
 static Rows rows(int nx, int ny, int items) {
     Rows r;
-    r.threads = (unsigned)(items < 256 ? (items + 31) / 32 * 32 : 256);
-    r.grid = dim3((items + r.threads - 1) / r.threads, ny, nx);
+    // evenly: 387 items (128^3) are a block of 416 threads, not 256 and 131
+    const int blocks = (items + 511) / 512, each = (items + blocks - 1) / blocks;
+    r.threads = (unsigned)(each + 31) / 32 * 32;
+    r.grid = dim3(blocks, ny, nx);
     return r;
 }
 
