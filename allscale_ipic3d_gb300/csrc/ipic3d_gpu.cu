@@ -276,10 +276,6 @@ enum StepKind : int {
     kStepMove = 3,       // the move alone (last step of a run)
 };
 
-// Steps of one replay in long runs: between replays the pending counts come
-// back and the next graph starts, 6 to 15 us in which the GPU waits.
-constexpr int kUnroll = 8;
-
 void release_pops(ipic3d_ctx* ctx) {
     for (auto& p : ctx->p32) p.release();
     for (auto& p : ctx->p64) p.release();
@@ -303,17 +299,40 @@ int64_t cell_capacity(const ipic3d_config& cfg, uint64_t n) {
     return std::max<int64_t>(cap, kSlotAlign);
 }
 
+// Steps of one replay in long runs: between replays the pending counts come
+// back and the next graph starts, 6 to 15 us in which the GPU waits.
+constexpr int kUnroll = 8;
+
+// Particles injected per step, at most.
+int64_t inject_bound(const ipic3d_ctx* ctx) {
+    if (!(ctx->cfg.flags & IPIC3D_F_INJECT_LOW_X)) return 0;
+    return (int64_t)(ctx->props.size[1] * ctx->props.size[2]) * ((int64_t)ctx->cfg.inject_per_cell + 1);
+}
+
+// Whether the pending list of the injected population (the first) holds what
+// can wait two replays after `waiting` particles did: the particles stored and
+// waiting then, at most its slots and `waiting`, and those injected since.
+template <typename T>
+bool unroll_safe(const ipic3d_ctx* ctx, const std::vector<PopStore<T>>& pops, uint64_t waiting) {
+    const int64_t in = 2 * kUnroll * inject_bound(ctx);
+    return in == 0 || pops.empty() || (int64_t)pops[0].pending_cap - pops[0].capacity >= in + (int64_t)waiting;
+}
+
 template <typename T>
 int alloc_pop(ipic3d_ctx* ctx, PopStore<T>& P, const std::vector<uint64_t>& counts, int64_t extra_pending) {
     const int64_t nc = ctx->ncells();
     P.h_start.assign(nc + 1, 0);
     for (int64_t c = 0; c < nc; ++c) P.h_start[c + 1] = P.h_start[c] + cell_capacity(ctx->cfg, counts[c]);
     P.capacity = P.h_start[nc];
-    // every particle can wait at most once per step: capacity entries suffice
-    P.pending_cap = (uint32_t)std::min<int64_t>(std::max<int64_t>(1 << 12, P.capacity), 0x7fffffff);
-    int64_t inject_cap = 0;
-    if (ctx->cfg.flags & IPIC3D_F_INJECT_LOW_X)
-        inject_cap = (int64_t)(ctx->props.size[1] * ctx->props.size[2]) * ((int64_t)ctx->cfg.inject_per_cell + 1);
+    // Every particle can wait at most once per step: capacity entries suffice
+    // for the particles of the layout. Those injected since (into the first
+    // population) are as many as the steps until a re-layout bring: room for
+    // two replays of kUnroll steps (unroll_safe) beside 3 % waiting already.
+    const int64_t inject_cap = inject_bound(ctx);
+    int64_t wait = std::max<int64_t>(1 << 12, P.capacity);
+    if (inject_cap && P.q == ctx->cfg.inject_q && P.qom == ctx->cfg.inject_qom)
+        wait += P.capacity / 32 + 2 * kUnroll * inject_cap;
+    P.pending_cap = (uint32_t)std::min<int64_t>(wait, 0x7fffffff);
     const int64_t ob = P.capacity + P.pending_cap + inject_cap + extra_pending;
     if (ob > 0x7fffffff) return fail(IPIC3D_E_CAPACITY, "population too large for 32-bit outbox indices");
     P.outbox_cap = (uint32_t)ob;
@@ -1114,11 +1133,6 @@ int ph_collect(ipic3d_ctx* ctx) {
     return IPIC3D_OK;
 }
 
-bool injects(const ipic3d_ctx* ctx) {
-    return (ctx->cfg.flags & IPIC3D_F_INJECT_LOW_X) && ctx->cfg.bc_low[0] == IPIC3D_BC_OPEN &&
-           ctx->cfg.inject_per_cell > 0;
-}
-
 // Clears the step counters and, with `moments`, J and rho (k_step_begin).
 int step_begin(ipic3d_ctx* ctx, bool counters, bool moments, cudaStream_t st) {
     CounterSet s{};
@@ -1223,7 +1237,9 @@ int move_impl(ipic3d_ctx* ctx, bool deposit, bool next_solve = false, bool clear
     for (auto& S : s32) n += launch_push_pending<float>(g, S, aux);
     for (auto& S : s64) n += launch_push_pending<double>(g, S, aux);
     ph_end(ctx, IPIC3D_PHASE_PENDING);
-    if (injects(ctx)) {
+    const bool inject = (ctx->cfg.flags & IPIC3D_F_INJECT_LOW_X) && ctx->cfg.bc_low[0] == IPIC3D_BC_OPEN &&
+                        ctx->cfg.inject_per_cell > 0;
+    if (inject) {
         ph_begin(ctx, IPIC3D_PHASE_INJECT);
         if (ctx->fp32)
             n += launch_inject<float>(g, ctx->p32[0].view(), ctx->cfg.inject_per_cell, ctx->cfg.inject_drift,
@@ -1774,11 +1790,10 @@ int ipic3d_gpu_step(ipic3d_ctx* ctx, uint64_t num_steps) {
     // the longer graph pays for itself over a few replays). A re-layout then
     // comes up to two replays after its limit is passed, which no run has been
     // seen to suffer from (converging flows of 0.3M and 1M particles, 30 to
-    // 200 steps: as fast or faster, with half the re-layouts). Injection is
-    // another matter: the pending list is sized for the particles of the last
-    // layout, and holds the injected ones too only if the universe is laid out
-    // anew within two steps
-    const bool unroll = use_graph && num_steps >= 3 * kUnroll && !injects(ctx);
+    // 200 steps: as fast or faster, with half the re-layouts); with injection
+    // the pending list has to hold what comes meanwhile
+    const bool unroll = use_graph && num_steps >= 3 * kUnroll;
+    const auto safe = [&] { return unroll_safe(ctx, ctx->p32, pend_limit) && unroll_safe(ctx, ctx->p64, pend_limit); };
     uint64_t round = 0;  // replays (or eager steps) so far
     for (uint64_t done = 0; done < num_steps; ++round) {
         uint64_t steps = 1;
@@ -1792,11 +1807,11 @@ int ipic3d_gpu_step(ipic3d_ctx* ctx, uint64_t num_steps) {
         } else if (overlap && (presolved || done + 1 < num_steps)) {
             if (!presolved && (rc = run_graph(ctx, kStepSolve))) return rc;
             const bool last = done + 1 == num_steps;
-            if (unroll && num_steps - done > kUnroll) steps = kUnroll;
+            if (unroll && num_steps - done > kUnroll && safe()) steps = kUnroll;
             if ((rc = run_graph(ctx, last ? kStepMove : kStepMoveSolve, (int)steps))) return rc;
             presolved = !last;
         } else if (use_graph) {  // a lone step (or no field solver): one graph
-            if (unroll && !overlap && num_steps - done > kUnroll) steps = kUnroll;
+            if (unroll && !overlap && num_steps - done > kUnroll && safe()) steps = kUnroll;
             if ((rc = run_graph(ctx, kStepFull, (int)steps))) return rc;
         } else {
             if ((rc = enqueue_step(ctx))) return rc;
