@@ -106,7 +106,8 @@ struct Pop {
     StepCounters* ctr;
     int64_t capacity;       // total slots
     double q, qom;
-    int32_t pad[2];
+    int32_t tile_cells;     // most cells that a tile of kSlotsPerCta slots touches
+    int32_t pad;
 };
 
 // Up to kSetPops populations of one universe advanced by one launch

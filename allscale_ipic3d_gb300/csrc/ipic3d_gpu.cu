@@ -67,6 +67,7 @@ struct PopStore {
     double q = 0, qom = 0;
     int64_t capacity = 0;
     uint32_t pending_cap = 0, outbox_cap = 0;
+    int32_t tile_cells = 0;
     T *x = nullptr, *y = nullptr, *z = nullptr, *u = nullptr, *v = nullptr, *w = nullptr;
     uint32_t* id = nullptr;
     int64_t* start = nullptr;
@@ -107,7 +108,8 @@ struct PopStore {
         P.capacity = capacity;
         P.q = q;
         P.qom = qom;
-        P.pad[0] = P.pad[1] = 0;
+        P.tile_cells = tile_cells;
+        P.pad = 0;
         return P;
     }
 };
@@ -368,6 +370,7 @@ int alloc_pop(ipic3d_ctx* ctx, PopStore<T>& P, const std::vector<uint64_t>& coun
     // push CTA b covers slots [b*kSlotsPerCta, (b+1)*kSlotsPerCta): its cells
     const int64_t nb = (P.capacity + kSlotsPerCta - 1) / kSlotsPerCta;
     std::vector<int2> cc((size_t)std::max<int64_t>(nb, 1));
+    P.tile_cells = 0;
     int64_t c = 0;
     for (int64_t b = 0; b < nb; ++b) {
         const int64_t first = b * kSlotsPerCta, last = std::min(first + kSlotsPerCta, P.capacity) - 1;
@@ -375,6 +378,7 @@ int alloc_pop(ipic3d_ctx* ctx, PopStore<T>& P, const std::vector<uint64_t>& coun
         int64_t e = c;
         while (P.h_start[e + 1] <= last) ++e;
         cc[b] = make_int2((int)c, (int)(e - c + 1));
+        P.tile_cells = std::max(P.tile_cells, (int32_t)(e - c + 1));
         if (e - c + 1 > kMaxCellsPerCta) return fail(IPIC3D_E_INVALID, "layout: a push CTA spans too many cells");
     }
     CU(cudaMalloc(&P.cta_cells, cc.size() * sizeof(int2)));
@@ -2071,6 +2075,7 @@ struct ipic3d_batch {
     uint32_t* h_flag = nullptr;  // pinned ring of two
     cudaEvent_t flag_ev[2] = {nullptr, nullptr};
     int64_t nctas = 0, nplace = 0;
+    int tile_cells = 0;  // the most cells of any tile
     int max_s = 0;
     int64_t max_cells = 0, max_nodes = 0;
     bool tables = false;
@@ -2196,6 +2201,8 @@ int batch_tables(ipic3d_batch* b) {
     cur.swap(nj);
     b->ij.swap(ni);
     b->nctas = (int64_t)cta.size();
+    b->tile_cells = 0;
+    for (const auto& j : cur) b->tile_cells = std::max(b->tile_cells, (int)j.P.tile_cells);
     b->nplace = (int64_t)place.size();
     b->max_s = max_s;
     b->max_cells = max_cells;
@@ -2234,7 +2241,7 @@ int batch_enqueue_step(ipic3d_batch* b) {
     if (nj > 0) {
         if ((rc = fork(0, st, aux))) return rc;
         if (b->tune_timing) CU(cudaEventRecord(b->tune_ev[0], st));
-        n += launch_push_batch<T>(jobs, b->d_cta, b->nctas, 0, jobs_of<T>(b)[0].g, b->tuner.next(), st);
+        n += launch_push_batch<T>(jobs, b->d_cta, b->nctas, 0, jobs_of<T>(b)[0].g, b->tile_cells, b->tuner.next(), st);
         if (b->tune_timing) CU(cudaEventRecord(b->tune_ev[1], st));
         n += launch_push_pending_batch<T>(jobs, nj, aux);
         if ((rc = fork(1, aux, st))) return rc;

@@ -22,7 +22,8 @@ using PipeJobsFn = void (*)(const PopJob<float>*, const int2*, int, PushShape);
 
 // The compile-time policies that are instantiated (kPipe* bit sets): the
 // step with the dipole mover, the field-gather mover with or without the
-// dipole term, each with or without the deposit; and the deposit alone.
+// dipole term, each with or without the deposit; the deposit alone; and the
+// gather with deposit for launches without a sparse tile (pipe_policy).
 constexpr int kPipeVariants[] = {
     kPipeStep | kPipeDipole,
     kPipeStep | kPipeDipole | kPipeDeposit,
@@ -31,6 +32,7 @@ constexpr int kPipeVariants[] = {
     kPipeStep | kPipeGather | kPipeDipole,
     kPipeStep | kPipeGather | kPipeDipole | kPipeDeposit,
     kPipeDeposit,
+    kPipeStep | kPipeGather | kPipeDeposit | kPipeItems,
 };
 
 template <int kF>
@@ -52,18 +54,38 @@ PipeJobsFn pipe_jobs_kernel(int f) {
         case kPipeStep | kPipeGather | kPipeDipole: return pipe_jobs_fn<kPipeStep | kPipeGather | kPipeDipole>();
         case kPipeStep | kPipeGather | kPipeDipole | kPipeDeposit:
             return pipe_jobs_fn<kPipeStep | kPipeGather | kPipeDipole | kPipeDeposit>();
+        case kPipeStep | kPipeGather | kPipeDeposit | kPipeItems:
+            return pipe_jobs_fn<kPipeStep | kPipeGather | kPipeDeposit | kPipeItems>();
         case kPipeDeposit: return pipe_jobs_fn<kPipeDeposit>();
         default: return nullptr;
     }
 }
 
-// The policy bits of a launch: mode 0 = step, 1 = deposit only.
-int pipe_policy(const Geom& g, int mode) {
+// the device-side limits of a shape (item a power of two from 32 to a
+// tile, item mode only where the cells' coefficients fit the stage)
+PushShape clamp_shape(PushShape s) {
+    int item = 32;
+    while (item * 2 <= std::min(kTileSlots, s.item)) item *= 2;
+    s.item = item;
+    s.item_cells = std::max(0, std::min(kItemMaxCells, s.item_cells));
+    return s;
+}
+
+// The policy bits of a launch over tiles of at most `tile_cells` cells: mode
+// 0 = step, 1 = deposit only.
+int pipe_policy(const Geom& g, int mode, int tile_cells, const PushShape& shp) {
     int f = g.deposit ? kPipeDeposit : 0;
     if (mode == 0) {
         f |= kPipeStep;
         if (g.mover == 1) f |= kPipeGather;
         if (g.mover != 1 || (g.flags & 4u)) f |= kPipeDipole;
+        // Full cells: an instance without slot mode, whose code beside the
+        // item mode's costs the gather + deposit instance 44 bytes of spills
+        // (134M particles in 64^3 uneven cells: push 1.637 -> 1.617 ms, step
+        // 1.816 -> 1.792; a batch of 64 universes 0.752 -> 0.736 ms). The
+        // others have none, or, with the dipole term, gain nothing from it.
+        if (f == (kPipeStep | kPipeGather | kPipeDeposit) && tile_cells <= clamp_shape(shp).item_cells)
+            f |= kPipeItems;
     }
     return f;
 }
@@ -77,6 +99,8 @@ PipeFn pipe_kernel(int f) {
         case kPipeStep | kPipeGather | kPipeDipole: return pipe_fn<kPipeStep | kPipeGather | kPipeDipole>();
         case kPipeStep | kPipeGather | kPipeDipole | kPipeDeposit:
             return pipe_fn<kPipeStep | kPipeGather | kPipeDipole | kPipeDeposit>();
+        case kPipeStep | kPipeGather | kPipeDeposit | kPipeItems:
+            return pipe_fn<kPipeStep | kPipeGather | kPipeDeposit | kPipeItems>();
         case kPipeDeposit: return pipe_fn<kPipeDeposit>();
         default: return nullptr;
     }
@@ -135,15 +159,6 @@ int pipe_grid(const PushShape& shp, int64_t tiles) {
     return (int)std::min<int64_t>((int64_t)per_sm * sms, tiles);
 }
 
-// the device-side limits of a shape (item a power of two from 32 to a
-// tile, item mode only where the cells' coefficients fit the stage)
-PushShape clamp_shape(PushShape s) {
-    int item = 32;
-    while (item * 2 <= std::min(kTileSlots, s.item)) item *= 2;
-    s.item = item;
-    s.item_cells = std::max(0, std::min(kItemMaxCells, s.item_cells));
-    return s;
-}
 }  // namespace
 
 Push32Const push32_const(const Geom& g, const Pop<float>& P) {
@@ -173,8 +188,11 @@ Push32Const push32_const(const Geom& g, const Pop<float>& P) {
 template <>
 int launch_push<float>(const Geom& g, const PopSet<float>& S, int mode, const PushShape& shp, cudaStream_t st) {
     if (mode != 0 && !g.deposit) return 0;  // nothing to deposit
-    PipeFn fn = pipe_kernel(pipe_policy(g, mode));
-    if (!fn || S.n <= 0) return 0;
+    if (S.n <= 0) return 0;
+    int tile_cells = 0;
+    for (int i = 0; i < S.n; ++i) tile_cells = std::max(tile_cells, S.p[i].tile_cells);
+    PipeFn fn = pipe_kernel(pipe_policy(g, mode, tile_cells, shp));
+    if (!fn) return 0;
     TileMap tm{};
     tm.n = S.n;
     Push32Set pcs{};
@@ -216,10 +234,10 @@ int launch_cell_coef(const Geom& g, float* coef, cudaStream_t st) {
 // the batched FP32 step: the pipelined push over every job's tiles
 template <>
 int launch_push_batch<float>(const PopJob<float>* jobs, const int2* cta_job, int64_t nctas, int mode,
-                             const Geom& g0, const PushShape& shp, cudaStream_t st) {
+                             const Geom& g0, int tile_cells, const PushShape& shp, cudaStream_t st) {
     if (nctas <= 0) return 0;
     if (mode != 0 && !g0.deposit) return 0;
-    PipeJobsFn fn = pipe_jobs_kernel(pipe_policy(g0, mode));
+    PipeJobsFn fn = pipe_jobs_kernel(pipe_policy(g0, mode, tile_cells, shp));
     if (!fn) return 0;
     fn<<<pipe_grid(shp, nctas), kPipeThreads, pipe_smem_bytes<kPipeStages>(), st>>>(jobs, cta_job, (int)nctas,
                                                                                     clamp_shape(shp));

@@ -99,7 +99,7 @@ template int launch_pending_count<double>(const Pop<double>&, int32_t*, cudaStre
 
 template <>
 int launch_push_batch<double>(const PopJob<double>* jobs, const int2* cta_job, int64_t nctas, int mode,
-                              const Geom& g, const PushShape&, cudaStream_t st) {
+                              const Geom& g, int, const PushShape&, cudaStream_t st) {
     if (nctas <= 0 || (mode != 0 && !g.deposit)) return 0;
     const Shape64 sh = shape64(nctas * kSlotsPerCta, nctas, g.deposit != 0);
     const unsigned grid = (unsigned)(nctas * sh.parts);

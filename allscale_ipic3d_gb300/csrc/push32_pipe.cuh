@@ -250,6 +250,7 @@ enum : int {
     kPipeGather = 2,   // field-gather mover: E, B from the cell's polynomial
     kPipeDipole = 4,   // analytic dipole B added
     kPipeDeposit = 8,  // cloud-in-cell deposit of J and rho
+    kPipeItems = 16,   // no tile has more than item_cells cells: no slot mode
 };
 
 __device__ __forceinline__ PState<float> load_slot(const PipeStage& st, int sl) {
@@ -805,7 +806,7 @@ __device__ __forceinline__ bool push_tile_warp(const Geom& g, const Pop<float>& 
     int first = 0;
     if (lane == 0) first = atomicAdd(td.claim, 1) == 0;
     first = __shfl_sync(0xffffffffu, first, 0);
-    if (nc > shp.item_cells) {
+    if (!(kF & kPipeItems) && nc > shp.item_cells) {
         if (first && lane == 0) mbar_arrive(td.ready);
         // slices are claimed like items: 8 slices for 11 warps, the others
         // go on to the next stage's
