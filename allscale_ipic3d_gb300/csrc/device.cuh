@@ -259,13 +259,6 @@ __device__ __forceinline__ int fast_div(int a, int d, float inv_d) {
     return q;
 }
 
-// Files slot `slot` as a hole of cell c (its slots start at cstart).
-template <typename T>
-__device__ __forceinline__ void file_hole(const Pop<T>& P, int c, int64_t cstart, int64_t slot) {
-    const int k = atomicAdd(P.hole_cnt + c, 1);
-    P.hole_list[cstart + k] = (int32_t)slot;
-}
-
 // t = (a * n1 + b) * n2 + c for t in [0, n0 * n1 * n2): 32-bit divisions
 // when t fits (64-bit division by a runtime divisor is a long software
 // sequence on the GPU).

@@ -224,6 +224,14 @@ IPG_HD double quotient(double a, double w, double inv, int exact) {
     return fused(fused(-w, q, a), inv, q);
 }
 
+// 1 / d to an ulp from y with relative error e = 1 - d y below 2^-20: two terms
+// of the geometric series 1 / d = y (1 + e + e^2 + ...), the third-order Newton
+// iteration (Brent & Zimmermann, 4.2).
+IPG_HD double refine_reciprocal(double d, double y) {
+    const double e = fused(-d, y, 1.0);
+    return fused(y, fused(e, e, e), y);
+}
+
 // FP32 estimates (relative error at most 2^-22 for the functions below)
 IPG_HD float estimate_rcp(float x) {
 #ifdef __CUDA_ARCH__

@@ -52,37 +52,15 @@ constexpr int kCoefStride64 = 50;  // 48 + 2: the four groups of a warp read dif
 
 // ---- field --------------------------------------------------------------------
 
-// Approximations of the FP64 unit's seed instructions (relative error at
-// most 2^-20), refined below.
-__device__ __forceinline__ double seed_rsqrt(double x) {
-    double r;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    return r;
-}
-__device__ __forceinline__ double seed_rcp(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    return r;
-}
-
-// 1 / d: y (1 + e + e^2), e = 1 - d y
+// 1 / d from the FP64 unit's approximation (relative error below 2^-20).
 __device__ __forceinline__ double reciprocal(double d) {
-    const double y = seed_rcp(d);
-    const double e = __fma_rn(-d, y, 1.0);
-    return __fma_rn(y, __fma_rn(e, e, e), y);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    return soft::refine_reciprocal(d, y);
 }
 
-// r2^(-5/2) out of the integer path's range: y = r2^(-1/2) by y (1 + e / 2 + 3 e^2 / 8), e = 1 - r2 y^2, and
-// one correction of y^5 from the residual of y^2
-__device__ __forceinline__ double inverse_pow25(double r2) {
-    double y = seed_rsqrt(r2);
-    const double e = __fma_rn(-__dmul_rn(r2, y), y, 1.0);
-    y = __fma_rn(y, __dmul_rn(e, __fma_rn(0.375, e, 0.5)), y);
-    const double y2 = __dmul_rn(y, y);
-    const double f = __dmul_rn(__dmul_rn(y2, y2), y);
-    const double d = __fma_rn(-r2, y2, 1.0);
-    return __fma_rn(f, __dmul_rn(2.5, d), f);
-}
+// mft / r2^2.5 out of the integer path's range.
+__device__ __noinline__ double dipole_factor(double mft, double r2) { return mft / pow25_rn(r2); }
 
 // The field of a cell in 64-bit fixed point. A component's 8 corner values
 // share the largest one's exponent e_max: fixed = value 2^(1081 - e_max), below
@@ -245,7 +223,8 @@ __device__ __noinline__ PState<double> boris_large64(double ex, double ey, doubl
 // The field mover's step from the gathered E, B in F.
 __device__ __forceinline__ void move_field64(const Geom& g, const Push64Const& pc, double qom, double (&F)[6],
                                              PState<double>& p) {
-    if (g.flags & 4u /*IPIC3D_F_DIPOLE_IN_GATHER*/) {
+    // (without a dipole moment the dipole's field is zero at a finite distance)
+    if ((g.flags & 4u /*IPIC3D_F_DIPOLE_IN_GATHER*/) && !(pc.no_field && coordinates_regular(p.x, p.y, p.z))) {
         const double r2 = __fma_rn(p.x, p.x, __fma_rn(p.y, p.y, __dmul_rn(p.z, p.z)));
         // mft / r2^2.5 on the integer pipe
         double f;
@@ -253,7 +232,7 @@ __device__ __forceinline__ void move_field64(const Geom& g, const Push64Const& p
             bool sure;  // either neighbour will do where it is not
             f = soft::pack(soft::div(pc.d.mft, soft::divisor(soft::pow25(soft::unpack(r2), sure))));
         } else {
-            f = __dmul_rn(g.mft, inverse_pow25(r2));
+            f = dipole_factor(g.mft, r2);
         }
         const double z3 = __dmul_rn(3.0, p.z), zf = __dmul_rn(z3, f);
         F[3] = __fma_rn(p.x, zf, F[3]);
