@@ -3,8 +3,9 @@
 
 The FP64 particle kernels and the field kernels are compiled with
 ``-fmad=false``: the reference's x86 build never fuses a multiply with an
-add, and the FP64 path reproduces its rounding term by term. The FP32
-kernels keep fused multiply-adds.
+add, and the dipole mover, the export, the tracer and the field solvers
+round as it does (the FP64 field mover and deposit fuse where they say so).
+The FP32 kernels keep fused multiply-adds.
 """
 import os
 import shutil

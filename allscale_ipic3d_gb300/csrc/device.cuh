@@ -21,9 +21,7 @@
 
 namespace ipg {
 
-constexpr int kVec = 4;                 // particles per thread (one float4 / 2x double2)
-constexpr int kPushThreads = 256;       // threads per CTA of the push kernel
-constexpr int kSlotsPerCta = kVec * kPushThreads;
+constexpr int kSlotsPerCta = 1024;      // slots of a tile
 constexpr int kSetPops = 4;             // populations per launch of the population-set kernels
 constexpr int kSlotAlign = 8;          // start[] and every cell's capacity are multiples of 8
 constexpr int kPlaceThreads = 128;

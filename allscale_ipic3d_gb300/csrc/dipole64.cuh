@@ -6,8 +6,8 @@
 // and sub-partition), so the field, the squares, the quotients and the
 // position's products run on the integer pipe (fp64_int.cuh) and the
 // velocity's cross products and the sums that can cancel stay FP64: 35 FP64
-// instructions per particle step in place of about 149, beside about 1600
-// others (pipe use: FP64 83 %, integer 59 %). Moving 3 or 6 products of the
+// instructions per particle step in place of about 149, beside about 1700
+// others (pipe use: FP64 78 %, integer ALU 66 %). Moving 3 or 6 products of the
 // cross products over as well was slower (tracer, 16M particles x 151 steps:
 // 177 and 189 ms against 163 ms; all FP64 641 ms).
 #pragma once

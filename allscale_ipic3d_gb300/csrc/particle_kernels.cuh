@@ -1,18 +1,17 @@
-// Particle kernels of the GB300 path, templated on the storage type:
-//   T = double : absolute FP64 positions, the reference's arithmetic order
-//                (compiled with -fmad=false so no product is fused);
-//   T = float  : FP32 positions relative to the cell origin in cell widths.
-//
-// One step of the reference's active loop (simulator.h:214-223) is
-//   k_push      mover (cell.h:896-964) + export (cell.h:975-1159), in place,
-//               fused with the cloud-in-cell deposit of the moved particles
-//               (cell.h:787-824, scatter form) for the next step's solver;
-//               leavers go to an outbox (the TransferBuffers of
-//               transfer_buffer.h:48-95, compacted with warp ballots);
-//   k_push_pending  the same for particles that found no slot last step;
-//   k_inject    x=0 injection (not in the reference);
-//   k_place     import (cell.h:1195-1310): one warp per cell fills the holes
-//               left by leavers with arrivals and compacts the cell.
+// What the FP32 and FP64 particle kernels share, templated on the storage
+// type (double: absolute positions; float: positions relative to the cell
+// origin in cell widths): r^2.5 and the Boris rotation as the reference
+// rounds them, the sub-cycle rule, the deposit of single particles, the
+// outbox and arrival lists (the TransferBuffers of transfer_buffer.h:48-95),
+// and these kernels of a step of the reference's active loop
+// (simulator.h:214-223):
+//   k_inject          x = 0 injection (not in the reference);
+//   k_place           import (cell.h:1195-1310): a warp scans a few cells and
+//                     fills the holes left by leavers with arrivals;
+//   k_pending_rotate  hands the particles without a slot to the next step;
+//   k_relayout_copy, k_pending_place, k_pending_count  the re-layout.
+// The mover, export and deposit of the bulk are in push32_pipe.cuh and
+// push64.cuh, of the particles that waited in push32.cuh and push64.cuh.
 #pragma once
 
 #include <type_traits>

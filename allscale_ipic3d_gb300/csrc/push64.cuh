@@ -4,7 +4,7 @@
 // GB300's FP64 pipe bounds it (one warp instruction per 64 to 76 cycles and
 // SM sub-partition), so what counts is the number of FP64 instructions a
 // warp issues -- idle lanes cost as much as busy ones -- then how many warps
-// there are to fill the gaps, and the size of the loop (five warps a
+// there are to fill the gaps, and the size of the loop (four or five warps a
 // sub-partition, each elsewhere in it, share the instruction cache). Per 32
 // particles of a step with field gather, dipole and deposit:
 //   * the field is the cell's trilinear polynomial, built once per work item
@@ -17,11 +17,11 @@
 //   * comparisons run on the doubles' bit patterns in the integer pipe;
 //   * rare parts (walls, planet, sub-cycles, positions outside the cell) are
 //     calls: predicated off they would still take the FP64 pipe.
-// 62 FP64 instructions (items' shares and idle lanes included) and 2,600
+// 62 FP64 instructions (items' shares and idle lanes included) and 2,700
 // others in place of 541 FP64 ones before. The dipole mover without the
 // gather rounds exactly as the reference does (dipole64.cuh). Measured push
 // per step, before and after: 8.4M particles, gather + dipole + deposit
-// 9.18 -> 1.30 ms (FP64 pipe 67 % busy, issue slots 47 %); 306k particles,
+// 9.18 -> 1.30 ms (FP64 pipe 66 % busy, issue slots 46 %); 306k particles,
 // two species, gather + deposit 0.593 -> 0.081 ms; 33k particles 0.140 ->
 // 0.021 ms (a warp's serial chain); 1.05M particles, dipole mover, a sixth of
 // them leaving their cells 0.489 -> 0.150 ms (FP64 pipe 58 %, integer 42 %).
@@ -65,7 +65,8 @@ __device__ __noinline__ double dipole_factor(double mft, double r2) { return mft
 // The field of a cell in 64-bit fixed point. A component's 8 corner values
 // share the largest one's exponent e_max: fixed = value 2^(1081 - e_max), below
 // 2^59, so that one unit is 2^-59 of the largest corner (FP64's own rounding
-// is 2^-53 of it). The trilinear polynomial's coefficients are differences of
+// is 2^-53 of it; a corner below 2^-6 of the largest keeps fewer than 53 bits,
+// which shows only at positions that the others hardly reach). The trilinear polynomial's coefficients are differences of
 // these integers, exact, and the position in the cell is a 64-bit fraction:
 // a product is the high half of 64 x 64 bits. Seven of them and seven sums per
 // component take about 150 integer-pipe cycles per warp; the seven FP64

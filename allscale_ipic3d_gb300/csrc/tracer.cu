@@ -11,8 +11,8 @@
 // reference's order (built with -fmad=false): r^2.5 correctly rounded, the
 // sub-cycle rule, the Boris rotation and the periodic wrap are those of the
 // reference, so trajectories and counts match its host build. What bounds it
-// is the FP64 pipe (37 instructions per particle step at 64 to 76 cycles per
-// warp, 83 % busy), which is why most of the step's roundings are made on
+// is the FP64 pipe (35 instructions per particle step at 64 to 76 cycles per
+// warp, 78 % busy), which is why most of the step's roundings are made on
 // the integer pipe (dipole64.cuh) and the rare comparisons sit behind calls:
 // 16M particles x 151 steps 641 -> 163 ms, 20k x 41 steps 432 -> 162 us.
 #include <cmath>

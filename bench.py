@@ -158,7 +158,7 @@ def measured_peak():
 # 2; k_push64); a citation of that capture, not a measurement of this run.
 # One launch for both species.
 PUSH_TRAFFIC = {"fp32": (436869120, "ncu capture of k_push32_pipe<3, 2, 15> on this workload (cited, not of this run)"),
-                "fp64": (821560000, "ncu capture of k_push64<1, 1, 1> on this workload (cited, not of this run)")}
+                "fp64": (827579000, "ncu capture of k_push64<1, 1, 1> on this workload (cited, not of this run)")}
 
 
 def combine_ranks(ms, psteps, dist, device):
