@@ -11,7 +11,7 @@ namespace ipg {
 
 namespace {
 // How a launch over `slots` slots in `tiles` tiles is cut: particles per work
-// item, tiles per span, one-warp blocks per span.
+// item, tiles per span, blocks per span and warps per block.
 //   * Items are as long as leaves about six warps per sub-partition (152 SMs
 //     x 4): an item costs a quarter of a round or more, shorter ones leave
 //     a shorter tail and end more evenly. Gather + dipole + deposit, 256
@@ -26,21 +26,26 @@ namespace {
 //     (32^3 1.25 against 1.47, 14^3 0.145 against 0.148, 306k particles 0.081
 //     against 0.083); small universes keep a tile per span, whose table is
 //     sooner scanned (E x B 8^3: 0.021 against 0.029).
-//   * One warp a block: its registers are free as soon as it ends (blocks of
-//     4 warps: 32^3 1.39).
+//   * One warp a block: its registers are free as soon as it ends (blocks of 4
+//     warps: 32^3 1.39). Items of 8 and 16 with the deposit take four, which
+//     join the sums of a cell (Joint64).
 //   * A block takes one round of items, where there is no deposit and the
 //     launch is large four (32^3, dipole mover: 1.31 -> 1.22).
 struct Shape64 {
-    int item, span, parts;
+    int item, span, parts, warps;
 };
 Shape64 shape64(int64_t slots, int64_t tiles, bool deposit) {
     constexpr int64_t kSms = 152, kGroups = 6 * kSms * 4 * kWarpItems64;
-    Shape64 s{32, 1, 1};
+    Shape64 s{32, 1, 1, 1};
     if (deposit) s.item = slots >= kMaxItem64 * kGroups ? kMaxItem64 : 64;
     while (s.item > kGroup64 && slots < s.item * kGroups) s.item /= 2;
     if (tiles >= 2 * kSms) s.span = kMaxSpan64;
     s.parts = s.span * kSlotsPerCta / (s.item * kWarpItems64);
     if (!deposit && tiles >= 6 * kMaxSpan64 * kSms) s.parts /= 4;
+    if (deposit && s.item <= 2 * kGroup64) {
+        s.warps = Joint64::kWarps;
+        s.parts /= s.warps;
+    }
     return s;
 }
 
@@ -76,12 +81,17 @@ int launch_push<double>(const Geom& g, const PopSet<double>& S, int mode, const 
     const Shape64 sh = shape64(slots, tiles, g.deposit != 0);
     const dim3 grid((unsigned)((most + sh.span - 1) / sh.span), sh.parts, S.n);
     const Push64Set pcs = push64_set(g, S);
-    auto run = [&](auto k) { k<<<grid, 32, push64_smem_bytes(sh.span), st>>>(g, S, pcs, sh.span, sh.item); };
-    if (mode != 0) run(k_push64<false, false, true>);
-    else if (g.mover == 1 && g.deposit) run(k_push64<true, true, true>);
-    else if (g.mover == 1) run(k_push64<true, true, false>);
-    else if (g.deposit) run(k_push64<true, false, true>);
-    else run(k_push64<true, false, false>);
+    constexpr int kJ = Joint64::kWarps;
+    auto run = [&](auto k) {
+        k<<<grid, 32 * sh.warps, sh.warps * push64_smem_bytes(sh.span), st>>>(g, S, pcs, sh.span, sh.item);
+    };
+    const bool joined = sh.warps > 1;
+    if (mode != 0) joined ? run(k_push64<false, false, true, kJ>) : run(k_push64<false, false, true, 1>);
+    else if (g.mover == 1 && g.deposit)
+        joined ? run(k_push64<true, true, true, kJ>) : run(k_push64<true, true, true, 1>);
+    else if (g.mover == 1) run(k_push64<true, true, false, 1>);
+    else if (g.deposit) joined ? run(k_push64<true, false, true, kJ>) : run(k_push64<true, false, true, 1>);
+    else run(k_push64<true, false, false, 1>);
     return 1;
 }
 template <>
@@ -103,12 +113,18 @@ int launch_push_batch<double>(const PopJob<double>* jobs, const int2* cta_job, i
     if (nctas <= 0 || (mode != 0 && !g.deposit)) return 0;
     const Shape64 sh = shape64(nctas * kSlotsPerCta, nctas, g.deposit != 0);
     const unsigned grid = (unsigned)(nctas * sh.parts);
-    auto run = [&](auto k) { k<<<grid, 32, push64_smem_bytes(sh.span), st>>>(jobs, cta_job, sh.span, sh.item, sh.parts); };
-    if (mode != 0) run(k_push64_batch<false, false, true>);
-    else if (g.mover == 1 && g.deposit) run(k_push64_batch<true, true, true>);
-    else if (g.mover == 1) run(k_push64_batch<true, true, false>);
-    else if (g.deposit) run(k_push64_batch<true, false, true>);
-    else run(k_push64_batch<true, false, false>);
+    constexpr int kJ = Joint64::kWarps;
+    auto run = [&](auto k) {
+        k<<<grid, 32 * sh.warps, sh.warps * push64_smem_bytes(sh.span), st>>>(jobs, cta_job, sh.span, sh.item,
+                                                                              sh.parts);
+    };
+    const bool joined = sh.warps > 1;
+    if (mode != 0) joined ? run(k_push64_batch<false, false, true, kJ>) : run(k_push64_batch<false, false, true, 1>);
+    else if (g.mover == 1 && g.deposit)
+        joined ? run(k_push64_batch<true, true, true, kJ>) : run(k_push64_batch<true, true, true, 1>);
+    else if (g.mover == 1) run(k_push64_batch<true, true, false, 1>);
+    else if (g.deposit) joined ? run(k_push64_batch<true, false, true, kJ>) : run(k_push64_batch<true, false, true, 1>);
+    else run(k_push64_batch<true, false, false, 1>);
     return 1;
 }
 template <>

@@ -22,8 +22,8 @@
 // gather rounds exactly as the reference does (dipole64.cuh). Measured push
 // per step, before and after: 8.4M particles, gather + dipole + deposit
 // 9.18 -> 1.30 ms (FP64 pipe 66 % busy, issue slots 46 %); 306k particles,
-// two species, gather + deposit 0.593 -> 0.081 ms; 33k particles 0.140 ->
-// 0.021 ms (a warp's serial chain); 1.05M particles, dipole mover, a sixth of
+// two species, gather + deposit 0.593 -> 0.085 ms; 33k particles 0.140 ->
+// 0.022 ms (a warp's serial chain); 1.05M particles, dipole mover, a sixth of
 // them leaving their cells 0.489 -> 0.150 ms (FP64 pipe 58 %, integer 42 %).
 // Loading a round's particles a round ahead changed nothing.
 //
@@ -39,7 +39,7 @@
 // read from L1 and L2). A block is one warp, which takes the items of `span`
 // consecutive 1024-slot tiles, or every gridDim.y-th four of them: cells of
 // up to a tile belong to the span they start in, larger ones are cut at its
-// boundaries.
+// boundaries. Short items with the deposit: blocks of four warps (Joint64).
 #pragma once
 
 #include "dipole64.cuh"
@@ -66,12 +66,12 @@ __device__ __noinline__ double dipole_factor(double mft, double r2) { return mft
 // share the largest one's exponent e_max: fixed = value 2^(1081 - e_max), below
 // 2^59, so that one unit is 2^-59 of the largest corner (FP64's own rounding
 // is 2^-53 of it; a corner below 2^-6 of the largest keeps fewer than 53 bits,
-// which shows only at positions that the others hardly reach). The trilinear polynomial's coefficients are differences of
-// these integers, exact, and the position in the cell is a 64-bit fraction:
-// a product is the high half of 64 x 64 bits. Seven of them and seven sums per
-// component take about 150 integer-pipe cycles per warp; the seven FP64
-// multiply-adds they replace took 448 of the FP64 pipe, which bounds the
-// push.
+// which shows only at positions that the others hardly reach). The trilinear
+// polynomial's coefficients are differences of these integers, exact, and the
+// position in the cell is a 64-bit fraction: a product is the high half of 64
+// x 64 bits. Seven of them and seven sums per component take about 150
+// integer-pipe cycles per warp; the seven FP64 multiply-adds they replace took
+// 448 of the FP64 pipe, which bounds the push.
 
 // coefficients of 1, x, y, xy, z, xz, yz, xyz (index = bits x | y << 1 | z << 2)
 __device__ __forceinline__ int64_t scaled(int64_t c, uint64_t r) {  // floor(c r / 2^64)
@@ -499,7 +499,7 @@ constexpr int kMaxItem64 = 32 * kGroup64;  // a lane's rounds fit a word
 // warps per SM: 128 registers with the deposit (96 spill), 96 without
 constexpr int kDepWarps64 = 16, kMoveWarps64 = 20;
 
-// A block's dynamic shared memory: the cells of its span, their coefficients
+// A warp's dynamic shared memory: the cells of its span, their coefficients
 // per group.
 struct Push64Smem {
     int64_t* start;  // [cells + 1]
@@ -510,13 +510,13 @@ struct Push64Smem {
 __host__ __device__ constexpr size_t push64_smem_bytes(int span) {
     const int cells = span * kMaxCellsPerCta;
     return (size_t)(cells + 2) / 2 * 2 * sizeof(int64_t) + (size_t)kWarpItems64 * kCoefStride64 * sizeof(double) +
-           (size_t)(2 * cells + 1) * sizeof(int);
+           (size_t)(2 * cells + 1 + 3) / 4 * 4 * sizeof(int);
 }
-__device__ __forceinline__ Push64Smem push64_smem(int span) {
+__device__ __forceinline__ Push64Smem push64_smem(int span, int warp) {
     extern __shared__ __align__(16) unsigned char push64_raw[];
     const int cells = span * kMaxCellsPerCta;
     Push64Smem sm;
-    sm.start = reinterpret_cast<int64_t*>(push64_raw);
+    sm.start = reinterpret_cast<int64_t*>(push64_raw + warp * push64_smem_bytes(span));
     sm.coef = sm.start + (cells + 2) / 2 * 2;  // 16-byte aligned
     sm.count = reinterpret_cast<int*>(sm.coef + kWarpItems64 * kCoefStride64);
     sm.first = sm.count + cells;
@@ -606,9 +606,8 @@ __device__ __forceinline__ void leave64(const Geom& g, const Pop<double>& P, int
 // 8.3e-17 -> 2.0e-17 / 2.4e-17 / 2.7e-17, rho 2.7e-17 / 5.0e-17 / 6.4e-17 ->
 // 2.0e-17 / 2.9e-17 / 4.0e-17 (with the unit and the cut of the longest items
 // for all: rho 1.5e-16 / 1.1e-16 / 4.5e-17). Whole universes, error over the
-// size of J: 33k particles 1.9e-16 -> 1.5e-16, 4.8M of 600 a cell 2.7e-16 ->
-// 1.6e-16; of rho: 0.90e-16 -> 0.95e-16 and 1.62e-16 -> 0.95e-16 (short items
-// add to a node more often).
+// size of J: 33k particles 1.9e-16 -> 1.2e-16, 4.8M of 600 a cell 2.7e-16 ->
+// 1.6e-16; of rho: 0.88e-16 -> 0.83e-16 and 1.62e-16 -> 0.95e-16.
 // What is fine is the sum's size, not every node's share of it: a slow
 // particle beside a fast one of its cell, and a node that little of the cell
 // reaches, keep less than 53 bits. One particle at (0.01, 0.02, 0.03) of its
@@ -751,15 +750,257 @@ __device__ __noinline__ void deposit_fp64(const Geom& g, int cell, double x, dou
     deposit_one<double>(g, cell, p, q);
 }
 
+// Blocks of four warps, where items are short (8 or 16 particles): the items'
+// sums are added per cell before the nodes' atomics. Every addition to a node
+// rounds, and a warp's four items are half a cell of 64 particles: with a warp
+// per block rho was 5 to 10 % further from exact sums than FP64 sums of 32
+// lanes of 4 slots each (8^3 cells of 64: 0.93e-16 of its size against 0.87e-16,
+// 10^3 of 256: 1.23e-16 against 1.17e-16), joined it is closer (0.83e-16,
+// 0.86e-16). It costs 2 to 5 % of such a push (8^3: 21.7 -> 22.8 us).
+struct Joint64 {
+    static constexpr int kWarps = 4;
+    static constexpr int kRows = kWarps * kWarpItems64;
+    double sum[kRows][32];  // [item][component * 8 + corner]
+    int cell[kRows];        // -1: nothing, or joined with the item before
+
+    // Adds the rows of every cell to its nodes, a warp per cell.
+    __device__ __forceinline__ void flush(const Geom& g) const {
+        const int lane = threadIdx.x & 31;
+        const int mine = lane < kRows ? cell[lane] : -1;
+        for (int r = threadIdx.x >> 5; r < kRows; r += kWarps) {
+            const int c = __shfl_sync(0xffffffffu, mine, r);
+            unsigned rows = __ballot_sync(0xffffffffu, mine == c);
+            if (c < 0 || (rows & ((1u << r) - 1u))) continue;  // nothing, or the cell's first row has it
+            double s = 0.0;
+            for (; rows; rows &= rows - 1) s += sum[__ffs(rows) - 1][lane];
+            int x, y, z;
+            cell_coords(g, c, x, y, z);
+            const int64_t node = node_index(g, x + (lane & 1), y + ((lane >> 1) & 1), z + ((lane >> 2) & 1));
+            const int q = lane >> 3;
+            atomicAdd(q < 3 ? g.J + 3 * node + q : g.rho + node, s);
+        }
+    }
+};
+
+// The cells of a block's span and its items.
+struct Span64 {
+    int base, top;  // slots
+    int c0, nc;     // cells
+    int total;      // items
+};
+
 // kStep: mover + export (else the deposit of the particles as they are);
-// kField: field-gather mover (else the dipole mover); kDep: deposit.
-template <bool kStep, bool kField, bool kDep>
-__device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P, const Push64Const& pc, int64_t tile,
-                                            int span, int part, int parts, int item) {
+// kField: field-gather mover (else the dipole mover); kDep: deposit; kWarps:
+// warps of the block (more than one: their sums are joined, Joint64).
+// Four items of the span from j0 < total, by one warp.
+template <bool kStep, bool kField, bool kDep, int kWarps>
+__device__ __forceinline__ void push64_items(const Geom& g, const Pop<double>& P, const Push64Const& pc,
+                                             const Push64Smem& sm, const Span64& S, int item, int j0, float reach,
+                                             Joint64* joint, uint32_t& nmig, uint32_t& nrem) {
     constexpr unsigned kAll = 0xffffffffu;
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = kWarps > 1 ? threadIdx.x >> 5 : 0;
     const int gl = lane & (kGroup64 - 1), sub = lane / kGroup64;
-    const Push64Smem sm = push64_smem(span);
+    const int c0 = S.c0, nc = S.nc, total = S.total;
+    int64_t* const coef = sm.coef + sub * kCoefStride64;
+    const int j = min(j0 + sub, total - 1);
+    int i = 0;
+    {
+        int hi = nc - 1;
+        while (i < hi) {
+            const int mid = (i + hi + 1) >> 1;
+            if (sm.first[mid] <= j) i = mid; else hi = mid - 1;
+        }
+    }
+    int64_t lo, end;
+    span_range64(sm, i, S.base, S.top, lo, end);
+    const int pieces = sm.first[i + 1] - sm.first[i];
+    const int piece = ((int)(end - lo) + pieces * kGroup64 - 1) / (pieces * kGroup64) * kGroup64;
+    const int a = (int)lo + (j - sm.first[i]) * piece;
+    int len = max(0, min(piece, (int)end - a));
+    if (j0 + sub >= total) len = 0;
+    const int cell = c0 + i;
+    const int64_t cstart = sm.start[i];
+    Cell64 c;
+    cell_coords(g, cell, c.x, c.y, c.z);
+    double mid[3];
+    {   // lane 0, 1, 2 of the group: the axis' centre
+        const int pos = gl == 0 ? c.x : gl == 1 ? c.y : c.z;
+        const double cen = gl < 3 ? cell_centre(g, gl, pos) : 0.0;
+        const double middle = gl < 3 ? cell_middle(g, gl, pos) : 0.0;
+        const float mine = gl < 3 ? planet_gap(g, gl, cen) : 0.f;
+        float gap[3];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            c.cen[b] = __shfl_sync(kAll, cen, b, kGroup64);
+            mid[b] = __shfl_sync(kAll, middle, b, kGroup64);
+            gap[b] = __shfl_sync(kAll, mine, b, kGroup64);
+        }
+        planet_flags(g, gap, reach, c);
+    }
+    // lane k: corner k, then coefficient k; the components' exponents in
+    // pairs (every lane of the group has them)
+    uint32_t exps[3] = {0u, 0u, 0u};
+    bool fixed = true;
+    if (kStep && kField) {
+        const double* f = corner_field(g, c.x, c.y, c.z, gl);
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const double v = field_value(pc, __ldg(f + q));
+            int e = soft::exponent_of(v);
+            bool zero = (soft::bits_of(v) << 1) == 0;
+#pragma unroll
+            for (int bit = 1; bit < 8; bit <<= 1) e = max(e, __shfl_xor_sync(kAll, e, bit));
+            fixed = fixed && fixed_range(e) && (e != 0 || zero);
+            int64_t n = to_fixed(v, e);
+#pragma unroll
+            for (int bit = 1; bit < 8; bit <<= 1) {
+                const int64_t o = __shfl_xor_sync(kAll, n, bit);
+                if (gl & bit) n -= o;
+            }
+            coef[q * 8 + gl] = n;
+            exps[q >> 1] |= (uint32_t)e << (16 * (q & 1));
+        }
+        fixed = (__ballot_sync(kAll, fixed) >> (sub * kGroup64) & 0xffu) == 0xffu;
+        __syncwarp();
+    }
+    uint32_t adds = 0;            // bit r: the lane's particle of round r adds to the moments
+    int top[3] = {0, 0, 0};       // the components' largest exponents among them
+    const int rounds = __reduce_max_sync(kAll, (len + kGroup64 - 1) / kGroup64);
+    for (int r = 0; r < rounds; ++r) {
+        const int k = r * kGroup64 + gl;
+        const bool has = k < len;
+        const int slot = a + k;
+        // lanes without a particle: the cell's centre at rest
+        PState<double> p = {c.cen[0], c.cen[1], c.cen[2], 0.0, 0.0, 0.0};
+        if (has) p = {P.x[slot], P.y[slot], P.z[slot], P.u[slot], P.v[slot], P.w[slot]};
+        double rel[3];
+        bool stays;
+        if (kStep) {
+            if (kField) {
+                const double at[3] = {p.x - mid[0], p.y - mid[1], p.z - mid[2]};
+                double F[6];
+                if (fixed && in_cell(g, at)) {
+                    const uint64_t rx = fraction(at[0], g.inv_w[0]), ry = fraction(at[1], g.inv_w[1]),
+                                   rz = fraction(at[2], g.inv_w[2]);
+                    // a loop, the results passing through F: unrolled, the
+                    // gather alone was a third of the instruction stream
+                    // (push 1.60 -> 1.43 ms)
+#pragma unroll 1
+                    for (int q = 0; q < 6; ++q) {
+                        const uint32_t e = q < 2 ? exps[0] : q < 4 ? exps[1] : exps[2];
+                        const double f = from_fixed(poly_fixed(coef + 8 * q, rx, ry, rz),
+                                                    (int)(e >> (16 * (q & 1)) & 0xffffu));
+#pragma unroll
+                        for (int k = 0; k < 5; ++k) F[k] = F[k + 1];
+                        F[5] = f;
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 6; ++q)
+                        F[q] = has ? gather_fp64(g, c.x, c.y, c.z, pc.field_scale, at[0], at[1], at[2], q) : 0.0;
+                }
+                move_field64(g, pc, P.qom, F, p);
+            } else if (has) {
+                move_dipole64(g, pc, P.qom, p);
+            }
+            int dest = cell;
+            int outcome = has ? export64(g, c, p, rel, dest) : -1;
+            if (outcome == kStay) {
+                P.x[slot] = p.x; P.y[slot] = p.y; P.z[slot] = p.z;
+                P.u[slot] = p.u; P.v[slot] = p.v; P.w[slot] = p.w;
+            }
+            if (__any_sync(kAll, outcome > kStay))
+                leave64(g, P, outcome, cell, cstart, slot, dest, p, kDep, nmig, nrem);
+            stays = outcome == kStay;
+        } else {
+            rel[0] = p.x - c.cen[0];
+            rel[1] = p.y - c.cen[1];
+            rel[2] = p.z - c.cen[2];
+            stays = has;
+        }
+        if (kDep && stays) {
+            const int e[3] = {soft::exponent_of(p.u), soft::exponent_of(p.v), soft::exponent_of(p.w)};
+            if (in_cell(g, rel) && moment_range(p.u) && moment_range(p.v) && moment_range(p.w)) {
+                adds |= 1u << r;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) top[q] = max(top[q], e[q]);
+            } else {
+                deposit_fp64(g, cell, p.x, p.y, p.z, p.u, p.v, p.w, P.q);
+            }
+        }
+    }
+    if (kDep && __any_sync(kAll, adds != 0)) {
+        Moments64 sums;
+        sums.clear();
+        // groups with items of the same cell (they follow one another) add up
+        // before the FP64 atomics, which round: next: the following
+        // group's cell is this one's, after: the one after it too
+        const int c1 = __shfl_down_sync(kAll, cell, kGroup64), c2 = __shfl_down_sync(kAll, cell, 2 * kGroup64);
+        const int before = __shfl_up_sync(kAll, cell, kGroup64);
+        const bool next = sub < kWarpItems64 - 1 && c1 == cell, after = sub < kWarpItems64 - 2 && c2 == cell;
+        const bool first = sub == 0 || before != cell;
+        const bool shared = __any_sync(kAll, next);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) top[q] = __reduce_max_sync(0xffu << (sub * kGroup64), top[q]);
+        if (shared) {
+            int t[3] = {top[0], top[1], top[2]};
+#pragma unroll
+            for (int k = 1; k < kWarpItems64; ++k) {
+                const bool same = __shfl_xor_sync(kAll, cell, k * kGroup64) == cell;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const int o = __shfl_xor_sync(kAll, t[q], k * kGroup64);
+                    if (same) top[q] = max(top[q], o);
+                }
+            }
+        }
+        // at most so many of the cell's particles in an item, in the warp
+        // (the same in all groups of the cell)
+        const int in_item = min(item, sm.count[cell - c0]), in_warp = min(kWarpItems64 * item, sm.count[cell - c0]);
+        const int room = Moments64::headroom(in_item);
+        for (int r = 0; r < rounds; ++r) {
+            const int slot = a + r * kGroup64 + gl;
+            const bool in = (adds >> r & 1u) != 0;
+            double rel[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
+            if (in) {
+                rel[0] = P.x[slot] - mid[0];
+                rel[1] = P.y[slot] - mid[1];
+                rel[2] = P.z[slot] - mid[2];
+                v[0] = P.u[slot]; v[1] = P.v[slot]; v[2] = P.w[slot];
+            }
+            sums.add(g, room, in, rel, v, top);
+        }
+        sums.corners(room, __popc(adds));
+        const int rho_shift = Moments64::sum_shift(in_warp, room), shift = min(sums.spare_bits(), rho_shift);
+        sums.reduce(shift, rho_shift);
+        if (shared) sums.join(next, after);
+        if (kWarps > 1) {
+            __syncwarp();
+            if (first) {
+                double* const row = joint->sum[warp * kWarpItems64 + sub];
+                if (gl == 0) joint->cell[warp * kWarpItems64 + sub] = cell;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) row[8 * q + gl] = sums.velocity(q, P.q, top[q], room, shift);
+                row[24 + gl] = sums.density(P.q, room, rho_shift);
+            }
+        } else if (first) {
+            const int64_t node = node_index(g, c.x + (gl & 1), c.y + ((gl >> 1) & 1), c.z + (gl >> 2));
+#pragma unroll
+            for (int q = 0; q < 3; ++q)
+                atomicAdd(g.J + 3 * node + q, sums.velocity(q, P.q, top[q], room, shift));
+            atomicAdd(g.rho + node, sums.density(P.q, room, rho_shift));
+        }
+    }
+}
+
+// The items of a span that block `part` of `parts` takes.
+template <bool kStep, bool kField, bool kDep, int kWarps>
+__device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P, const Push64Const& pc, int64_t tile,
+                                            int span, int part, int parts, int item, Joint64* joint) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = kWarps > 1 ? threadIdx.x >> 5 : 0;
+    const Push64Smem sm = push64_smem(span, warp);
     // the cells of the span: consecutive tiles' cells follow one another
     const int base = (int)tile * kSlotsPerCta, top = (int)min(base + (int64_t)span * kSlotsPerCta, P.capacity);
     const int2 cc = __ldg(P.cta_cells + tile), ce = __ldg(P.cta_cells + (top - 1) / kSlotsPerCta);
@@ -790,191 +1031,19 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
     }
     __syncwarp();
     const int total = sm.first[nc];
-    int64_t* const coef = sm.coef + sub * kCoefStride64;
     const float reach = planet_reach(g);
     uint32_t nmig = 0, nrem = 0;
 
-    for (int j0 = part * kWarpItems64; j0 < total; j0 += parts * kWarpItems64) {
-        const int j = min(j0 + sub, total - 1);
-        int i = 0;
-        {
-            int hi = nc - 1;
-            while (i < hi) {
-                const int mid = (i + hi + 1) >> 1;
-                if (sm.first[mid] <= j) i = mid; else hi = mid - 1;
-            }
-        }
-        int64_t lo, end;
-        span_range64(sm, i, base, top, lo, end);
-        const int pieces = sm.first[i + 1] - sm.first[i];
-        const int piece = ((int)(end - lo) + pieces * kGroup64 - 1) / (pieces * kGroup64) * kGroup64;
-        const int a = (int)lo + (j - sm.first[i]) * piece;
-        int len = max(0, min(piece, (int)end - a));
-        if (j0 + sub >= total) len = 0;
-        const int cell = c0 + i;
-        const int64_t cstart = sm.start[i];
-        Cell64 c;
-        cell_coords(g, cell, c.x, c.y, c.z);
-        double mid[3];
-        {   // lane 0, 1, 2 of the group: the axis' centre
-            const int pos = gl == 0 ? c.x : gl == 1 ? c.y : c.z;
-            const double cen = gl < 3 ? cell_centre(g, gl, pos) : 0.0;
-            const double middle = gl < 3 ? cell_middle(g, gl, pos) : 0.0;
-            const float mine = gl < 3 ? planet_gap(g, gl, cen) : 0.f;
-            float gap[3];
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                c.cen[b] = __shfl_sync(kAll, cen, b, kGroup64);
-                mid[b] = __shfl_sync(kAll, middle, b, kGroup64);
-                gap[b] = __shfl_sync(kAll, mine, b, kGroup64);
-            }
-            planet_flags(g, gap, reach, c);
-        }
-        // lane k: corner k, then coefficient k; the components' exponents in
-        // pairs (every lane of the group has them)
-        uint32_t exps[3] = {0u, 0u, 0u};
-        bool fixed = true;
-        if (kStep && kField) {
-            const double* f = corner_field(g, c.x, c.y, c.z, gl);
-            __syncwarp();
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                const double v = field_value(pc, __ldg(f + q));
-                int e = soft::exponent_of(v);
-                bool zero = (soft::bits_of(v) << 1) == 0;
-#pragma unroll
-                for (int bit = 1; bit < 8; bit <<= 1) e = max(e, __shfl_xor_sync(kAll, e, bit));
-                fixed = fixed && fixed_range(e) && (e != 0 || zero);
-                int64_t n = to_fixed(v, e);
-#pragma unroll
-                for (int bit = 1; bit < 8; bit <<= 1) {
-                    const int64_t o = __shfl_xor_sync(kAll, n, bit);
-                    if (gl & bit) n -= o;
-                }
-                coef[q * 8 + gl] = n;
-                exps[q >> 1] |= (uint32_t)e << (16 * (q & 1));
-            }
-            fixed = (__ballot_sync(kAll, fixed) >> (sub * kGroup64) & 0xffu) == 0xffu;
-            __syncwarp();
-        }
-        uint32_t adds = 0;            // bit r: the lane's particle of round r adds to the moments
-        int top[3] = {0, 0, 0};       // the components' largest exponents among them
-        const int rounds = __reduce_max_sync(kAll, (len + kGroup64 - 1) / kGroup64);
-        for (int r = 0; r < rounds; ++r) {
-            const int k = r * kGroup64 + gl;
-            const bool has = k < len;
-            const int slot = a + k;
-            // lanes without a particle: the cell's centre at rest
-            PState<double> p = {c.cen[0], c.cen[1], c.cen[2], 0.0, 0.0, 0.0};
-            if (has) p = {P.x[slot], P.y[slot], P.z[slot], P.u[slot], P.v[slot], P.w[slot]};
-            double rel[3];
-            bool stays;
-            if (kStep) {
-                if (kField) {
-                    const double at[3] = {p.x - mid[0], p.y - mid[1], p.z - mid[2]};
-                    double F[6];
-                    if (fixed && in_cell(g, at)) {
-                        const uint64_t rx = fraction(at[0], g.inv_w[0]), ry = fraction(at[1], g.inv_w[1]),
-                                       rz = fraction(at[2], g.inv_w[2]);
-                        // a loop, the results passing through F: unrolled, the
-                        // gather alone was a third of the instruction stream
-                        // (push 1.60 -> 1.43 ms)
-#pragma unroll 1
-                        for (int q = 0; q < 6; ++q) {
-                            const uint32_t e = q < 2 ? exps[0] : q < 4 ? exps[1] : exps[2];
-                            const double f = from_fixed(poly_fixed(coef + 8 * q, rx, ry, rz),
-                                                        (int)(e >> (16 * (q & 1)) & 0xffffu));
-#pragma unroll
-                            for (int k = 0; k < 5; ++k) F[k] = F[k + 1];
-                            F[5] = f;
-                        }
-                    } else {
-#pragma unroll
-                        for (int q = 0; q < 6; ++q)
-                            F[q] = has ? gather_fp64(g, c.x, c.y, c.z, pc.field_scale, at[0], at[1], at[2], q) : 0.0;
-                    }
-                    move_field64(g, pc, P.qom, F, p);
-                } else if (has) {
-                    move_dipole64(g, pc, P.qom, p);
-                }
-                int dest = cell;
-                int outcome = has ? export64(g, c, p, rel, dest) : -1;
-                if (outcome == kStay) {
-                    P.x[slot] = p.x; P.y[slot] = p.y; P.z[slot] = p.z;
-                    P.u[slot] = p.u; P.v[slot] = p.v; P.w[slot] = p.w;
-                }
-                if (__any_sync(kAll, outcome > kStay))
-                    leave64(g, P, outcome, cell, cstart, slot, dest, p, kDep, nmig, nrem);
-                stays = outcome == kStay;
-            } else {
-                rel[0] = p.x - c.cen[0];
-                rel[1] = p.y - c.cen[1];
-                rel[2] = p.z - c.cen[2];
-                stays = has;
-            }
-            if (kDep && stays) {
-                const int e[3] = {soft::exponent_of(p.u), soft::exponent_of(p.v), soft::exponent_of(p.w)};
-                if (in_cell(g, rel) && moment_range(p.u) && moment_range(p.v) && moment_range(p.w)) {
-                    adds |= 1u << r;
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) top[q] = max(top[q], e[q]);
-                } else {
-                    deposit_fp64(g, cell, p.x, p.y, p.z, p.u, p.v, p.w, P.q);
-                }
-            }
-        }
-        if (kDep && __any_sync(kAll, adds != 0)) {
-            Moments64 sums;
-            sums.clear();
-            // groups with items of the same cell (they follow one another) add up
-            // before the FP64 atomics, which round: next: the following
-            // group's cell is this one's, after: the one after it too
-            const int c1 = __shfl_down_sync(kAll, cell, kGroup64), c2 = __shfl_down_sync(kAll, cell, 2 * kGroup64);
-            const int before = __shfl_up_sync(kAll, cell, kGroup64);
-            const bool next = sub < kWarpItems64 - 1 && c1 == cell, after = sub < kWarpItems64 - 2 && c2 == cell;
-            const bool first = sub == 0 || before != cell;
-            const bool shared = __any_sync(kAll, next);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) top[q] = __reduce_max_sync(0xffu << (sub * kGroup64), top[q]);
-            if (shared) {
-                int t[3] = {top[0], top[1], top[2]};
-#pragma unroll
-                for (int k = 1; k < kWarpItems64; ++k) {
-                    const bool same = __shfl_xor_sync(kAll, cell, k * kGroup64) == cell;
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) {
-                        const int o = __shfl_xor_sync(kAll, t[q], k * kGroup64);
-                        if (same) top[q] = max(top[q], o);
-                    }
-                }
-            }
-            // at most so many of the cell's particles in an item, in the warp
-            // (the same in all groups of the cell)
-            const int in_item = min(item, sm.count[cell - c0]), in_warp = min(kWarpItems64 * item, sm.count[cell - c0]);
-            const int room = Moments64::headroom(in_item);
-            for (int r = 0; r < rounds; ++r) {
-                const int slot = a + r * kGroup64 + gl;
-                const bool in = (adds >> r & 1u) != 0;
-                double rel[3] = {0.0, 0.0, 0.0}, v[3] = {0.0, 0.0, 0.0};
-                if (in) {
-                    rel[0] = P.x[slot] - mid[0];
-                    rel[1] = P.y[slot] - mid[1];
-                    rel[2] = P.z[slot] - mid[2];
-                    v[0] = P.u[slot]; v[1] = P.v[slot]; v[2] = P.w[slot];
-                }
-                sums.add(g, room, in, rel, v, top);
-            }
-            sums.corners(room, __popc(adds));
-            const int rho_shift = Moments64::sum_shift(in_warp, room), shift = min(sums.spare_bits(), rho_shift);
-            sums.reduce(shift, rho_shift);
-            if (shared) sums.join(next, after);
-            if (first) {
-                const int64_t node = node_index(g, c.x + (gl & 1), c.y + ((gl >> 1) & 1), c.z + (gl >> 2));
-#pragma unroll
-                for (int q = 0; q < 3; ++q)
-                    atomicAdd(g.J + 3 * node + q, sums.velocity(q, P.q, top[q], room, shift));
-                atomicAdd(g.rho + node, sums.density(P.q, room, rho_shift));
-            }
+    const Span64 S = {base, top, c0, nc, total};
+    for (int jb = part * kWarps * kWarpItems64; jb < total; jb += parts * kWarps * kWarpItems64) {
+        const int j0 = jb + warp * kWarpItems64;
+        if (kWarps > 1 && lane < kWarpItems64) joint->cell[warp * kWarpItems64 + lane] = -1;
+        if (kWarps == 1 || j0 < total)
+            push64_items<kStep, kField, kDep, kWarps>(g, P, pc, sm, S, item, j0, reach, joint, nmig, nrem);
+        if (kWarps > 1) {
+            __syncthreads();
+            joint->flush(g);
+            if (jb + parts * kWarps * kWarpItems64 < total) __syncthreads();
         }
     }
     if (kStep) {
@@ -987,15 +1056,26 @@ __device__ __forceinline__ void push64_body(const Geom& g, const Pop<double>& P,
     }
 }
 
+template <int kWarps>
+__device__ __forceinline__ Joint64* joint64() {
+    if constexpr (kWarps > 1) {
+        __shared__ Joint64 joint;
+        return &joint;
+    } else {
+        return nullptr;
+    }
+}
+
 // Block (span, part) of population blockIdx.z of the set.
-template <bool kStep, bool kField, bool kDep>
-__global__ void __launch_bounds__(32, kDep ? kDepWarps64 : kMoveWarps64)
+template <bool kStep, bool kField, bool kDep, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, (kDep ? kDepWarps64 : kMoveWarps64) / kWarps)
     k_push64(Geom g, const __grid_constant__ PopSet<double> S, const __grid_constant__ Push64Set pcs, int span,
              int item) {
     const Pop<double>& P = S.p[blockIdx.z];
     const int64_t tile = (int64_t)blockIdx.x * span;
     if (tile * kSlotsPerCta >= P.capacity) return;
-    push64_body<kStep, kField, kDep>(g, P, pcs.c[blockIdx.z], tile, span, blockIdx.y, gridDim.y, item);
+    push64_body<kStep, kField, kDep, kWarps>(g, P, pcs.c[blockIdx.z], tile, span, blockIdx.y, gridDim.y, item,
+                                             joint64<kWarps>());
 }
 
 // Batched: block b is part b % parts of cta_job[b / parts] = (job, tile of the
@@ -1004,15 +1084,17 @@ __global__ void __launch_bounds__(32, kDep ? kDepWarps64 : kMoveWarps64)
 // tiles along x, every fourth block had work, and the SMs, which hand
 // one-warp blocks to their four sub-partitions in turn, ran it all on one
 // (64 universes of 34M particles: 15.3 ms a step, now 7.0).
-template <bool kStep, bool kField, bool kDep>
-__global__ void __launch_bounds__(32, kDep ? kDepWarps64 : kMoveWarps64)
-    k_push64_batch(const PopJob<double>* __restrict__ jobs, const int2* __restrict__ cta_job, int span, int item, int parts) {
+template <bool kStep, bool kField, bool kDep, int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, (kDep ? kDepWarps64 : kMoveWarps64) / kWarps)
+    k_push64_batch(const PopJob<double>* __restrict__ jobs, const int2* __restrict__ cta_job, int span, int item,
+                   int parts) {
     __shared__ PopJob<double> job;
     const unsigned tile = blockIdx.x / (unsigned)parts;
     const int2 cj = __ldg(cta_job + tile);
     if (cj.y % span != 0) return;
     load_job(job, jobs + cj.x);
-    push64_body<kStep, kField, kDep>(job.g, job.P, job.pc, cj.y, span, (int)(blockIdx.x - tile * parts), parts, item);
+    push64_body<kStep, kField, kDep, kWarps>(job.g, job.P, job.pc, cj.y, span, (int)(blockIdx.x - tile * parts), parts,
+                                             item, joint64<kWarps>());
 }
 
 // ---- particles that waited for a slot ---------------------------------------------

@@ -124,3 +124,30 @@ def test_sums_keep_their_last_places(long_items, kind):
                 top, total = max(abs(t) for t in q), sum(abs(t) for t in terms)
                 tol = abs(Q) * (Fraction(fine) * top + 2 * -(-n // item) * total / 2 ** 53)
                 assert abs(Fraction(got[a]) - Fraction(Q) * sum(terms)) <= tol, (n, k, a, got[a], float(tol))
+
+
+def test_cells_reach_their_nodes_in_one_addition():
+    """Work items of 8, cells of 16 items each, no two of which share a node:
+    the items' sums are added in a fixed order and reach the nodes in one
+    addition each, so every projection gives the same bits (several additions
+    to a node round by their order)."""
+    n, per = 9, 128
+    rng = np.random.default_rng(9)
+    c = np.array([(x, y, z) for x in range(0, n, 2) for y in range(0, n, 2) for z in range(0, n, 2)])
+    counts = np.zeros(n ** 3, np.uint64)
+    counts[(c[:, 0] * n + c[:, 1]) * n + c[:, 2]] = per
+    p = np.zeros(len(c) * per, abi.PARTICLE_DTYPE)
+    p["position"] = np.repeat(c, per, 0) + rng.random((len(p), 3))
+    p["velocity"] = rng.normal(0.0, 1.0, (len(p), 3))
+    p["q"], p["qom"] = Q, 1.0
+    props = abi.Props.make(size=(n,) * 3, dt=0.1)
+    sim = gpu_sim(props, abi.Config.make(mover=abi.MOVER_FIELD, projector=abi.PROJECT_CIC))
+    sim.upload_fields(np.zeros(abi.field_shape(props)))
+    sim.upload_particles(p, counts)
+    sim.project()
+    first = sim.download_fields()[2:]
+    for _ in range(15):
+        sim.project()
+        for a, b in zip(sim.download_fields()[2:], first):
+            np.testing.assert_array_equal(a, b)
+    sim.close()
