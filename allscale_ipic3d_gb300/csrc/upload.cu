@@ -116,12 +116,17 @@ __device__ __forceinline__ bool same_value(double a, double b) {
 // records, one after the other (the lanes' moment sums run through them in
 // order): a chunk of a dense region holds few cells. So the next round's
 // records are loaded while this one is worked on, blocks are two warps (a
-// chunk of 100 cells spreads over 50 SMs), the per-species tables stay in
-// registers (kPops), and a round issues no FP64 comparison and no division
-// by a power of two. 16.8M particles, half of them in a blob of up to 4000 a
-// cell: a chunk's kernel took 236 us on average, three times its 16 MB copy;
-// now the copies hide it (upload 16.5 -> 6.0 ms, 5.1 ms of it the link).
-template <bool kDeposit, int kPops, typename T>
+// chunk of 100 cells spreads over 50 SMs), the populations' slots stay in
+// registers, and a round issues no FP64 comparison and no division by a power
+// of two. 16.8M particles, half of them in a blob of up to 4000 a cell: a
+// chunk's kernel took 236 us on average, three times its 16 MB copy; now the
+// copies hide it (upload 16.5 -> 6.0 ms, 5.1 ms of it the link).
+// kMany: more than two populations; lane k keeps population k's slots and
+// count. (Every lane those of all, up to 16, in registers: 138 of them, and a
+// long set-up where cells hold few particles. FP64, 64^3 cells of one particle,
+// upload of 3 / 16 species: 0.705 / 1.08 ms with one form for any number and
+// 256 threads a block, 0.835 / 1.18 so, 0.624 / 0.746 now.)
+template <bool kDeposit, bool kMany, typename T>
 __global__ void __launch_bounds__(kUploadThreads)
     k_upload_cells(const ipic3d_particle* __restrict__ p, const uint32_t* __restrict__ ids,
                    const int64_t* __restrict__ in_off, int c0, int c1, const __grid_constant__ SpeciesTable sp,
@@ -134,15 +139,17 @@ __global__ void __launch_bounds__(kUploadThreads)
     const double oy = g.origin[1] + (double)cy * g.w[1];
     const double oz = g.origin[2] + (double)cz * g.w[2];
     const int64_t a = in_off[c], b = in_off[c + 1];
+    constexpr int kPops = kMany ? 1 : 2;
     int base[kPops], cap[kPops];
     int64_t start[kPops];
 #pragma unroll
     for (int k = 0; k < kPops; ++k) {
         base[k] = cap[k] = 0;
         start[k] = 0;
-        if (k >= U.npop) continue;
-        start[k] = U.start[k][c];
-        cap[k] = (int)(U.start[k][c + 1] - start[k]);
+        const int pop = kMany ? lane : k;
+        if (pop >= U.npop) continue;
+        start[k] = U.start[pop][c];
+        cap[k] = (int)(U.start[pop][c + 1] - start[k]);
     }
     float acc[32];
     if (kDeposit) {
@@ -167,12 +174,19 @@ __global__ void __launch_bounds__(kUploadThreads)
         float wq = 0.f;
         T x = 0, y = 0, z = 0;
         if (i < b) {
+            const auto is = [&](int k) { return same_value(sp.q[k], r3.x) && same_value(sp.qom[k], r3.y); };
+            if constexpr (kMany) {
+                for (int k = 0; s < 0 && k < sp.n; ++k)
+                    if (is(k)) s = k;
+                if (s >= 0) wq = (float)sp.q[s];
+            } else {
 #pragma unroll
-            for (int k = kPops - 1; k >= 0; --k)
-                if (k < sp.n && same_value(sp.q[k], r3.x) && same_value(sp.qom[k], r3.y)) {
-                    s = k;
-                    wq = (float)sp.q[k];
-                }
+                for (int k = 1; k >= 0; --k)
+                    if (k < sp.n && is(k)) {
+                        s = k;
+                        wq = (float)sp.q[k];
+                    }
+            }
             if (s < 0) unknown = true;
         }
         if (s >= 0) {
@@ -187,22 +201,38 @@ __global__ void __launch_bounds__(kUploadThreads)
             }
         }
         const T u = (T)r1.y, v = (T)r2.x, w = (T)r2.y;
-#pragma unroll
-        for (int k = 0; k < kPops; ++k) {
-            if (k >= U.npop) break;
-            const unsigned bal = __ballot_sync(0xffffffffu, s == k);
-            if (s == k) {
-                const int r = base[k] + __popc(bal & ((1u << lane) - 1u));
-                if (r < cap[k]) {
-                    const int64_t slot = start[k] + r;
-                    U.x[k][slot] = x; U.y[k][slot] = y; U.z[k][slot] = z;
-                    U.u[k][slot] = u; U.v[k][slot] = v; U.w[k][slot] = w;
-                    if (U.id[k]) U.id[k][slot] = ids ? ids[i] : (uint32_t)i;
-                } else {
-                    full = true;
-                }
+        const auto store = [&](int k, int64_t slot) {
+            U.x[k][slot] = x; U.y[k][slot] = y; U.z[k][slot] = z;
+            U.u[k][slot] = u; U.v[k][slot] = v; U.w[k][slot] = w;
+            if (U.id[k]) U.id[k][slot] = ids ? ids[i] : (uint32_t)i;
+        };
+        const unsigned below = (1u << lane) - 1u;
+        if constexpr (kMany) {
+            int rank = 0, mine = 0;
+            for (int k = 0; k < U.npop; ++k) {
+                const unsigned bal = __ballot_sync(0xffffffffu, s == k);
+                if (s == k) rank = __popc(bal & below);
+                if (lane == k) mine = __popc(bal);
             }
-            base[k] += __popc(bal);
+            const int from = s < 0 ? 0 : s;
+            const int r = __shfl_sync(0xffffffffu, base[0], from) + rank;
+            const int room = __shfl_sync(0xffffffffu, cap[0], from);
+            const int64_t first = __shfl_sync(0xffffffffu, start[0], from);
+            base[0] += mine;
+            if (s >= 0 && r < room) store(s, first + r);
+            else if (s >= 0) full = true;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                if (k >= U.npop) break;
+                const unsigned bal = __ballot_sync(0xffffffffu, s == k);
+                if (s == k) {
+                    const int r = base[k] + __popc(bal & below);
+                    if (r < cap[k]) store(k, start[k] + r);
+                    else full = true;
+                }
+                base[k] += __popc(bal);
+            }
         }
         if (kDeposit && s >= 0)
             add_moments_q(acc, (float)x, (float)y, (float)z, (float)r1.y, (float)r2.x, (float)r2.y, wq);
@@ -211,7 +241,7 @@ __global__ void __launch_bounds__(kUploadThreads)
     if (__any_sync(0xffffffffu, full) && lane == 0) atomicExch(flags + 1, 1);
 #pragma unroll
     for (int k = 0; k < kPops; ++k)
-        if (k < U.npop && lane == k) U.count[k][c] = base[k] < cap[k] ? base[k] : cap[k];
+        if (lane < U.npop && (kMany || lane == k)) U.count[lane][c] = min(base[k], cap[k]);
     if (kDeposit) {
         // lane v: summed moment v = 8 Q + m; three axis butterflies give the
         // corner sums (corner m, component Q); one FP64 atomic each
@@ -258,13 +288,12 @@ int launch_upload_cells(const void* parts, const uint32_t* ids, const int64_t* i
     auto run = [&](auto k) {
         k<<<blocks, kUploadThreads, 0, st>>>((const ipic3d_particle*)parts, ids, in_off, c0, c1, sp, U, g, dep, flags);
     };
-    // the per-species tables in registers for up to 2 populations
     if (dep.on) {
-        if (U.npop <= 2) run(k_upload_cells<true, 2, T>);
-        else run(k_upload_cells<true, kUploadMaxPops, T>);
+        if (U.npop <= 2) run(k_upload_cells<true, false, T>);
+        else run(k_upload_cells<true, true, T>);
     } else {
-        if (U.npop <= 2) run(k_upload_cells<false, 2, T>);
-        else run(k_upload_cells<false, kUploadMaxPops, T>);
+        if (U.npop <= 2) run(k_upload_cells<false, false, T>);
+        else run(k_upload_cells<false, true, T>);
     }
     return 1;
 }
