@@ -2075,7 +2075,7 @@ struct ipic3d_batch {
     uint32_t* h_flag = nullptr;  // pinned ring of two
     cudaEvent_t flag_ev[2] = {nullptr, nullptr};
     int64_t nctas = 0, nplace = 0;
-    int tile_cells = 0;  // the most cells of any tile
+    BatchTraits traits;
     int max_s = 0;
     int64_t max_cells = 0, max_nodes = 0;
     bool tables = false;
@@ -2201,8 +2201,11 @@ int batch_tables(ipic3d_batch* b) {
     cur.swap(nj);
     b->ij.swap(ni);
     b->nctas = (int64_t)cta.size();
-    b->tile_cells = 0;
-    for (const auto& j : cur) b->tile_cells = std::max(b->tile_cells, (int)j.P.tile_cells);
+    b->traits = BatchTraits{};
+    for (const auto& j : cur) {
+        b->traits.tile_cells = std::max(b->traits.tile_cells, (int)j.P.tile_cells);
+        b->traits.sub_cycles = b->traits.sub_cycles || many_sub_cycles(j.g, j.P.qom);
+    }
     b->nplace = (int64_t)place.size();
     b->max_s = max_s;
     b->max_cells = max_cells;
@@ -2241,7 +2244,7 @@ int batch_enqueue_step(ipic3d_batch* b) {
     if (nj > 0) {
         if ((rc = fork(0, st, aux))) return rc;
         if (b->tune_timing) CU(cudaEventRecord(b->tune_ev[0], st));
-        n += launch_push_batch<T>(jobs, b->d_cta, b->nctas, 0, jobs_of<T>(b)[0].g, b->tile_cells, b->tuner.next(), st);
+        n += launch_push_batch<T>(jobs, b->d_cta, b->nctas, 0, jobs_of<T>(b)[0].g, b->traits, b->tuner.next(), st);
         if (b->tune_timing) CU(cudaEventRecord(b->tune_ev[1], st));
         n += launch_push_pending_batch<T>(jobs, nj, aux);
         if ((rc = fork(1, aux, st))) return rc;

@@ -33,9 +33,14 @@ template <typename T>
 int launch_pending_count(const Pop<T>& P, int32_t* per_cell, cudaStream_t st);
 
 // batched ensemble: job tables built by the host (particles_fp64/32.cu)
+// what the push's instances and split depend on besides the job tables.
+struct BatchTraits {
+    int tile_cells = 0;       // the most cells of any tile
+    bool sub_cycles = false;  // many_sub_cycles of any job
+};
 template <typename T>
 int launch_push_batch(const PopJob<T>* jobs, const int2* cta_job, int64_t nctas, int mode, const Geom& g0,
-                      int tile_cells, const PushShape& shp, cudaStream_t st);  // g0: the policy fields (mover, flags, deposit) shared by the jobs
+                      const BatchTraits& traits, const PushShape& shp, cudaStream_t st);  // g0: the policy fields (mover, flags, deposit) shared by the jobs
 template <typename T>
 int launch_push_pending_batch(const PopJob<T>* jobs, int njobs, cudaStream_t st);
 // tab: nblocks entries (job, block of the job), place_blocks(ncells,
@@ -54,6 +59,8 @@ int launch_batch_status(const PopJob<T>* jobs, int njobs, JobStatus* out, cudaSt
 int launch_cell_coef_batch(const InstJob* inst, int ninst, int64_t max_cells, cudaStream_t st);  // particles_fp32.cu
 Push32Const push32_const(const Geom& g, const Pop<float>& P);                                    // particles_fp32.cu
 Push64Const push64_const(const Geom& g, const Pop<double>& P);                                   // particles_fp64.cu
+// whether the dipole can ask for 8 sub-cycles or more somewhere in the domain (particles_fp64.cu)
+bool many_sub_cycles(const Geom& g, double qom);
 cudaError_t init_push32(int dev);  // once per device, before any capture (particles_fp32.cu)
 int push32_blocks_per_sm(int dev);  // resident pipelined-push blocks per SM (after init_push32)
 int launch_ghost_batch(const InstJob* jobs, int ninst, int max_s, cudaStream_t st);              // fields.cu

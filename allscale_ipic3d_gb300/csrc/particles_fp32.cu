@@ -234,10 +234,10 @@ int launch_cell_coef(const Geom& g, float* coef, cudaStream_t st) {
 // the batched FP32 step: the pipelined push over every job's tiles
 template <>
 int launch_push_batch<float>(const PopJob<float>* jobs, const int2* cta_job, int64_t nctas, int mode,
-                             const Geom& g0, int tile_cells, const PushShape& shp, cudaStream_t st) {
+                             const Geom& g0, const BatchTraits& traits, const PushShape& shp, cudaStream_t st) {
     if (nctas <= 0) return 0;
     if (mode != 0 && !g0.deposit) return 0;
-    PipeJobsFn fn = pipe_jobs_kernel(pipe_policy(g0, mode, tile_cells, shp));
+    PipeJobsFn fn = pipe_jobs_kernel(pipe_policy(g0, mode, traits.tile_cells, shp));
     if (!fn) return 0;
     fn<<<pipe_grid(shp, nctas), kPipeThreads, pipe_smem_bytes<kPipeStages>(), st>>>(jobs, cta_job, (int)nctas,
                                                                                     clamp_shape(shp));

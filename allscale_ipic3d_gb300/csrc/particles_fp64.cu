@@ -31,13 +31,18 @@ namespace {
 //     join the sums of a cell (Joint64).
 //   * A block takes one round of items, where there is no deposit and the
 //     launch is large four (32^3, dipole mover: 1.31 -> 1.22).
+//   * Items of 32 at most where the dipole can ask for many sub-cycles
+//     (many_sub_cycles): a round of 8 particles close to it takes up to 0.25 ms,
+//     and an item's rounds follow one another (planet of one cell, bz 30, dipole
+//     mover with deposit, push of 26^3 cells of 256: 3.98 ms -> 1.61, of 24^3
+//     cells of 64: 0.97 -> 0.63).
 struct Shape64 {
     int item, span, parts, warps;
 };
-Shape64 shape64(int64_t slots, int64_t tiles, bool deposit) {
+Shape64 shape64(int64_t slots, int64_t tiles, bool deposit, bool sub_cycles) {
     constexpr int64_t kSms = 152, kGroups = 6 * kSms * 4 * kWarpItems64;
     Shape64 s{32, 1, 1, 1};
-    if (deposit) s.item = slots >= kMaxItem64 * kGroups ? kMaxItem64 : 64;
+    if (deposit && !sub_cycles) s.item = slots >= kMaxItem64 * kGroups ? kMaxItem64 : 64;
     while (s.item > kGroup64 && slots < s.item * kGroups) s.item /= 2;
     if (tiles >= 2 * kSms) s.span = kMaxSpan64;
     s.parts = s.span * kSlotsPerCta / (s.item * kWarpItems64);
@@ -55,6 +60,25 @@ Push64Set push64_set(const Geom& g, const PopSet<double>& S) {
     return pcs;
 }
 }  // namespace
+
+bool many_sub_cycles(const Geom& g, double qom) {
+    if (g.mft == 0.0 || (g.mover == 1 && !(g.flags & 4u))) return false;
+    double r2 = 0.0;  // of the closest point of the domain to the dipole
+    for (int a = 0; a < 3; ++a) {
+        const double out = std::max(g.origin[a], -(g.origin[a] + g.L[a]));
+        if (out > 0.0) r2 += out * out;
+    }
+    // the planet drops what comes closer
+    if (g.object_center[0] == 0.0 && g.object_center[1] == 0.0 && g.object_center[2] == 0.0)
+        r2 = std::max(r2, g.planet_r2);
+    // too few particles to matter (32^3 cells of 256, |B| above the line within
+    // 0.3 cells, field mover: 1.64 ms without the short items, 1.86 with them;
+    // within 0.63 cells 2.11 and 1.90)
+    const double half = 0.5 * std::min(g.w[0], std::min(g.w[1], g.w[2]));
+    r2 = std::max(r2, half * half);
+    const double b2 = 4.0 * g.mft * g.mft / (r2 * r2 * r2);  // at the pole
+    return g.dt * (4.0 * std::fabs(qom)) * b2 * g.inv_pic >= 8.0;
+}
 
 Push64Const push64_const(const Geom& g, const Pop<double>& P) {
     Push64Const c;
@@ -78,7 +102,9 @@ int launch_push<double>(const Geom& g, const PopSet<double>& S, int mode, const 
         slots += S.p[i].capacity;
     }
     if (most <= 0 || (mode != 0 && !g.deposit)) return 0;
-    const Shape64 sh = shape64(slots, tiles, g.deposit != 0);
+    bool sub_cycles = false;
+    for (int i = 0; i < S.n; ++i) sub_cycles = sub_cycles || many_sub_cycles(g, S.p[i].qom);
+    const Shape64 sh = shape64(slots, tiles, g.deposit != 0, sub_cycles);
     const dim3 grid((unsigned)((most + sh.span - 1) / sh.span), sh.parts, S.n);
     const Push64Set pcs = push64_set(g, S);
     constexpr int kJ = Joint64::kWarps;
@@ -109,9 +135,9 @@ template int launch_pending_count<double>(const Pop<double>&, int32_t*, cudaStre
 
 template <>
 int launch_push_batch<double>(const PopJob<double>* jobs, const int2* cta_job, int64_t nctas, int mode,
-                              const Geom& g, int, const PushShape&, cudaStream_t st) {
+                              const Geom& g, const BatchTraits& traits, const PushShape&, cudaStream_t st) {
     if (nctas <= 0 || (mode != 0 && !g.deposit)) return 0;
-    const Shape64 sh = shape64(nctas * kSlotsPerCta, nctas, g.deposit != 0);
+    const Shape64 sh = shape64(nctas * kSlotsPerCta, nctas, g.deposit != 0, traits.sub_cycles);
     const unsigned grid = (unsigned)(nctas * sh.parts);
     constexpr int kJ = Joint64::kWarps;
     auto run = [&](auto k) {
